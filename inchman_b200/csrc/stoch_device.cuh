@@ -179,12 +179,18 @@ __device__ __forceinline__ void homog_lost(int n, float pmove, Stream& st, int x
     l[0] = l[1] = l[2] = l[3] = 0;
     const int moved = binomial(st, n, pmove);
     if (moved <= 64) {
-        uint32_t w = 0;
-        for (int i = 0; i < moved; ++i) {
-            if ((i & 15) == 0) w = st.next();
-            const uint32_t d = (w >> (2 * (i & 15))) & 3u;
-            l[0] += d == 0u; l[1] += d == 1u; l[2] += d == 2u; l[3] += d == 3u;
+        // sixteen 2-bit directions per draw, counted by their bits
+        int c1 = 0, c2 = 0, c3 = 0;
+        for (int left = moved; left > 0; left -= 16) {
+            uint32_t w = st.next();
+            if (left < 16) w &= (1u << (2 * left)) - 1u;
+            const uint32_t lo = w & 0x55555555u, hi = (w >> 1) & 0x55555555u;
+            const int both = __popc(lo & hi);
+            c3 += both;
+            c1 += __popc(lo) - both;
+            c2 += __popc(hi) - both;
         }
+        l[0] = moved - c1 - c2 - c3; l[1] = c1; l[2] = c2; l[3] = c3;
     } else {
         l[0] = binomial(st, moved, 0.25f);
         l[1] = binomial(st, moved - l[0], 1.0f / 3.0f);

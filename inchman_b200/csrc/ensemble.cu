@@ -21,6 +21,7 @@
 #include <cuda_runtime.h>
 #include "host_common.h"
 #include "stoch_device.cuh"
+#include "netpack.h"
 #include "../../include/gpgmp_c.h"
 
 using namespace gpgmp;
@@ -33,12 +34,20 @@ struct Ctrl {
     int nsnap;
 };
 
+// the reaction structs and their dependency masks, or the packed tables
+constexpr size_t kEnsTables = (sizeof(gpgmp_reaction) + sizeof(uint32_t) * 4) * MAX_REACTIONS;
+static_assert(kEnsTables >= (sizeof(float4) + sizeof(uint4)) * MAX_REACTIONS + sizeof(float) * 1024 &&
+                  kEnsTables % 16 == 0,
+              "the packed tables and one slot per thread");
+
 struct EnsArgs {
     const gpgmp_instance* inst;
     const int32_t* order;
     int max_reactions;
     const float* diffusion;
     const gpgmp_reaction* reactions;
+    const PackedReaction* packed;   // beside reactions
+    const int32_t* nnet;            // per instance: pack_network's, 0 where its network does not fit
     int32_t* state;
     int32_t* snapshots;
     float* snap_times;       // [instance][max_snapshots] (index = snapshot_offset / block... host computes)
@@ -52,17 +61,22 @@ struct EnsArgs {
     int max_species;
 };
 
-__global__ void k_ensemble(EnsArgs A) {
+template <int NT>
+__global__ void __launch_bounds__(NT) k_ensemble(EnsArgs A) {
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ gpgmp_instance s_inst;
     __shared__ Ctrl c;
     __shared__ float s_D[MAX_SPECIES], s_dt[MAX_SPECIES], s_next[MAX_SPECIES];
     __shared__ int s_item;
-    const int NT = blockDim.x;
+    // one network at a time: the packed tables or the reaction structs and their dependencies
     gpgmp_reaction* rt = reinterpret_cast<gpgmp_reaction*>(smem);
     uint32_t* deps = reinterpret_cast<uint32_t*>(smem + sizeof(gpgmp_reaction) * MAX_REACTIONS);
-    int* xs = reinterpret_cast<int*>(deps + 4 * MAX_REACTIONS);
+    float4* ent = reinterpret_cast<float4*>(smem);
+    uint4* nets = reinterpret_cast<uint4*>(ent + MAX_REACTIONS);
+    int* xs = reinterpret_cast<int*>(smem + kEnsTables);
     float* hs = reinterpret_cast<float*>(xs + (size_t)A.max_species * NT);
+    // the packed form's slot 0 of every thread lies in the part of the tables that it leaves free
+    float* slots = reinterpret_cast<float*>(xs) - NT + threadIdx.x;
     int32_t* lost = A.lost + (int64_t)blockIdx.x * A.lost_stride;
     for (;;) {
         if (threadIdx.x == 0) s_item = (int)atomicAdd(A.queue, 1u);
@@ -73,9 +87,15 @@ __global__ void k_ensemble(EnsArgs A) {
         if (threadIdx.x == 0) s_inst = A.inst[id];
         __syncthreads();
         const int W = s_inst.width, area = W * W, S = s_inst.num_species, R = s_inst.num_reactions;
-        for (int i = threadIdx.x; i < R; i += NT) rt[i] = A.reactions[s_inst.reaction_offset + i];
-        __syncthreads();
-        build_deps(rt, R, deps);
+        const gpgmp_reaction* reactions = A.reactions + s_inst.reaction_offset;
+        const int nnet = A.nnet[id];
+        if (nnet > 0) {
+            packed_tables<NT>(A.packed + s_inst.reaction_offset, R, ent, nets);
+        } else {
+            for (int i = threadIdx.x; i < R; i += NT) rt[i] = reactions[i];
+            __syncthreads();
+            build_deps(rt, R, deps);
+        }
         int32_t* st = A.state + s_inst.state_offset;
         const uint32_t key0 = s_inst.seed, key1 = s_inst.realisation;
         const int bm[4] = {s_inst.boundary_mask[0], s_inst.boundary_mask[1], s_inst.boundary_mask[2],
@@ -139,12 +159,21 @@ __global__ void k_ensemble(EnsArgs A) {
                 int* x = xs + threadIdx.x;
                 int err = 0;
                 for (int cell = threadIdx.x; cell < area; cell += NT) {
-                    for (int s = 0; s < S; ++s) x[s * NT] = st[(int64_t)s * area + cell];
                     Stream rs;
                     rs.init(key0, key1, sd, (uint32_t)cell, PH_SSA);
+                    const auto at = [&](int s) -> int32_t& { return st[(int64_t)s * area + cell]; };
+                    if (nnet > 0) {
+                        err |= packed_window<NT>(
+                            reactions, R, at, S, slots, rs, c.window,
+                            [&](float* xf, Stream& q, SsaPos& pos) {
+                                return ssa_packed<NT>(ent, nets, nnet, R, xf, hs + threadIdx.x, q, c.window, pos);
+                            });
+                        continue;
+                    }
+                    for (int s = 0; s < S; ++s) x[s * NT] = at(s);
                     err |= R > 6 ? ssa_cell_inc(rt, deps, R, x, NT, hs + threadIdx.x, rs, c.window)
                                  : ssa_cell(rt, R, x, NT, rs, c.window);
-                    for (int s = 0; s < S; ++s) st[(int64_t)s * area + cell] = x[s * NT];
+                    for (int s = 0; s < S; ++s) at(s) = x[s * NT];
                 }
                 if (err) atomicOr(&A.status[id], err);
                 sd++;
@@ -222,6 +251,8 @@ struct gpgmp_ensemble {
     float* d_diff = nullptr;
     float* d_lambda = nullptr;
     gpgmp_reaction* d_reac = nullptr;
+    PackedReaction* d_packed = nullptr;
+    int32_t* d_nnet = nullptr;
     int32_t* d_status = nullptr;
     int64_t* d_steps = nullptr;
     int64_t* d_snap_time_off = nullptr;
@@ -249,7 +280,7 @@ namespace {
 void ens_free(gpgmp_ensemble* h) {
     if (h->exec) cudaGraphExecDestroy(h->exec);
     if (h->graph) cudaGraphDestroy(h->graph);
-    void* ptrs[] = {h->d_inst, h->d_order, h->d_diff, h->d_lambda, h->d_reac, h->d_status, h->d_steps,
+    void* ptrs[] = {h->d_inst, h->d_order, h->d_diff, h->d_lambda, h->d_reac, h->d_packed, h->d_nnet, h->d_status, h->d_steps,
                     h->d_snap_time_off, h->d_snap_times, h->d_lost, h->d_queue};
     for (void* p : ptrs)
         if (p) cudaFree(p);
@@ -265,18 +296,27 @@ double est_cost(const gpgmp_instance& I, const float* diffusion) {
     return (double)I.width * I.width * I.num_species * steps * (1.0 + I.num_reactions / 4.0);
 }
 
+const void* ens_kernel(int threads) {
+    switch (threads) {
+        case 128: return (const void*)k_ensemble<128>;
+        case 256: return (const void*)k_ensemble<256>;
+        case 512: return (const void*)k_ensemble<512>;
+        default: return (const void*)k_ensemble<1024>;
+    }
+}
+
 int configure(gpgmp_ensemble* h, int threads, int ctas_per_sm) {
     if (threads != 128 && threads != 256 && threads != 512 && threads != 1024)
         return set_error(GPGMP_ERR_INVALID, "threads per CTA must be 128, 256, 512 or 1024");
     h->threads = threads;
-    h->smem = sizeof(gpgmp_reaction) * MAX_REACTIONS + sizeof(uint32_t) * 4 * MAX_REACTIONS +
-              sizeof(int) * (size_t)h->max_species * threads + sizeof(float) * (size_t)h->max_reactions * threads;
-    CK(cudaFuncSetAttribute(k_ensemble, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)h->smem));
+    h->smem = kEnsTables + sizeof(int) * (size_t)h->max_species * threads +
+              sizeof(float) * (size_t)h->max_reactions * threads;
+    CK(cudaFuncSetAttribute(ens_kernel(threads), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)h->smem));
     int dev = 0, sms = 0;
     CK(cudaGetDevice(&dev));
     CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     int occ = 0;
-    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_ensemble, threads, h->smem));
+    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, ens_kernel(threads), threads, h->smem));
     if (occ < 1) return set_error(GPGMP_ERR_UNSUPPORTED, "ensemble kernel does not fit an SM");
     h->num_sms = sms;
     h->ctas_per_sm = std::max(1, std::min(ctas_per_sm, occ));
@@ -334,6 +374,15 @@ int gpgmp_ensemble_create(const gpgmp_instance* instances, int32_t n, const floa
             snap_total += I.max_snapshots;
         }
     }
+    std::vector<PackedReaction> packed(n_reactions > 0 ? n_reactions : 1);
+    std::vector<int32_t> nnet(n, 0);
+    for (int i = 0; i < n; ++i) {
+        const gpgmp_instance& I = instances[i];
+        int changed = 1;
+        if (I.num_reactions > 0 && pack_network(reactions + I.reaction_offset, I.num_reactions, I.num_species,
+                                                packed.data() + I.reaction_offset, &changed))
+            nnet[i] = changed;
+    }
     std::vector<int32_t> order(n);
     for (int i = 0; i < n; ++i) order[i] = i;
     std::vector<double> cost(n);
@@ -346,6 +395,8 @@ int gpgmp_ensemble_create(const gpgmp_instance* instances, int32_t n, const floa
     A((void**)&h->d_diff, sizeof(float) * n_diffusion);
     A((void**)&h->d_lambda, sizeof(float) * n_diffusion);
     A((void**)&h->d_reac, sizeof(gpgmp_reaction) * (n_reactions > 0 ? n_reactions : 1));
+    A((void**)&h->d_packed, sizeof(PackedReaction) * (n_reactions > 0 ? n_reactions : 1));
+    A((void**)&h->d_nnet, sizeof(int32_t) * n);
     A((void**)&h->d_status, sizeof(int32_t) * n);
     A((void**)&h->d_steps, sizeof(int64_t) * n);
     A((void**)&h->d_snap_time_off, sizeof(int64_t) * n);
@@ -358,6 +409,9 @@ int gpgmp_ensemble_create(const gpgmp_instance* instances, int32_t n, const floa
         e = cudaMemcpy(h->d_lambda, lambda, sizeof(float) * n_diffusion, cudaMemcpyHostToDevice);
     if (e == cudaSuccess && n_reactions > 0)
         e = cudaMemcpy(h->d_reac, reactions, sizeof(gpgmp_reaction) * n_reactions, cudaMemcpyHostToDevice);
+    if (e == cudaSuccess && n_reactions > 0)
+        e = cudaMemcpy(h->d_packed, packed.data(), sizeof(PackedReaction) * n_reactions, cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) e = cudaMemcpy(h->d_nnet, nnet.data(), sizeof(int32_t) * n, cudaMemcpyHostToDevice);
     if (e == cudaSuccess)
         e = cudaMemcpy(h->d_snap_time_off, snap_off.data(), sizeof(int64_t) * n, cudaMemcpyHostToDevice);
     h->snap_time_total = snap_total;
@@ -410,6 +464,7 @@ int gpgmp_ensemble_run(gpgmp_ensemble* h, int32_t* state, int32_t* snapshots, vo
         CK(cudaStreamCreateWithFlags(&cap, cudaStreamNonBlocking));
         EnsArgs a{};
         a.inst = h->d_inst; a.order = h->d_order; a.diffusion = h->d_diff; a.reactions = h->d_reac;
+        a.packed = h->d_packed; a.nnet = h->d_nnet;
         a.state = state; a.snapshots = snapshots; a.snap_times = h->d_snap_times;
         a.snap_time_off = h->d_snap_time_off; a.status = h->d_status; a.steps = h->d_steps;
         a.lost = h->d_lost; a.lost_stride = 4 * (int64_t)h->max_area; a.queue = h->d_queue; a.n_inst = h->n;
@@ -419,7 +474,8 @@ int gpgmp_ensemble_run(gpgmp_ensemble* h, int32_t* state, int32_t* snapshots, vo
         if (e == cudaSuccess) {
             cudaMemsetAsync(h->d_queue, 0, sizeof(unsigned int), cap);
             cudaMemsetAsync(h->d_status, 0, sizeof(int32_t) * h->n, cap);
-            k_ensemble<<<h->grid, h->threads, h->smem, cap>>>(a);
+            void* args[] = {&a};
+            cudaLaunchKernel(ens_kernel(h->threads), dim3(h->grid), dim3(h->threads), args, h->smem, cap);
             e = cudaStreamEndCapture(cap, &h->graph);
         }
         cudaStreamDestroy(cap);

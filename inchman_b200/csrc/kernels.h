@@ -32,6 +32,14 @@ struct GridDesc {
     int tile;
     int ssa_threads;
 };
+// A network in the packed form of the SSA (pack_network), on the host and on the device;
+// host == nullptr where it does not fit that form
+struct PackedReaction;
+struct NetDesc {
+    const PackedReaction* host;
+    const PackedReaction* dev;
+    int nnet;
+};
 // the tile of shape index i is w x h cells; SSA block size choice i is that many threads
 void diffusion_tile_shape(int index, int* w, int* h);
 int ssa_thread_choice(int index);
@@ -39,7 +47,8 @@ int ssa_thread_choice(int index);
 cudaError_t launch_init_poisson(const GridDesc& g, Planes planes, uint32_t seed, const float* d_lambda,
                                 cudaStream_t st);
 cudaError_t launch_ssa(const GridDesc& g, Planes planes, const gpgmp_reaction* d_reactions, int nreac,
-                       uint32_t seed, uint32_t step_seed, float window, int32_t* d_status, cudaStream_t st);
+                       const NetDesc& net, uint32_t seed, uint32_t step_seed, float window, int32_t* d_status,
+                       cudaStream_t st);
 cudaError_t launch_homog_diffuse(const GridDesc& g, const int32_t* in, int32_t* out, int species, uint32_t seed,
                                  uint32_t step_seed, float pmove, cudaStream_t st);
 cudaError_t launch_source(const GridDesc& g, int32_t* plane_base, int species, uint32_t seed, uint32_t step_seed,

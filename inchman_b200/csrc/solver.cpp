@@ -18,6 +18,7 @@
 #include "host_common.h"
 #include "jit.h"
 #include "individual.h"
+#include "netpack.h"
 
 using namespace gpgmp;
 
@@ -47,6 +48,10 @@ struct gpgmp_solver {
     float* d_fbuf[2] = {nullptr, nullptr};
     int fcur = 0;
     gpgmp_reaction* d_reactions = nullptr;
+    std::vector<PackedReaction> packed;      // the network in the SSA's packed form; empty where it does not fit
+    PackedReaction* d_packed = nullptr;
+    int nnet = 1;
+    NetDesc net() const { return {packed.empty() ? nullptr : packed.data(), d_packed, nnet}; }
     uint32_t* d_rmask = nullptr;      // localised reactions: [words][area] bits (GridDesc::rmask), or NULL
     int32_t* d_status = nullptr;
     float* d_diff = nullptr;
@@ -150,7 +155,7 @@ int normalize(gpgmp_solver* h) {
 void free_all(gpgmp_solver* h) {
     void* ptrs[] = {h->d_buf[0], h->d_buf[1], h->d_fbuf[0], h->d_fbuf[1], h->d_reactions, h->d_status, h->d_diff,
                     h->d_Dx, h->d_Dy, h->d_rx, h->d_ry, h->d_minkey, h->d_lambda, h->d_stage, h->d_meanx,
-                    h->d_msums, h->d_fields, h->d_rmask};
+                    h->d_msums, h->d_fields, h->d_rmask, h->d_packed};
     for (void* p : ptrs)
         if (p) cudaFree(p);
     for (IndList& l : h->ind) ind_free(l);
@@ -531,6 +536,16 @@ int gpgmp_solver_create(const gpgmp_model_desc* model, int32_t num_realisations,
         CKC(cudaMemcpy(h->d_reactions, h->reactions.data(), sizeof(gpgmp_reaction) * h->reactions.size(),
                        cudaMemcpyHostToDevice));
     }
+    if (!h->reactions.empty() && !h->deterministic) {
+        h->packed.resize(h->reactions.size());
+        if (pack_network(h->reactions.data(), (int)h->reactions.size(), model->num_species, h->packed.data(), &h->nnet)) {
+            CKC(cudaMalloc(&h->d_packed, sizeof(PackedReaction) * h->packed.size()));
+            CKC(cudaMemcpy(h->d_packed, h->packed.data(), sizeof(PackedReaction) * h->packed.size(),
+                           cudaMemcpyHostToDevice));
+        } else {
+            h->packed.clear();
+        }
+    }
     if (model->reaction_mask && !h->reactions.empty()) {
         // localised reactions (Solver.cpp:352-390 builds the same mask as a float image):
         // one bit per reaction and cell, 32 reactions to a word, words cell-contiguous
@@ -677,7 +692,7 @@ int gpgmp_do_reactions(gpgmp_solver* h, float deltat, int32_t* seed) {
                                                          (int)h->reactions.size(), h->seed, (uint32_t)*seed, deltat,
                                                          h->d_status, h->stream)
                                         : launch_ssa(h->g, planes_of(h), h->d_reactions, (int)h->reactions.size(),
-                                                     h->seed, (uint32_t)*seed, deltat, h->d_status, h->stream));
+                                                     h->net(), h->seed, (uint32_t)*seed, deltat, h->d_status, h->stream));
     (*seed)++;
     if (rc) return rc;
     // the individual species follow the new counts (Solver.cpp:240-247: one seed each)
@@ -936,7 +951,7 @@ int gpgmp_solver_autotune(gpgmp_solver* h, float window, int32_t reps, float* ms
             for (int k = 0; k < reps && e == cudaSuccess; ++k) {
                 e = restore();
                 if (e == cudaSuccess)
-                    e = time_it([&] { return launch_ssa(g, spare, h->d_reactions, nreac, h->seed, 7u, window, d_st,
+                    e = time_it([&] { return launch_ssa(g, spare, h->d_reactions, nreac, h->net(), h->seed, 7u, window, d_st,
                                                         h->stream); }, &ms);
                 total += ms;
             }

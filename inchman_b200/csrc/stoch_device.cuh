@@ -66,11 +66,10 @@ struct GatedHazard {
 };
 
 // Runs one SSA window on the counts x[s * stride]; returns a GPGMP_SIM_* bit or 0.
+// From time t and after `events` events where a window is continued.
 template <class HZ>
 __device__ __forceinline__ int ssa_cell_h(const gpgmp_reaction* rt, int R, int* x, int stride, Stream& st,
-                                          float window, const HZ& hz) {
-    float t = 0.0f;
-    int events = 0;
+                                          float window, const HZ& hz, float t = 0.0f, int events = 0) {
     for (;;) {
         float h0 = 0.0f;
         for (int r = 0; r < R; ++r) h0 = h0 + hz(rt, r, x, stride);
@@ -171,6 +170,199 @@ __device__ __forceinline__ int ssa_cell_inc(const gpgmp_reaction* rt, const uint
         }
         if (++events >= SSA_EVENT_CAP) return SIM_EVENT_CAP;
     }
+}
+
+// ---- packed networks -------------------------------------------------------------
+// A network whose reactions have at most two reactant molecules and change at most four
+// species (pack_network, netpack.h) runs its windows on float copies of the counts, which
+// are exact below 2^24.  Every hazard then is the same three operations, rate * x[s1] *
+// (x[s2] - sub): an absent reactant is slot 0, which holds 1 (the
+// products by 1 and the difference of 0 are exact; species s is slot s + 1), and 2A has s2 = s1, sub = 1, so the
+// values and their running sums are those of ssa_cell bit for bit.  No table of the
+// reaction structs is walked, nothing is converted per event and the sums are kept for the
+// selection instead of formed twice: A + B <-> C on 1M cells, a window of 1.7 events per
+// cell, 47 us instead of 78; predator and prey on 8.4M cells, 112 us instead of 171; 592
+// random networks of 8 to 32 reactions, 75 ms instead of 238.
+// A cell whose counts are negative or reach 2^24 goes on in ssa_slow, which keeps the
+// counts as integers in the same slots.
+struct PackedReaction {
+    float rate, sub;
+    int32_t s1, s2;      // slots of the reactants
+    uint32_t net[4];     // slot << 16 | upper half of the float change; unused: 0
+};
+constexpr float kPackedMax = 16777216.0f;
+
+// Where a window stands: time, events, the last draws and how many of them are used.
+struct SsaPos {
+    float t;
+    int events;
+    uint32_t w[4];
+    int used;
+};
+
+enum { SSA_SLOW = -1 };     // returned where the window has to go on in ssa_slow
+
+// the time of an event from its draw and the total hazard (a draw's logarithm is 0 or
+// between 2^-24 and 17 in size, so div_mid's range is the hazard's)
+__device__ __forceinline__ float ssa_wait(uint32_t draw, float h0) {
+    const float l = -log_draw(draw);
+    return h0 > 8.6736174e-19f && h0 < 1.1529215e18f ? div_mid(l, h0) : l / h0;
+}
+
+// applies one event's changes; true while every changed count stays below 2^24
+template <int STRIDE>
+__device__ __forceinline__ bool packed_apply(const uint4& n, int nnet, float* x) {
+    const uint32_t e[4] = {n.x, n.y, n.z, n.w};
+    float top = 0.0f;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        if (i < nnet) {
+            float* p = x + (e[i] >> 16) * STRIDE;
+            const float v = *p + __uint_as_float(e[i] << 16);
+            *p = v;
+            top = fmaxf(top, v);
+        }
+    }
+    return top < kPackedMax;
+}
+
+// One window of a network of NR reactions given by value (kernel parameters): the running
+// sums stay in registers.  nets: the changes of every reaction in shared memory.
+template <int NR>
+struct SmallNet {
+    float rate[NR], sub[NR];
+    int32_t s1[NR], s2[NR];
+    uint4 net[NR];
+    int32_t nnet;            // most species that one reaction changes
+};
+template <int NR, int STRIDE>
+__device__ __forceinline__ int ssa_small(const SmallNet<NR>& net, const uint4* nets, float* x, Stream& st,
+                                         float window, SsaPos& pos) {
+    pos.t = 0.0f;
+    pos.events = 0;
+    for (;;) {
+        st.block(pos.w);
+#pragma unroll
+        for (int half = 0; half < 2; ++half) {
+            float c[NR], h0 = 0.0f;
+#pragma unroll
+            for (int q = 0; q < NR; ++q) {
+                h0 = h0 + net.rate[q] * x[net.s1[q] * STRIDE] * (x[net.s2[q] * STRIDE] - net.sub[q]);
+                c[q] = h0;
+            }
+            if (!(h0 > 0.0f)) return 0;
+            const float r2 = u01(pos.w[2 * half + 1]) * h0;
+            pos.t = pos.t + ssa_wait(pos.w[2 * half], h0);
+            if (!(pos.t < window)) return 0;
+            int j = NR;
+#pragma unroll
+            for (int q = NR - 1; q >= 0; --q) j = r2 < c[q] ? q : j;
+            bool small = true;
+            if (j < NR) small = packed_apply<STRIDE>(nets[j], net.nnet, x);
+            if (++pos.events >= SSA_EVENT_CAP) return SIM_EVENT_CAP;
+            if (!small) {
+                pos.used = 2 * half + 2;
+                return SSA_SLOW;
+            }
+        }
+    }
+}
+
+// The same for a network in shared memory (ent: rate, sub, s1 * STRIDE, s2 * STRIDE as
+// bits), with the running sums in c[q * STRIDE]: they only grow, so the selection halves
+// its range instead of walking it.
+template <int STRIDE>
+__device__ __forceinline__ int ssa_packed(const float4* ent, const uint4* nets, int nnet, int R, float* x, float* c,
+                                          Stream& st, float window, SsaPos& pos) {
+    int top = 1;
+    while (2 * top <= R) top *= 2;
+    pos.t = 0.0f;
+    pos.events = 0;
+    pos.used = 4;
+    for (;;) {
+        if (pos.used == 4) {
+            st.block(pos.w);
+            pos.used = 0;
+        }
+        float h0 = 0.0f;
+#pragma unroll 4
+        for (int q = 0; q < R; ++q) {
+            const float4 e = ent[q];
+            h0 = h0 + e.x * x[__float_as_int(e.z)] * (x[__float_as_int(e.w)] - e.y);
+            c[q * STRIDE] = h0;
+        }
+        if (!(h0 > 0.0f)) return 0;
+        const uint32_t a = pos.used ? pos.w[2] : pos.w[0], b = pos.used ? pos.w[3] : pos.w[1];
+        pos.used += 2;
+        const float r2 = u01(b) * h0;
+        pos.t = pos.t + ssa_wait(a, h0);
+        if (!(pos.t < window)) return 0;
+        int j = 0;
+        for (int s = top; s > 0; s >>= 1)
+            if (j + s <= R && !(r2 < c[(j + s - 1) * STRIDE])) j += s;
+        bool small = true;
+        if (j < R) small = packed_apply<STRIDE>(nets[j], nnet, x);
+        if (++pos.events >= SSA_EVENT_CAP) return SIM_EVENT_CAP;
+        if (!small) return SSA_SLOW;
+    }
+}
+
+// The tables of ssa_packed in shared memory, by all threads of a block (which then syncs).
+template <int STRIDE>
+__device__ __forceinline__ void packed_tables(const PackedReaction* __restrict__ p, int R, float4* ent, uint4* nets) {
+    for (int q = threadIdx.x; q < R; q += blockDim.x) {
+        ent[q] = make_float4(p[q].rate, p[q].sub, __int_as_float(p[q].s1 * STRIDE), __int_as_float(p[q].s2 * STRIDE));
+        nets[q] = make_uint4(p[q].net[0], p[q].net[1], p[q].net[2], p[q].net[3]);
+    }
+}
+
+// The counts of one cell from memory (at(s): species s) into the float slots; false where
+// a count is outside the floats' exact range (the slots then hold the integers' bits).
+template <int STRIDE, class AT>
+__device__ __forceinline__ bool packed_load(const AT& at, int S, float* x) {
+    bool fits = true;
+    for (int s = 0; s < S; ++s) {
+        const int v = at(s);
+        fits = fits && (uint32_t)v < (1u << 24);
+        x[(s + 1) * STRIDE] = (float)v;
+    }
+    if (!fits)
+        for (int s = 0; s < S; ++s) x[(s + 1) * STRIDE] = __int_as_float(at(s));
+    x[0] = 1.0f;
+    return fits;
+}
+// The rest of a window on integer counts (the slots hold their bits).
+template <int STRIDE>
+__device__ __noinline__ int ssa_slow(const gpgmp_reaction* rt, int R, float* x, const Stream& from, float window,
+                                     const SsaPos& pos) {
+    Stream st = from;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) st.buf[i] = pos.w[i];
+    st.idx = pos.used;
+    return ssa_cell_h(rt, R, reinterpret_cast<int*>(x + STRIDE), STRIDE, st, window, MassActionHazard{}, pos.t, pos.events);
+}
+// One window of one cell: load, run (`run` is ssa_small or ssa_packed), store.  Returns a
+// GPGMP_SIM_* bit or 0.
+template <int STRIDE, class AT, class RUN>
+__device__ __forceinline__ int packed_window(const gpgmp_reaction* rt, int R, const AT& at, int S, float* x,
+                                             Stream& st, float window, const RUN& run) {
+    SsaPos pos;
+    int e = SSA_SLOW;
+    if (packed_load<STRIDE>(at, S, x)) {
+        e = run(x, st, pos);
+        if (e != SSA_SLOW) {
+            for (int s = 0; s < S; ++s) at(s) = (int)x[(s + 1) * STRIDE];
+            return e;
+        }
+        for (int s = 1; s <= S; ++s) x[s * STRIDE] = __int_as_float((int)x[s * STRIDE]);
+    } else {
+        pos.t = 0.0f;
+        pos.events = 0;
+        pos.used = 4;
+    }
+    e = ssa_slow<STRIDE>(rt, R, x, st, window, pos);
+    for (int s = 0; s < S; ++s) at(s) = __float_as_int(x[(s + 1) * STRIDE]);
+    return e;
 }
 
 // Four lost counts (-x, +x, -y, +y) of one cell of n particles.

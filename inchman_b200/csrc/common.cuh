@@ -249,7 +249,7 @@ __device__ __forceinline__ float gp_sinhf(float e) {
 // fused multiply-add and q0 + y (a - q0 b) rounds to a / b).  Checked against the
 // division for every significand of a and every b of the table; it holds while the
 // remainder does not underflow, |a| > 2^-100 (binomial_count says why that suffices).
-constexpr int kRecipMax = 64;
+constexpr int kRecipMax = 64, kRecipHead = 12;
 #define GPGMP_RECIP4(i) 1.0f / (i), 1.0f / (i + 1), 1.0f / (i + 2), 1.0f / (i + 3)
 #define GPGMP_RECIP16(i) GPGMP_RECIP4(i), GPGMP_RECIP4(i + 4), GPGMP_RECIP4(i + 8), GPGMP_RECIP4(i + 12)
 static __constant__ float kRecip[kRecipMax] = {GPGMP_RECIP16(1.0f), GPGMP_RECIP16(17.0f), GPGMP_RECIP16(33.0f),
@@ -287,16 +287,26 @@ __device__ __forceinline__ int binomial_count(float u, int m, float f, float r) 
     int k = 0;
     float cdf = f;
     if (m < (1 << 24)) {
-        float left = (float)m, next = 1.0f;
-        const int kmax = m < kRecipMax ? m : kRecipMax;
-#pragma unroll 8
-        for (; k < kRecipMax; ++k) {
-            if (!(u >= cdf && k < kmax)) break;
-            f = div_small(f * (left * r), next, kRecip[k]);
+        float left = (float)m;
+        // the first terms with their divisors as constants; past k = m the terms are zero,
+        // so the test for it waits until after
+#pragma unroll
+        for (; k < kRecipHead; ++k) {
+            if (u < cdf) break;
+            f = div_small(f * (left * r), (float)(k + 1), 1.0f / (float)(k + 1));
             left -= 1.0f;
-            next += 1.0f;
             cdf = cdf + f;
         }
+        if (k == kRecipHead && m > kRecipHead) {
+            const int kmax = m < kRecipMax ? m : kRecipMax;
+            for (; k < kmax; ++k) {
+                if (u < cdf) break;
+                f = div_small(f * (left * r), (float)(k + 1), kRecip[k]);
+                left -= 1.0f;
+                cdf = cdf + f;
+            }
+        }
+        k = k < m ? k : m;
     }
     while (u >= cdf && k < m) {
         f = f * ((float)(m - k) * r) / (float)(k + 1);
@@ -306,22 +316,57 @@ __device__ __forceinline__ int binomial_count(float u, int m, float f, float r) 
     return k;
 }
 
-__device__ __forceinline__ int binomial(Stream& st, int n, float p) {
-    if (n <= 0 || !(p > 0.0f)) return 0;
-    if (p >= 1.0f) return n;
-    const bool flip = p > 0.5f;
-    const float q = flip ? 1.0f - p : p;
-    const float r = q / (1.0f - q);
-    const float chunkf = 30.0f / q;
-    int chunk = chunkf >= 2147483520.0f ? INT_MAX : (int)chunkf;
-    if (chunk < 1) chunk = 1;
+// What a binomial draw needs from its probability p, worked out once where many draws
+// share it: q / (1 - q), the counts per draw for q = min(p, 1 - p), and (1 - q)^(2^i) for
+// the powers.
+template <int BITS>
+struct BinomialSetup {
+    float sq[BITS], r;
+    int chunk;
+    int kind;      // 0: none (p <= 0 or NaN), 1: p <= 1/2, 2: p > 1/2 (counts those left), 3: all (p >= 1)
+    __device__ __forceinline__ void init(float p) {
+        kind = !(p > 0.0f) ? 0 : p >= 1.0f ? 3 : p > 0.5f ? 2 : 1;
+        const float q = p > 0.5f ? 1.0f - p : p;
+        sq[0] = 1.0f - q;
+#pragma unroll
+        for (int i = 1; i < BITS; ++i) sq[i] = sq[i - 1] * sq[i - 1];
+        r = q / (1.0f - q);
+        const float chunkf = 30.0f / q;
+        chunk = chunkf >= 2147483520.0f ? INT_MAX : (int)chunkf;
+        if (chunk < 1) chunk = 1;
+    }
+    // (1 - q)^m, the products of pow_int
+    __device__ __forceinline__ float power(int m) const {
+        if (m >= (1 << BITS)) return pow_int(sq[0], m);
+        float f = (m & 1) ? sq[0] : 1.0f;
+#pragma unroll
+        for (int i = 1; i < BITS; ++i) f = f * ((m & (1 << i)) ? sq[i] : 1.0f);
+        return f;
+    }
+    // n from one draw: whether n needs at most one, and its count (n > 0, kind 1 or 2)
+    __device__ __forceinline__ bool single(int n) const { return n <= chunk && kind != 3; }
+    __device__ __forceinline__ int count(uint32_t draw, int n) const {
+        const int k = binomial_count(u01(draw), n, power(n), r);
+        return kind == 2 ? n - k : k;
+    }
+};
+template <int BITS>
+__device__ __forceinline__ int binomial(Stream& st, int n, const BinomialSetup<BITS>& b) {
+    if (n <= 0 || b.kind == 0) return 0;
+    if (b.kind == 3) return n;
     int rem = n, total = 0;
     while (rem > 0) {
-        const int m = rem < chunk ? rem : chunk;
-        total += binomial_count(u01(st.next()), m, pow_int(1.0f - q, m), r);
+        const int m = rem < b.chunk ? rem : b.chunk;
+        total += binomial_count(u01(st.next()), m, pow_int(b.sq[0], m), b.r);
         rem -= m;
     }
-    return flip ? n - total : total;
+    return b.kind == 2 ? n - total : total;
+}
+__device__ __forceinline__ int binomial(Stream& st, int n, float p) {
+    if (n <= 0 || !(p > 0.0f)) return 0;
+    BinomialSetup<1> b;
+    b.init(p);
+    return binomial(st, n, b);
 }
 
 // Unit-rate arrivals before lam: the logarithms of a block's four draws are independent,

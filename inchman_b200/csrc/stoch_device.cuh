@@ -231,7 +231,7 @@ __device__ __forceinline__ bool packed_apply(const uint4& n, int nnet, float* x)
 template <int NR>
 struct SmallNet {
     float rate[NR], sub[NR];
-    int32_t s1[NR], s2[NR];
+    int32_t o1[NR], o2[NR];  // slots of the reactants, times the threads of a block
     uint4 net[NR];
     int32_t nnet;            // most species that one reaction changes
 };
@@ -247,7 +247,7 @@ __device__ __forceinline__ int ssa_small(const SmallNet<NR>& net, const uint4* n
             float c[NR], h0 = 0.0f;
 #pragma unroll
             for (int q = 0; q < NR; ++q) {
-                h0 = h0 + net.rate[q] * x[net.s1[q] * STRIDE] * (x[net.s2[q] * STRIDE] - net.sub[q]);
+                h0 = h0 + net.rate[q] * x[net.o1[q]] * (x[net.o2[q]] - net.sub[q]);
                 c[q] = h0;
             }
             if (!(h0 > 0.0f)) return 0;
@@ -423,24 +423,51 @@ __device__ __forceinline__ void sweep_probs_fpe(float D, float r, float dt, floa
     *Pm = pm < 0.0f ? 0.0f : (pm > rest ? rest : pm);
 }
 
-// (minus, plus) counts of one cell for a directional sweep.
-__device__ __forceinline__ void sweep_lost(int n, float D, float r, float dt, float dx, Stream& st, bool at_lo,
-                                           bool at_hi, int mask_lo, int mask_hi, int* minus, int* plus,
-                                           bool fpe = false) {
-    float Pp, Pm;
-    if (fpe)
-        sweep_probs_fpe(D, r, dt, dx, &Pp, &Pm);
-    else
-        sweep_probs(D, r, dt, dx, &Pp, &Pm);
-    const float Pt = Pp + Pm;
-    const int moved = binomial(st, n, Pt);
-    int p = Pt > 0.0f ? binomial(st, moved, Pp / Pt) : 0;
-    int m = moved - p;
-    if (at_lo && mask_lo == 0) m = 0;
-    if (at_hi && mask_hi == 0) p = 0;
-    *minus = m;
-    *plus = p;
-}
+// A directional sweep of one cell: the draw of the moved particles and of those among them
+// that go towards +, set up once from the cell's fields; draw() takes one realisation's
+// count.
+struct SweepCell {
+    BinomialSetup<7> moved;
+    BinomialSetup<4> plus;
+    bool stay_lo, stay_hi;      // a reflecting wall below / above
+    __device__ __forceinline__ void init(float D, float r, float dt, float dx, bool lo, bool hi, bool fpe) {
+        float Pp, Pm;
+        if (fpe)
+            sweep_probs_fpe(D, r, dt, dx, &Pp, &Pm);
+        else
+            sweep_probs(D, r, dt, dx, &Pp, &Pm);
+        const float Pt = Pp + Pm;
+        moved.init(Pt);
+        plus.init(Pt > 0.0f ? Pp / Pt : 0.0f);
+        stay_lo = lo;
+        stay_hi = hi;
+    }
+    // (minus, plus) counts of n particles
+    __device__ __forceinline__ void draw(int n, Stream& st, int* minus, int* plus_out) const {
+        int k = 0, p = 0;
+        if (n > 0 && moved.kind != 0) {
+            Stream again = st;
+            uint32_t w[4];
+            st.block(w);
+            if (moved.single(n) && plus.kind != 3) {     // one draw each, but for large counts
+                k = moved.count(w[0], n);
+                if (k > 0 && plus.kind != 0) {
+                    if (k <= plus.chunk) {
+                        p = plus.count(w[1], k);
+                    } else {
+                        again.next();
+                        p = binomial(again, k, plus);
+                    }
+                }
+            } else {
+                k = binomial(again, n, moved);
+                p = binomial(again, k, plus);
+            }
+        }
+        *minus = stay_lo ? 0 : k - p;
+        *plus_out = stay_hi ? 0 : p;
+    }
+};
 
 // Evaluated in double; below |eps| = 1e-3 tanh and temp come from their series
 // (tanh eps = eps - eps^3/3, temp = 1/3 + 4 eps^2/45) because the closed form

@@ -15,7 +15,8 @@ namespace {
 constexpr int kIncMinReactions = 6;   // networks above this size keep per-reaction hazards
 constexpr int NT = 256;               // threads of a diffusion tile block
 
-// Launch shapes the autotuner chooses from (GridDesc::tile, GridDesc::ssa_threads):
+// Launch shapes the autotuner chooses from (GridDesc::tile, GridDesc::ssa_threads; the
+// drift-diffusion sweeps have one shape):
 // diffusion tiles of TW x TH cells for 256 threads (1, 2 or 4 cells per thread in the
 // gather; the one-cell halo is recomputed, so wider tiles recompute less), and SSA
 // blocks of 64, 128 or 256 threads (one cell per thread).  Every draw is keyed by its
@@ -24,11 +25,35 @@ constexpr int kTileW[kNumDiffusionTiles] = {32, 32, 64, 16, 64, 32};
 constexpr int kTileH[kNumDiffusionTiles] = {16, 8, 8, 16, 16, 32};
 constexpr int kSsaThreadChoices[kNumSsaThreadChoices] = {128, 64, 256};
 
-__global__ void k_init_poisson(Planes planes, int S, int area, int R, uint32_t seed, const float* __restrict__ lam) {
+// n / d for n < 2^31 by one multiplication: with s = ceil(log2 d) and m = ceil(2^(31+s) / d)
+// < 2^32 the error of m is below 2^s, so n m / 2^(31+s) exceeds n / d by less than 1 / d
+// (Granlund & Montgomery 1994).
+struct FastDiv {
+    uint32_t d, m;
+    int s;
+    __host__ explicit FastDiv(uint32_t div) : d(div), m(0), s(0) {
+        while ((1ull << s) < d) ++s;
+        m = (uint32_t)((((1ull << 31) << s) + d - 1) / d);
+    }
+    __device__ __forceinline__ uint32_t operator()(uint32_t n) const {
+        return (uint32_t)(((uint64_t)n * m) >> (31 + s));
+    }
+};
+
+// realisation and cell of index i of all the cells (a 64-bit division costs as much as a
+// random block, so it is left to totals of 2^31 cells and more)
+__device__ __forceinline__ void split_cell(int64_t i, int64_t total, const FastDiv& area, int* r, int* c) {
+    *r = total < ((int64_t)1 << 31) ? (int)area((uint32_t)i) : (int)(i / area.d);
+    *c = (int)(i - (int64_t)*r * area.d);
+}
+
+__global__ void k_init_poisson(Planes planes, int S, FastDiv area_div, int R, uint32_t seed,
+                               const float* __restrict__ lam) {
+    const int area = (int)area_div.d;
     const int64_t total = (int64_t)R * area;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
-        const int r = (int)(i / area);
-        const int c = (int)(i - (int64_t)r * area);
+        int r, c;
+        split_cell(i, total, area_div, &r, &c);
         for (int s = 0; s < S; ++s) {
             Stream st;
             st.init(seed, (uint32_t)r, 0u, (uint32_t)c, PH_INIT | ((uint32_t)s << 8));
@@ -81,7 +106,7 @@ __global__ void __launch_bounds__(kSsaThreads) k_ssa(Planes planes, int S, int a
 // The same windows for a network in the packed form: NR reactions as kernel parameters,
 // their running sums in registers (ssa_small), or any number in shared memory (ssa_packed).
 template <int NR, int kSsaThreads>
-__global__ void __launch_bounds__(kSsaThreads) k_ssa_small(Planes planes, int S, int area, int R,
+__global__ void __launch_bounds__(kSsaThreads) k_ssa_small(Planes planes, int S, FastDiv area_div, int R,
                                                            const gpgmp_reaction* __restrict__ reactions,
                                                            const __grid_constant__ SmallNet<NR> net, uint32_t seed,
                                                            uint32_t step_seed, float window,
@@ -91,10 +116,13 @@ __global__ void __launch_bounds__(kSsaThreads) k_ssa_small(Planes planes, int S,
     if (threadIdx.x < NR) s_net[threadIdx.x] = net.net[threadIdx.x];
     __syncthreads();
     const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (i >= (int64_t)R * area) return;
-    const int r = (int)(i / area);
-    const int c = (int)(i - (int64_t)r * area);
-    const auto at = [&](int s) -> int32_t& { return planes.p[s][((int64_t)r * S + s) * area + c]; };
+    const int area = (int)area_div.d;
+    const int64_t total = (int64_t)R * area;
+    if (i >= total) return;
+    int r, c;
+    split_cell(i, total, area_div, &r, &c);
+    const int64_t first = (int64_t)r * S * area + c;
+    const auto at = [&](int s) -> int32_t& { return planes.p[s][first + (int64_t)s * area]; };
     Stream st;
     st.init(seed, (uint32_t)r, step_seed, (uint32_t)c, PH_SSA);
     const int e = packed_window<kSsaThreads>(
@@ -104,7 +132,7 @@ __global__ void __launch_bounds__(kSsaThreads) k_ssa_small(Planes planes, int S,
 }
 
 template <int kSsaThreads>
-__global__ void __launch_bounds__(kSsaThreads) k_ssa_packed(Planes planes, int S, int area, int R,
+__global__ void __launch_bounds__(kSsaThreads) k_ssa_packed(Planes planes, int S, FastDiv area_div, int R,
                                                             const gpgmp_reaction* __restrict__ reactions, int nreac,
                                                             const PackedReaction* __restrict__ packed, int nnet,
                                                             uint32_t seed, uint32_t step_seed, float window,
@@ -117,10 +145,13 @@ __global__ void __launch_bounds__(kSsaThreads) k_ssa_packed(Planes planes, int S
     packed_tables<kSsaThreads>(packed, nreac, ent, nets);
     __syncthreads();
     const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (i >= (int64_t)R * area) return;
-    const int r = (int)(i / area);
-    const int c = (int)(i - (int64_t)r * area);
-    const auto at = [&](int s) -> int32_t& { return planes.p[s][((int64_t)r * S + s) * area + c]; };
+    const int area = (int)area_div.d;
+    const int64_t total = (int64_t)R * area;
+    if (i >= total) return;
+    int r, c;
+    split_cell(i, total, area_div, &r, &c);
+    const int64_t first = (int64_t)r * S * area + c;
+    const auto at = [&](int s) -> int32_t& { return planes.p[s][first + (int64_t)s * area]; };
     Stream st;
     st.init(seed, (uint32_t)r, step_seed, (uint32_t)c, PH_SSA);
     const int e = packed_window<kSsaThreads>(
@@ -130,75 +161,132 @@ __global__ void __launch_bounds__(kSsaThreads) k_ssa_packed(Planes planes, int S
     if (e) atomicOr(&status[r], e);
 }
 
-// MODE 0: 2-D homogeneous jumps; 1: drift-diffusion sweep in x; 2: sweep in y.
-// A block owns a TW x TH tile, samples the lost counts of the tile and of its
-// one-cell halo (recomputed, the streams are keyed by cell) into shared memory,
+// 2-D homogeneous jumps.  A block owns a TW x TH tile, samples the lost counts of the tile
+// and of its one-cell halo (recomputed, the streams are keyed by cell) into shared memory,
 // then gathers.  Reads `in`, writes `out`: no block reads what another writes.
-template <int MODE, int TW, int TH>
+template <int TW, int TH>
 __global__ void __launch_bounds__(NT) k_diffuse_tile(const int* __restrict__ in, int* __restrict__ out, int W, int H,
                                                      int S, int species, uint32_t seed, uint32_t step_seed,
-                                                     float pmove, int4 bm4, const float* __restrict__ Df,
-                                                     const float* __restrict__ rf, float dt, float dx, int fpe) {
-    constexpr int HX = (MODE == 2) ? 0 : 1;
-    constexpr int HY = (MODE == 1) ? 0 : 1;
-    constexpr int RW = TW + 2 * HX, RH = TH + 2 * HY;
-    constexpr int NL = (MODE == 0) ? 4 : 2;
-    __shared__ int s_lost[RH * RW * NL];
+                                                     float pmove, int4 bm4) {
+    constexpr int RW = TW + 2, RH = TH + 2;
+    __shared__ int s_lost[RH * RW * 4];
     __shared__ int s_n[TH * TW];
     const int area = W * H;
     const int r = blockIdx.z;
     const int x0 = blockIdx.x * TW, y0 = blockIdx.y * TH;
     const int64_t plane = ((int64_t)r * S + species) * area;
     const int bm[4] = {bm4.x, bm4.y, bm4.z, bm4.w};
-    const uint32_t phase = PH_DIFF | ((uint32_t)species << 8) | (uint32_t)MODE;
+    const uint32_t phase = PH_DIFF | ((uint32_t)species << 8);
     for (int i = threadIdx.x; i < RW * RH; i += NT) {
         const int lx = i % RW, ly = i / RW;
-        const int gx = x0 + lx - HX, gy = y0 + ly - HY;
+        const int gx = x0 + lx - 1, gy = y0 + ly - 1;
         int l[4] = {0, 0, 0, 0};
         if (gx >= 0 && gx < W && gy >= 0 && gy < H) {
             const int c = gy * W + gx;
             const int n = in[plane + c];
             Stream st;
             st.init(seed, (uint32_t)r, step_seed, (uint32_t)c, phase);
-            if (MODE == 0) {
-                homog_lost(n, pmove, st, gx, gy, W, H, bm, l);
-            } else if (MODE == 1) {
-                const int64_t fi = (int64_t)species * area + c;
-                sweep_lost(n, Df[fi], rf[fi], dt, dx, st, gx == 0, gx == W - 1, bm[0], bm[1], &l[0], &l[1],
-                           fpe != 0);
-            } else {
-                const int64_t fi = (int64_t)species * area + c;
-                sweep_lost(n, Df[fi], rf[fi], dt, dx, st, gy == 0, gy == H - 1, bm[2], bm[3], &l[0], &l[1],
-                           fpe != 0);
-            }
-            if (lx >= HX && lx < HX + TW && ly >= HY && ly < HY + TH) s_n[(ly - HY) * TW + (lx - HX)] = n;
+            homog_lost(n, pmove, st, gx, gy, W, H, bm, l);
+            if (lx >= 1 && lx < 1 + TW && ly >= 1 && ly < 1 + TH) s_n[(ly - 1) * TW + (lx - 1)] = n;
         }
 #pragma unroll
-        for (int d = 0; d < NL; ++d) s_lost[i * NL + d] = l[d];
+        for (int d = 0; d < 4; ++d) s_lost[i * 4 + d] = l[d];
     }
     __syncthreads();
     for (int i = threadIdx.x; i < TW * TH; i += NT) {
         const int lx = i % TW, ly = i / TW;
         const int gx = x0 + lx, gy = y0 + ly;
         if (gx >= W || gy >= H) continue;
-        const int o = (ly + HY) * RW + (lx + HX);
+        const int o = (ly + 1) * RW + (lx + 1);
         int v = s_n[i];
-        if (MODE == 0) {
-            v -= s_lost[o * 4] + s_lost[o * 4 + 1] + s_lost[o * 4 + 2] + s_lost[o * 4 + 3];
-            if (gx > 0) v += s_lost[(o - 1) * 4 + 1];
-            if (gx < W - 1) v += s_lost[(o + 1) * 4 + 0];
-            if (gy > 0) v += s_lost[(o - RW) * 4 + 3];
-            if (gy < H - 1) v += s_lost[(o + RW) * 4 + 2];
-        } else if (MODE == 1) {
-            v -= s_lost[o * 2] + s_lost[o * 2 + 1];
-            if (gx > 0) v += s_lost[(o - 1) * 2 + 1];
-            if (gx < W - 1) v += s_lost[(o + 1) * 2];
-        } else {
-            v -= s_lost[o * 2] + s_lost[o * 2 + 1];
-            if (gy > 0) v += s_lost[(o - RW) * 2 + 1];
-            if (gy < H - 1) v += s_lost[(o + RW) * 2];
-        }
+        v -= s_lost[o * 4] + s_lost[o * 4 + 1] + s_lost[o * 4 + 2] + s_lost[o * 4 + 3];
+        if (gx > 0) v += s_lost[(o - 1) * 4 + 1];
+        if (gx < W - 1) v += s_lost[(o + 1) * 4 + 0];
+        if (gy > 0) v += s_lost[(o - RW) * 4 + 3];
+        if (gy < H - 1) v += s_lost[(o + RW) * 4 + 2];
         out[plane + gy * W + gx] = v;
+    }
+}
+
+// Drift-diffusion sweep in x (DIR 0) or y (DIR 1), written out of place.  A thread owns one
+// cell of a 32 x 8 (x) or 8 x 32 (y) tile, works out its probabilities and draw set-ups
+// once and samples it in up to kSweepReal realisations; the tile is 32 cells long in the
+// sweep's direction so that its 16 halo cells, sampled again here, are 1/16 of the work,
+// and one barrier serves all the realisations.  Issue slots bound it (the random block and
+// the two searches), not its 8 bytes per cell:
+// 8.4M cells 140 us (67 MB; 198 us with one realisation and one set-up per cell and tile,
+// whose quarter-tile of halo rows was sampled again).
+constexpr int kSweepReal = 8;
+template <int DIR>
+__global__ void __launch_bounds__(NT, 4) k_sweep(const int* __restrict__ in, int* __restrict__ out, int W, int H, int S,
+                                              int R, int species, uint32_t seed, uint32_t step_seed, int wall_lo,
+                                              int wall_hi, const float* __restrict__ Df, const float* __restrict__ rf,
+                                              float dt, float dx, int fpe) {
+    constexpr int TW = DIR == 0 ? 32 : 8, TH = DIR == 0 ? 8 : 32;
+    constexpr int LINE = 34;                       // cells along the sweep with both halo cells
+    constexpr int STEP = DIR == 0 ? 1 : TW;        // to the next cell along the sweep
+    constexpr int CELLS = LINE * 8;
+    static_assert(TW * TH == NT && CELLS == NT + 16, "a thread per cell and 16 halo cells");
+    __shared__ int s_minus[kSweepReal][CELLS], s_plus[kSweepReal][CELLS], s_kept[kSweepReal][NT];
+    const int64_t area = (int64_t)W * H;
+    const int r0 = blockIdx.z * kSweepReal;
+    const int nr = min(kSweepReal, R - r0);
+    const int x0 = blockIdx.x * TW, y0 = blockIdx.y * TH;
+    const uint32_t phase = PH_DIFF | ((uint32_t)species << 8) | (uint32_t)(DIR + 1);
+    const int64_t plane0 = ((int64_t)r0 * S + species) * area, plane_step = (int64_t)S * area;
+    const auto set_up = [&](SweepCell& cell, int gx, int gy) {
+        const int64_t fi = (int64_t)species * area + (int64_t)gy * W + gx;
+        const int p = DIR == 0 ? gx : gy, last = (DIR == 0 ? W : H) - 1;
+        cell.init(Df[fi], rf[fi], dt, dx, p == 0 && wall_lo == 0, p == last && wall_hi == 0, fpe != 0);
+    };
+    // the halo: cell i & 1 ? after : before the tile's line i >> 1, of realisation h >> 4
+    for (int h = threadIdx.x; h < 16 * nr; h += NT) {
+        const int i = h & 15, k = h >> 4, line = i >> 1, after = i & 1;
+        const int gx = x0 + (DIR == 0 ? (after ? TW : -1) : line);
+        const int gy = y0 + (DIR == 0 ? line : (after ? TH : -1));
+        int minus = 0, plus = 0;
+        if (gx >= 0 && gx < W && gy >= 0 && gy < H) {
+            SweepCell cell;
+            set_up(cell, gx, gy);
+            const int c = gy * W + gx;
+            Stream st;
+            st.init(seed, (uint32_t)(r0 + k), step_seed, (uint32_t)c, phase);
+            cell.draw(in[plane0 + k * plane_step + c], st, &minus, &plus);
+        }
+        const int o = DIR == 0 ? line * LINE + (after ? TW + 1 : 0) : (after ? TH + 1 : 0) * TW + line;
+        s_minus[k][o] = minus;
+        s_plus[k][o] = plus;
+    }
+    const int lx = threadIdx.x % TW, ly = threadIdx.x / TW;
+    const int gx = x0 + lx, gy = y0 + ly;
+    const int o = DIR == 0 ? ly * LINE + lx + 1 : (ly + 1) * TW + lx;
+    const bool own = gx < W && gy < H;
+    const int c = gy * W + gx;
+    if (own) {
+        SweepCell cell;
+        set_up(cell, gx, gy);
+        int next = in[plane0 + c];
+#pragma unroll 1
+        for (int k = 0; k < nr; ++k) {
+            const int n = next;
+            if (k + 1 < nr) next = in[plane0 + (k + 1) * plane_step + c];
+            Stream st;
+            st.init(seed, (uint32_t)(r0 + k), step_seed, (uint32_t)c, phase);
+            int minus, plus;
+            cell.draw(n, st, &minus, &plus);
+            s_minus[k][o] = minus;
+            s_plus[k][o] = plus;
+            s_kept[k][threadIdx.x] = n - minus - plus;
+        }
+    }
+    __syncthreads();
+    if (!own) return;
+    const int p = DIR == 0 ? gx : gy, last = (DIR == 0 ? W : H) - 1;
+    for (int k = 0; k < nr; ++k) {
+        int v = s_kept[k][threadIdx.x];
+        if (p > 0) v += s_plus[k][o - STEP];
+        if (p < last) v += s_minus[k][o + STEP];
+        out[plane0 + k * plane_step + c] = v;
     }
 }
 
@@ -553,7 +641,7 @@ inline unsigned grid_for(int64_t n, int threads) {
 cudaError_t launch_init_poisson(const GridDesc& g, Planes planes, uint32_t seed, const float* d_lambda,
                                 cudaStream_t st) {
     const int area = g.W * g.H;
-    k_init_poisson<<<grid_for((int64_t)g.R * area, 256), 256, 0, st>>>(planes, g.S, area, g.R, seed, d_lambda);
+    k_init_poisson<<<grid_for((int64_t)g.R * area, 256), 256, 0, st>>>(planes, g.S, FastDiv(area), g.R, seed, d_lambda);
     return cudaGetLastError();
 }
 
@@ -574,14 +662,14 @@ cudaError_t launch_ssa_small(const GridDesc& g, Planes planes, const gpgmp_react
         const PackedReaction& p = net.host[q];
         sn.rate[q] = p.rate;
         sn.sub[q] = p.sub;
-        sn.s1[q] = p.s1;
-        sn.s2[q] = p.s2;
+        sn.o1[q] = p.s1 * NTH;
+        sn.o2[q] = p.s2 * NTH;
         sn.net[q] = make_uint4(p.net[0], p.net[1], p.net[2], p.net[3]);
     }
     sn.nnet = net.nnet;
     const size_t smem = sizeof(float) * (g.S + 1) * NTH;
     k_ssa_small<NR, NTH><<<(unsigned)((total + NTH - 1) / NTH), NTH, smem, st>>>(
-        planes, g.S, area, g.R, d_reactions, sn, seed, step_seed, window, d_status);
+        planes, g.S, FastDiv(area), g.R, d_reactions, sn, seed, step_seed, window, d_status);
     return cudaGetLastError();
 }
 // The packed form where the network has one and every reaction is on everywhere; the
@@ -614,7 +702,7 @@ cudaError_t launch_ssa_t(const GridDesc& g, Planes planes, const gpgmp_reaction*
                                 sizeof(float) * (g.S + 1) * NTH;
             cudaError_t e = allow_smem(k_ssa_packed<NTH>, smem);
             if (e != cudaSuccess) return e;
-            k_ssa_packed<NTH><<<blocks, NTH, smem, st>>>(planes, g.S, area, g.R, d_reactions, nreac, net.dev, net.nnet,
+            k_ssa_packed<NTH><<<blocks, NTH, smem, st>>>(planes, g.S, FastDiv(area), g.R, d_reactions, nreac, net.dev, net.nnet,
                                                          seed, step_seed, window, d_status);
             return cudaGetLastError();
         }
@@ -640,33 +728,24 @@ cudaError_t launch_ssa_m(const GridDesc& g, Planes planes, const gpgmp_reaction*
 #undef GPGMP_SSA
 }
 
-template <int MODE, int TW, int TH>
+template <int TW, int TH>
 cudaError_t launch_tile_t(const GridDesc& g, const int32_t* in, int32_t* out, int species, uint32_t seed,
-                          uint32_t step_seed, float pmove, const float* d_D, const float* d_r, float dt, float dx,
-                          int fpe, cudaStream_t st) {
+                          uint32_t step_seed, float pmove, cudaStream_t st) {
     dim3 grid((g.W + TW - 1) / TW, (g.H + TH - 1) / TH, g.R);
     const int4 bm = make_int4(g.bmask[0], g.bmask[1], g.bmask[2], g.bmask[3]);
-    k_diffuse_tile<MODE, TW, TH><<<grid, NT, 0, st>>>(in, out, g.W, g.H, g.S, species, seed, step_seed, pmove, bm,
-                                                      d_D, d_r, dt, dx, fpe);
+    k_diffuse_tile<TW, TH><<<grid, NT, 0, st>>>(in, out, g.W, g.H, g.S, species, seed, step_seed, pmove, bm);
     return cudaGetLastError();
 }
-template <int MODE>
-cudaError_t launch_tile(const GridDesc& g, const int32_t* in, int32_t* out, int species, uint32_t seed,
-                        uint32_t step_seed, float pmove, const float* d_D, const float* d_r, float dt, float dx,
-                        int fpe, cudaStream_t st) {
-#define GPGMP_TILE(I)                                                                                              \
-    case I:                                                                                                        \
-        return launch_tile_t<MODE, kTileW[I], kTileH[I]>(g, in, out, species, seed, step_seed, pmove, d_D, d_r, dt, \
-                                                          dx, fpe, st);
-    switch (g.tile) {
-        GPGMP_TILE(1)
-        GPGMP_TILE(2)
-        GPGMP_TILE(3)
-        GPGMP_TILE(4)
-        GPGMP_TILE(5)
-        default: GPGMP_TILE(0)
-    }
-#undef GPGMP_TILE
+
+template <int DIR>
+cudaError_t launch_sweep_t(const GridDesc& g, const int32_t* in, int32_t* out, int species, uint32_t seed,
+                           uint32_t step_seed, const float* d_D, const float* d_r, float dt, float dx, int fpe,
+                           cudaStream_t st) {
+    constexpr int TW = DIR == 0 ? 32 : 8, TH = DIR == 0 ? 8 : 32;
+    dim3 grid((g.W + TW - 1) / TW, (g.H + TH - 1) / TH, (g.R + kSweepReal - 1) / kSweepReal);
+    k_sweep<DIR><<<grid, NT, 0, st>>>(in, out, g.W, g.H, g.S, g.R, species, seed, step_seed, g.bmask[2 * DIR],
+                                      g.bmask[2 * DIR + 1], d_D, d_r, dt, dx, fpe);
+    return cudaGetLastError();
 }
 }  // namespace
 
@@ -686,7 +765,18 @@ cudaError_t launch_ssa(const GridDesc& g, Planes planes, const gpgmp_reaction* d
 
 cudaError_t launch_homog_diffuse(const GridDesc& g, const int32_t* in, int32_t* out, int species, uint32_t seed,
                                  uint32_t step_seed, float pmove, cudaStream_t st) {
-    return launch_tile<0>(g, in, out, species, seed, step_seed, pmove, nullptr, nullptr, 0.f, 0.f, 0, st);
+#define GPGMP_TILE(I)                                                                                         \
+    case I:                                                                                                   \
+        return launch_tile_t<kTileW[I], kTileH[I]>(g, in, out, species, seed, step_seed, pmove, st);
+    switch (g.tile) {
+        GPGMP_TILE(1)
+        GPGMP_TILE(2)
+        GPGMP_TILE(3)
+        GPGMP_TILE(4)
+        GPGMP_TILE(5)
+        default: GPGMP_TILE(0)
+    }
+#undef GPGMP_TILE
 }
 
 cudaError_t launch_source(const GridDesc& g, int32_t* plane_base, int species, uint32_t seed, uint32_t step_seed,
@@ -699,8 +789,8 @@ cudaError_t launch_source(const GridDesc& g, int32_t* plane_base, int species, u
 cudaError_t launch_sweep(const GridDesc& g, const int32_t* in, int32_t* out, int species, int sweep_y,
                          uint32_t seed, uint32_t step_seed, const float* d_D, const float* d_r, float dt, float dx,
                          cudaStream_t st, int fpe) {
-    return sweep_y ? launch_tile<2>(g, in, out, species, seed, step_seed, 0.f, d_D, d_r, dt, dx, fpe, st)
-                   : launch_tile<1>(g, in, out, species, seed, step_seed, 0.f, d_D, d_r, dt, dx, fpe, st);
+    return sweep_y ? launch_sweep_t<1>(g, in, out, species, seed, step_seed, d_D, d_r, dt, dx, fpe, st)
+                   : launch_sweep_t<0>(g, in, out, species, seed, step_seed, d_D, d_r, dt, dx, fpe, st);
 }
 
 cudaError_t launch_det_sweep(const GridDesc& g, const float* in, float* out, int species, int sweep_y,

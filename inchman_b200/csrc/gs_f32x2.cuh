@@ -38,25 +38,38 @@ struct GSCoef2 {
     }
 };
 
-// forward update of two cells at once: C the cells, L / R / U / D their left,
-// right, upper and lower neighbours (any pairing of cells; the arithmetic per cell
-// is the same as in the scalar kernels' gs_update).  DRIFT: 1 with the drift
+// forward update of two cells at once: C the cells, U / D their upper and lower
+// neighbours, h the sums and d (with drift) the differences of their left and right ones
+// (any pairing of cells; the arithmetic per cell is the same as in the scalar kernels'
+// gs_update).  DRIFT: 1 with the drift
 // terms, 0 without, -1 decided by k.drift at run time.
+template <int DRIFT>
+__device__ __forceinline__ void gs_update2s(const GSCoef2& k, float2 uh, float2 ud, float2 uU, float2 uC, float2 uD,
+                                            float2 vh, float2 vd, float2 vU, float2 vC, float2 vD, float2* un,
+                                            float2* vn) {
+    const float2 uvv = mul2(uC, mul2(vC, vC));
+    const float2 lu = fma2(k.m4, uC, add2(uh, add2(uU, uD)));
+    const float2 lv = fma2(k.m4, vC, add2(vh, add2(vU, vD)));
+    float2 a = fma2(k.du, lu, fma2(k.mdtF, uC, k.dtF));
+    float2 b = fma2(k.mdtFk, vC, mul2(k.dv, lv));
+    if (DRIFT == 1 || (DRIFT < 0 && k.drift)) {
+        a = fma2(k.hx, ud, fma2(k.hy, sub2(uU, uD), a));
+        b = fma2(k.hx, vd, fma2(k.hy, sub2(vU, vD), b));
+    }
+    *un = add2(uC, fma2(k.mdt, uvv, a));
+    *vn = add2(vC, fma2(k.dt, uvv, b));
+}
+// the same from the left and right neighbours
 template <int DRIFT = -1>
 __device__ __forceinline__ void gs_update2f(const GSCoef2& k, float2 uL, float2 uR, float2 uU, float2 uC, float2 uD,
                                             float2 vL, float2 vR, float2 vU, float2 vC, float2 vD, float2* un,
                                             float2* vn) {
-    const float2 uvv = mul2(uC, mul2(vC, vC));
-    const float2 lu = fma2(k.m4, uC, add2(add2(uL, uR), add2(uU, uD)));
-    const float2 lv = fma2(k.m4, vC, add2(add2(vL, vR), add2(vU, vD)));
-    float2 a = fma2(k.du, lu, fma2(k.mdtF, uC, k.dtF));
-    float2 b = fma2(k.mdtFk, vC, mul2(k.dv, lv));
+    float2 ud = uL, vd = vL;
     if (DRIFT == 1 || (DRIFT < 0 && k.drift)) {
-        a = fma2(k.hx, sub2(uL, uR), fma2(k.hy, sub2(uU, uD), a));
-        b = fma2(k.hx, sub2(vL, vR), fma2(k.hy, sub2(vU, vD), b));
+        ud = sub2(uL, uR);
+        vd = sub2(vL, vR);
     }
-    *un = add2(uC, fma2(k.mdt, uvv, a));
-    *vn = add2(vC, fma2(k.dt, uvv, b));
+    gs_update2s<DRIFT>(k, add2(uL, uR), ud, uU, uC, uD, add2(vL, vR), vd, vU, vC, vD, un, vn);
 }
 
 // forward update of the adjacent pair C = (x, x+1), L = (x-1, x), R = (x+1, x+2)

@@ -527,6 +527,7 @@ __global__ void __launch_bounds__(512, 1) k_gs_adjoint_cw(GSArgs<T> a, const T* 
 
 #include "gs_f32x2.cuh"
 #include "gs_rr.cuh"
+#include "gs_rb.cuh"
 #include "gs_mc.cuh"
 
 // register-resident forward kernel for an n x n float32 lattice with *wpc warps per
@@ -544,6 +545,74 @@ const void* rr_kernel(int n, int* wpc, bool drift, size_t* smem) {
     GS_RR_CASE(256, 4) GS_RR_CASE(256, 8) GS_RR_CASE(256, 16)
 #undef GS_RR_CASE
     return nullptr;
+}
+
+// Kernels of the batched forward: the 16-CTA clusters of gs_rr.cuh (wpc 0: its default
+// split) and the row blocks of gs_rb.cuh on smaller clusters.  at_once: clusters of that
+// size with one CTA per SM (the GPCs' SM counts leave 8 clusters of 16, 15 of 8, 33 of 4);
+// lat: us per step with at most one CTA on an SM, each: us per step for every further CTA
+// an SM holds, both measured without drift.  A batch takes the kernel whose step
+// max(lat, each * CTAs per SM) is the shortest: large clusters while SMs are idle (lat falls
+// with the cluster's size), whole lattices on an SM once they are not (each, per lattice,
+// falls with the rows per CTA).  us per step, before -> now: 64^2 x 256 1.57 -> 0.97,
+// 128^2 x 64 1.44 -> 0.87, 128^2 x 148 3.04 -> 1.59, 256^2 x 24 2.80 -> 1.54.
+struct RBConfig {
+    int n, cl, wpc, at_once;
+    float lat, each;
+    const void* k[2];      // without / with drift
+    uint32_t smem;
+};
+template <int N, int CL, int W>
+RBConfig rb_config(int at_once, float lat, float each) {
+    return {N, CL, W, at_once, lat, each,
+            {(const void*)k_gs_forward_rb<N, CL, W, 0>, (const void*)k_gs_forward_rb<N, CL, W, 1>},
+            RBShape<N, CL, W>::kSmem};
+}
+constexpr int kRBConfigs = 12;
+const RBConfig& rb_table(int i) {
+    static const RBConfig t[kRBConfigs] = {
+        {64, kRRCluster, 0, 8, 0.28f, 0.065f, {nullptr, nullptr}, 0},
+        rb_config<64, 4, 8>(33, 0.32f, 0.21f),
+        rb_config<64, 2, 8>(74, 0.42f, 0.28f),
+        rb_config<64, 1, 16>(148, 0.55f, 0.505f),
+        rb_config<64, 1, 8>(148, 0.62f, 0.485f),
+        {128, kRRCluster, 0, 8, 0.36f, 0.22f, {nullptr, nullptr}, 0},
+        rb_config<128, 8, 8>(15, 0.41f, 0.25f),
+        rb_config<128, 2, 16>(74, 0.86f, 0.84f),
+        rb_config<128, 1, 16>(148, 1.59f, 1.59f),
+        {256, kRRCluster, 0, 7, 0.74f, 0.70f, {nullptr, nullptr}, 0},
+        rb_config<256, 8, 16>(15, 1.07f, 1.04f),
+        rb_config<256, 4, 16>(33, 1.54f, 1.52f)};
+    return t[i];
+}
+// the kernel for `batch` lattices of side n, or nullptr: the 16-CTA clusters
+const RBConfig* rb_choose(int n, int batch) {
+    const RBConfig* best = nullptr;
+    float t = 0.f;
+    for (int i = 0; i < kRBConfigs; ++i) {
+        const RBConfig& m = rb_table(i);
+        if (m.n != n) continue;
+        const float ti = std::max(m.lat, m.each * (float)((batch + m.at_once - 1) / m.at_once));
+        if (!best || ti < t) {
+            best = &m;
+            t = ti;
+        }
+    }
+    return best && best->wpc ? best : nullptr;
+}
+void rb_launch_config(const RBConfig& m, int batch, cudaLaunchConfig_t* cfg, cudaLaunchAttribute* attr,
+                      cudaStream_t st) {
+    *cfg = {};
+    cfg->gridDim = dim3(m.cl * batch, 1, 1);
+    cfg->blockDim = dim3(32 * m.wpc, 1, 1);
+    cfg->dynamicSmemBytes = m.smem;
+    cfg->stream = st;
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = m.cl;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg->attrs = attr;
+    cfg->numAttrs = 1;
 }
 
 // Multi-cluster forward kernels (gs_mc.cuh): variant 40 + index.  Each spreads one
@@ -876,6 +945,7 @@ cudaError_t gs_forward_batch_f32(const GSParams& p, int batch, const GSBatchMemb
     int wpc = p.variant > 10 && p.variant < kMCVariant ? p.variant - 10 : 0;   // one lattice per cluster
     const void* rk = rr_kernel(p.n, &wpc, drift, &smem);
     if (!rk) return cudaErrorInvalidValue;
+    const RBConfig* rb = p.variant == 0 ? rb_choose(p.n, batch) : nullptr;
     GSArgs<float>* d = nullptr;
     cudaError_t e = pool_alloc((void**)&d, sizeof(GSArgs<float>) * batch, st);
     if (e != cudaSuccess) return e;
@@ -885,22 +955,30 @@ cudaError_t gs_forward_batch_f32(const GSParams& p, int batch, const GSBatchMemb
         float* no_trace = nullptr;
         int every = 1;
         void* args[] = {&a, (void*)&u0, (void*)&v0, &u, &v, &no_trace, &every, &d};
-        e = cudaFuncSetAttribute(rk, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(rk, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-        if (e == cudaSuccess) {
-            cudaLaunchConfig_t cfg = {};
-            cfg.gridDim = dim3(kRRCluster * batch, 1, 1);
-            cfg.blockDim = dim3(32 * wpc, 1, 1);
-            cfg.dynamicSmemBytes = smem;
-            cfg.stream = st;
-            cudaLaunchAttribute attr[1];
-            attr[0].id = cudaLaunchAttributeClusterDimension;
-            attr[0].val.clusterDim.x = kRRCluster;
-            attr[0].val.clusterDim.y = 1;
-            attr[0].val.clusterDim.z = 1;
-            cfg.attrs = attr;
-            cfg.numAttrs = 1;
-            e = cudaLaunchKernelExC(&cfg, rk, args);
+        cudaLaunchConfig_t cfg = {};
+        cudaLaunchAttribute attr[1];
+        if (rb) {
+            const void* fn = rb->k[drift ? 1 : 0];
+            void* rargs[] = {&d, (void*)&u0, (void*)&v0, &u, &v};
+            rb_launch_config(*rb, batch, &cfg, attr, st);
+            e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rb->smem);
+            if (e == cudaSuccess) e = cudaLaunchKernelExC(&cfg, fn, rargs);
+        } else {
+            e = cudaFuncSetAttribute(rk, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+            if (e == cudaSuccess) e = cudaFuncSetAttribute(rk, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+            if (e == cudaSuccess) {
+                cfg.gridDim = dim3(kRRCluster * batch, 1, 1);
+                cfg.blockDim = dim3(32 * wpc, 1, 1);
+                cfg.dynamicSmemBytes = smem;
+                cfg.stream = st;
+                attr[0].id = cudaLaunchAttributeClusterDimension;
+                attr[0].val.clusterDim.x = kRRCluster;
+                attr[0].val.clusterDim.y = 1;
+                attr[0].val.clusterDim.z = 1;
+                cfg.attrs = attr;
+                cfg.numAttrs = 1;
+                e = cudaLaunchKernelExC(&cfg, rk, args);
+            }
         }
     }
     cudaError_t e2 = pool_free(d, st);
@@ -929,25 +1007,22 @@ cudaError_t gs_auto_variant(int n, bool drift, int* variant) {
 }
 
 cudaError_t gs_batch_capacity(int n, int* clusters) {
-    size_t smem = 0;
-    int wpc = 0;
-    const void* rk = rr_kernel(n, &wpc, false, &smem);
-    if (!rk) return cudaErrorInvalidValue;
-    cudaError_t e = cudaFuncSetAttribute(rk, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(rk, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-    if (e != cudaSuccess) return e;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(kRRCluster, 1, 1);
-    cfg.blockDim = dim3(32 * wpc, 1, 1);
-    cfg.dynamicSmemBytes = smem;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = kRRCluster;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    return cudaOccupancyMaxActiveClusters(clusters, rk, &cfg);
+    // the kernels a batch may take, the one that holds the most lattices at once
+    *clusters = 0;
+    for (int i = 0; i < kRBConfigs; ++i) {
+        const RBConfig& m = rb_table(i);
+        if (m.n != n || !m.wpc) continue;
+        cudaError_t e = cudaFuncSetAttribute(m.k[0], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)m.smem);
+        if (e != cudaSuccess) return e;
+        cudaLaunchConfig_t cfg;
+        cudaLaunchAttribute attr[1];
+        rb_launch_config(m, 1, &cfg, attr, nullptr);
+        int c = 0;
+        e = cudaOccupancyMaxActiveClusters(&c, m.k[0], &cfg);
+        if (e != cudaSuccess) return e;
+        *clusters = std::max(*clusters, c);
+    }
+    return *clusters > 0 ? cudaSuccess : cudaErrorInvalidValue;
 }
 
 cudaError_t gs_forward_status(int* out, bool clear) {

@@ -123,8 +123,8 @@ def forward(u0, v0, p: GSParams, checkpoints=None):
 
 
 def forward_batch(u0, v0, p: GSParams, member_params=None):
-    """Independent float32 lattices u0, v0 [batch][n][n] in one launch (one 16-CTA
-    cluster each); member_params: optional [batch][6] (F, k, Du, Dv, vx, vy)."""
+    """Independent float32 lattices u0, v0 [batch][n][n] in one launch (one thread-block
+    cluster each, smaller for larger batches); member_params: optional [batch][6] (F, k, Du, Dv, vx, vy)."""
     import torch
     u0 = u0.contiguous()
     v0 = v0.contiguous()

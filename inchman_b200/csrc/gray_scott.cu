@@ -18,6 +18,7 @@
 // The adjoint runs the transposed step backwards over a segment of stored states,
 // with the adjoint fields in cluster shared memory the same way, and accumulates
 // the parameter gradients (F, k, Du, Dv, vx, vy) in double per thread.
+#include <algorithm>
 #include <cooperative_groups.h>
 #include <cstdint>
 #include <cstdio>
@@ -537,13 +538,34 @@ const void* rr_kernel(int n, int* wpc, bool drift, size_t* smem) {
 #define GS_RR_CASE(N_, W_)                                                                        \
     if (n == N_ && *wpc == W_) {                                                                  \
         *smem = RRShape<N_, W_>::kSmem;                                                           \
-        return drift ? (const void*)k_gs_forward_rr<N_, W_, 1> : (const void*)k_gs_forward_rr<N_, W_, 0>; \
+        return drift ? (const void*)k_gs_forward_rr<N_, W_, 1, float> : (const void*)k_gs_forward_rr<N_, W_, 0, float>; \
     }
     if (*wpc == 0) *wpc = n == 256 ? 8 : n == 128 ? 4 : 2;
     GS_RR_CASE(64, 1) GS_RR_CASE(64, 2) GS_RR_CASE(64, 4)
     GS_RR_CASE(128, 2) GS_RR_CASE(128, 4) GS_RR_CASE(128, 8)
     GS_RR_CASE(256, 4) GS_RR_CASE(256, 8) GS_RR_CASE(256, 16)
 #undef GS_RR_CASE
+    return nullptr;
+}
+
+// The register-resident kernels in double, for the sides whose rows fit the registers and
+// whose halo rows fit shared memory (the shared-memory column walk pays a cluster barrier
+// per step).  us per step, before -> now, forward and gradient's backward: 64^2 0.77 ->
+// 0.26 and 1.73 -> 0.76, 128^2 1.19 -> 0.44 and 2.36 -> 1.08; 128^2 with 8 warps per CTA
+// (one row each) instead of 4: 0.51 forward, the same backward.
+const void* rr_kernel_f64(int n, bool adjoint, bool drift, int* wpc, size_t* smem) {
+#define GS_RRD_CASE(N_, WF_, WA_)                                                                  \
+    if (n == N_) {                                                                                 \
+        *wpc = adjoint ? WA_ : WF_;                                                                \
+        *smem = adjoint ? RRAdjShape<N_, WA_, double>::kSmem : RRShape<N_, WF_, double>::kSmem;    \
+        if (adjoint)                                                                               \
+            return drift ? (const void*)k_gs_adjoint_rr<N_, WA_, 1, double>                        \
+                         : (const void*)k_gs_adjoint_rr<N_, WA_, 0, double>;                       \
+        return drift ? (const void*)k_gs_forward_rr<N_, WF_, 1, double>                            \
+                     : (const void*)k_gs_forward_rr<N_, WF_, 0, double>;                           \
+    }
+    GS_RRD_CASE(64, 4, 4) GS_RRD_CASE(128, 4, 8)
+#undef GS_RRD_CASE
     return nullptr;
 }
 
@@ -733,7 +755,7 @@ const void* rr_adj_kernel(int n, int* wpc, bool drift, size_t* smem) {
 #define GS_RRA_CASE(N_, W_)                                                                        \
     if (n == N_ && *wpc == W_) {                                                                   \
         *smem = RRAdjShape<N_, W_>::kSmem;                                                         \
-        return drift ? (const void*)k_gs_adjoint_rr<N_, W_, 1> : (const void*)k_gs_adjoint_rr<N_, W_, 0>; \
+        return drift ? (const void*)k_gs_adjoint_rr<N_, W_, 1, float> : (const void*)k_gs_adjoint_rr<N_, W_, 0, float>; \
     }
     if (*wpc == 0) *wpc = n == 256 ? 8 : n == 128 ? 4 : 2;
     GS_RRA_CASE(64, 1) GS_RRA_CASE(64, 2) GS_RRA_CASE(64, 4)
@@ -885,6 +907,16 @@ cudaError_t gs_forward(const GSParams& p, const T* u0, const T* v0, T* u, T* v, 
         if (rk) return launch_cluster<T>(rk, p.n, cl, smem, st, rargs, dim3(32 * wpc, 1, 1));
         if (p.variant != 0) return cudaErrorInvalidValue;
     }
+    if constexpr (std::is_same<T, double>::value) {
+        if (cl == kRRCluster && p.variant == 0) {
+            size_t smem = 0;
+            int wpc = 0;
+            const void* rk = rr_kernel_f64(p.n, false, p.vx != 0.0 || p.vy != 0.0, &wpc, &smem);
+            const GSArgs<T>* no_batch = nullptr;
+            void* rargs[] = {&a, (void*)&u0, (void*)&v0, &u, &v, &trace, &every, &no_batch};
+            if (rk) return launch_cluster<T>(rk, p.n, cl, smem, st, rargs, dim3(32 * wpc, 1, 1));
+        }
+    }
     const dim3 blk = sizeof(T) == 4 ? x2_block(p.n, cl, 512) : cw_block(p.n, cl);
     const void* fk = fwd_kernel<T>(p.n);
     if (blk.x != 0 && fk && p.variant != 1) return launch_cluster<T>(fk, p.n, cl, smem_bytes<T>(p.n, cl), st, args, blk);
@@ -922,6 +954,14 @@ cudaError_t gs_adjoint_segment(const GSParams& p, const T* states, int len, cons
         if (rk) return launch_cluster<T>(rk, p.n, cl, smem, st, args, dim3(32 * wpc, 1, 1));
         if (variant != 0) return cudaErrorInvalidValue;
     }
+    if constexpr (std::is_same<T, double>::value) {
+        if (cl == kRRCluster && p.variant == 0) {
+            size_t smem = 0;
+            int wpc = 0;
+            const void* rk = rr_kernel_f64(p.n, true, p.vx != 0.0 || p.vy != 0.0, &wpc, &smem);
+            if (rk) return launch_cluster<T>(rk, p.n, cl, smem, st, args, dim3(32 * wpc, 1, 1));
+        }
+    }
     const dim3 blk = sizeof(T) == 4 ? x2_block(p.n, cl, 512) : cw_block(p.n, cl, 512);
     const void* ak = adj_kernel<T>(p.n);
     // the packed float32 adjoint also holds two state buffers in shared memory
@@ -945,7 +985,7 @@ cudaError_t gs_forward_batch_f32(const GSParams& p, int batch, const GSBatchMemb
     int wpc = p.variant > 10 && p.variant < kMCVariant ? p.variant - 10 : 0;   // one lattice per cluster
     const void* rk = rr_kernel(p.n, &wpc, drift, &smem);
     if (!rk) return cudaErrorInvalidValue;
-    const RBConfig* rb = p.variant == 0 ? rb_choose(p.n, batch) : nullptr;
+    const RBConfig* rb = p.variant == 0 || p.variant >= kMCVariant ? rb_choose(p.n, batch) : nullptr;
     GSArgs<float>* d = nullptr;
     cudaError_t e = pool_alloc((void**)&d, sizeof(GSArgs<float>) * batch, st);
     if (e != cudaSuccess) return e;

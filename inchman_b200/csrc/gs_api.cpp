@@ -47,12 +47,15 @@ GSParams to_params(const gpgmp_gs_params* p) {
 }
 
 // the automatic interval: 100 steps in float32 (shorter segments add launches to a
-// latency-bound adjoint: 3.05 / 3.30 / 3.79 x the forward at 100 / 50 / 25 steps);
-// 25 in float64, whose two 25-state segment buffers (50 MB at 256^2) stay in L2 while
-// the adjoint reads them back (3.11 / 3.28 / 3.70 at 25 / 50 / 100 steps, the 50-step
-// buffers at the edge of L2 and 3.78 in some runs)
+// latency-bound adjoint: 3.05 / 3.30 / 3.79 x the forward at 100 / 50 / 25 steps); in
+// float64 as many of up to 100 steps as keep the two segment buffers at 50 MB, well inside
+// L2, while the adjoint reads them back: 25 at 256^2 (3.11 / 3.28 / 3.70 x at 25 / 50 / 100),
+// 100 at 128^2 (gradient of 1,000 steps 1.61 / 1.49 / 1.48 ms at 25 / 50 / 100) and below
 int ck_every(const gpgmp_gs_params* p, int elem_bytes) {
-    return p->checkpoint_every > 0 ? p->checkpoint_every : (elem_bytes == 8 ? 25 : 100);
+    if (p->checkpoint_every > 0) return p->checkpoint_every;
+    if (elem_bytes != 8) return 100;
+    const int64_t c = 25ll * 256 * 256 / std::max<int64_t>(1, (int64_t)p->n * p->n);
+    return (int)std::min<int64_t>(100, std::max<int64_t>(25, c));
 }
 
 template <typename T>
@@ -134,7 +137,7 @@ int adjoint(const gpgmp_gs_params* p, const T* ckpt, const T* lu, const T* lv, T
     if (sizeof(T) == 4 && g.variant == 0) {
         int v = 0;
         CK(gs_auto_variant(p->n, p->vx != 0.0 || p->vy != 0.0, &v));
-        if (v >= 40) {
+        if (v >= 40 && v < 50) {     // a multi-cluster kernel
             gr.variant = 40;
             ga.variant = v;
         }

@@ -11,47 +11,71 @@
 // grad_reduce).
 
 __device__ __forceinline__ float2 f2(float x) { return make_float2(x, x); }
+__device__ __forceinline__ double2 f2(double x) { return make_double2(x, x); }
+template <typename T>
+struct GSPair;
+template <>
+struct GSPair<float> { using type = float2; };
+template <>
+struct GSPair<double> { using type = double2; };
 __device__ __forceinline__ float2 add2(float2 a, float2 b) { return __fadd2_rn(a, b); }
 __device__ __forceinline__ float2 mul2(float2 a, float2 b) { return __fmul2_rn(a, b); }
 __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
 __device__ __forceinline__ float2 sub2(float2 a, float2 b) { return __ffma2_rn(make_float2(-1.f, -1.f), b, a); }
+// the same in double, two scalar operations each
+__device__ __forceinline__ double2 add2(double2 a, double2 b) {
+    return make_double2(__dadd_rn(a.x, b.x), __dadd_rn(a.y, b.y));
+}
+__device__ __forceinline__ double2 mul2(double2 a, double2 b) {
+    return make_double2(__dmul_rn(a.x, b.x), __dmul_rn(a.y, b.y));
+}
+__device__ __forceinline__ double2 fma2(double2 a, double2 b, double2 c) {
+    return make_double2(__fma_rn(a.x, b.x, c.x), __fma_rn(a.y, b.y, c.y));
+}
+__device__ __forceinline__ double2 sub2(double2 a, double2 b) {
+    return make_double2(__dadd_rn(a.x, -b.x), __dadd_rn(a.y, -b.y));
+}
+// u v^2 in the order of the kernels of each precision
+__device__ __forceinline__ float2 uvv2(float2 u, float2 v) { return mul2(u, mul2(v, v)); }
+__device__ __forceinline__ double2 uvv2(double2 u, double2 v) { return mul2(mul2(u, v), v); }
 __device__ __forceinline__ float2 ld2(const float* p) { return *reinterpret_cast<const float2*>(p); }
 __device__ __forceinline__ void st2(float* p, float2 v) { *reinterpret_cast<float2*>(p) = v; }
 
-struct GSCoef2 {
-    float2 du, dv, hx, hy, dt, mdt, dtF, mdtF, mdtFk, m4, one, two_dt;
+template <typename T>
+struct GSCoefP {
+    typename GSPair<T>::type du, dv, hx, hy, dt, mdt, dtF, mdtF, mdtFk, m4, one, two_dt;
     bool drift;
-    __device__ __forceinline__ explicit GSCoef2(const GSArgs<float>& a) {
+    __device__ __forceinline__ explicit GSCoefP(const GSArgs<T>& a) {
         du = f2(a.dt * a.Du);
         dv = f2(a.dt * a.Dv);
-        hx = f2(a.dt * a.vx * 0.5f);
-        hy = f2(a.dt * a.vy * 0.5f);
+        hx = f2(a.dt * a.vx * T(0.5));
+        hy = f2(a.dt * a.vy * T(0.5));
         dt = f2(a.dt);
         mdt = f2(-a.dt);
         dtF = f2(a.dt * a.F);
         mdtF = f2(-(a.dt * a.F));
         mdtFk = f2(-(a.dt * (a.F + a.k)));
-        m4 = f2(-4.f);
-        one = f2(1.f);
+        m4 = f2(T(-4));
+        one = f2(T(1));
         two_dt = f2(a.dt + a.dt);
-        drift = a.vx != 0.f || a.vy != 0.f;
+        drift = a.vx != T(0) || a.vy != T(0);
     }
 };
+using GSCoef2 = GSCoefP<float>;
 
 // forward update of two cells at once: C the cells, U / D their upper and lower
 // neighbours, h the sums and d (with drift) the differences of their left and right ones
 // (any pairing of cells; the arithmetic per cell is the same as in the scalar kernels'
 // gs_update).  DRIFT: 1 with the drift
 // terms, 0 without, -1 decided by k.drift at run time.
-template <int DRIFT>
-__device__ __forceinline__ void gs_update2s(const GSCoef2& k, float2 uh, float2 ud, float2 uU, float2 uC, float2 uD,
-                                            float2 vh, float2 vd, float2 vU, float2 vC, float2 vD, float2* un,
-                                            float2* vn) {
-    const float2 uvv = mul2(uC, mul2(vC, vC));
-    const float2 lu = fma2(k.m4, uC, add2(uh, add2(uU, uD)));
-    const float2 lv = fma2(k.m4, vC, add2(vh, add2(vU, vD)));
-    float2 a = fma2(k.du, lu, fma2(k.mdtF, uC, k.dtF));
-    float2 b = fma2(k.mdtFk, vC, mul2(k.dv, lv));
+template <int DRIFT, typename T, typename P>
+__device__ __forceinline__ void gs_update2s(const GSCoefP<T>& k, P uh, P ud, P uU, P uC, P uD, P vh, P vd, P vU, P vC,
+                                            P vD, P* un, P* vn) {
+    const P uvv = uvv2(uC, vC);
+    const P lu = fma2(k.m4, uC, add2(uh, add2(uU, uD)));
+    const P lv = fma2(k.m4, vC, add2(vh, add2(vU, vD)));
+    P a = fma2(k.du, lu, fma2(k.mdtF, uC, k.dtF));
+    P b = fma2(k.mdtFk, vC, mul2(k.dv, lv));
     if (DRIFT == 1 || (DRIFT < 0 && k.drift)) {
         a = fma2(k.hx, ud, fma2(k.hy, sub2(uU, uD), a));
         b = fma2(k.hx, vd, fma2(k.hy, sub2(vU, vD), b));
@@ -251,16 +275,16 @@ __device__ __forceinline__ void gs_adj_update2f(const GSCoef2& k, float2 aL, flo
 //   sum a lap(u) = sum u lap(a),   sum a (uR - uL) = -sum u (aR - aL)  (and in y).
 // t[2], t[3] as in gs_adj_update2f; t[4], t[5] hold the NEGATED drift sums.  The
 // adjoint fields an, bn are the same bits as gs_adj_update2f's.
-template <int DRIFT>
-__device__ __forceinline__ void gs_adj_update2s(const GSCoef2& k, float2 aL, float2 aR, float2 aU, float2 aC, float2 aD,
-                                                float2 bL, float2 bR, float2 bU, float2 bC, float2 bD, float2 uC,
-                                                float2 vC, float2* an, float2* bn, float2 t[6]) {
-    const float2 lap_a = fma2(k.m4, aC, add2(add2(aL, aR), add2(aU, aD)));
-    const float2 lap_b = fma2(k.m4, bC, add2(add2(bL, bR), add2(bU, bD)));
-    const float2 ba = sub2(bC, aC);
-    float2 x = fma2(k.du, lap_a, mul2(k.mdtF, aC));
-    float2 y = fma2(k.dv, lap_b, mul2(k.mdtFk, bC));
-    const float2 dxa = sub2(aR, aL), dya = sub2(aD, aU), dxb = sub2(bR, bL), dyb = sub2(bD, bU);
+template <int DRIFT, typename T, typename P>
+__device__ __forceinline__ void gs_adj_update2s(const GSCoefP<T>& k, P aL, P aR, P aU, P aC, P aD,
+                                                P bL, P bR, P bU, P bC, P bD, P uC,
+                                                P vC, P* an, P* bn, P t[6]) {
+    const P lap_a = fma2(k.m4, aC, add2(add2(aL, aR), add2(aU, aD)));
+    const P lap_b = fma2(k.m4, bC, add2(add2(bL, bR), add2(bU, bD)));
+    const P ba = sub2(bC, aC);
+    P x = fma2(k.du, lap_a, mul2(k.mdtF, aC));
+    P y = fma2(k.dv, lap_b, mul2(k.mdtFk, bC));
+    const P dxa = sub2(aR, aL), dya = sub2(aD, aU), dxb = sub2(bR, bL), dyb = sub2(bD, bU);
     if (DRIFT == 1) {
         x = fma2(k.hx, dxa, fma2(k.hy, dya, x));
         y = fma2(k.hx, dxb, fma2(k.hy, dyb, y));

@@ -55,6 +55,14 @@ __device__ __forceinline__ void rr_st_async(uint32_t addr, float2 v, uint32_t ba
                  "f"(v.x), "f"(v.y), "r"(bar)
                  : "memory");
 }
+__device__ __forceinline__ void rr_st_async(uint32_t addr, double2 v, uint32_t bar) {
+    asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v2.f64 [%0], {%1, %2}, [%3];\n" ::"r"(addr),
+                 "d"(v.x), "d"(v.y), "r"(bar)
+                 : "memory");
+}
+__device__ __forceinline__ void rr_st_local(uint32_t addr, double2 v) {
+    asm volatile("st.shared.v2.f64 [%0], {%1, %2};\n" ::"r"(addr), "d"(v.x), "d"(v.y) : "memory");
+}
 __device__ __forceinline__ void rr_st_local(uint32_t addr, float4 v) {
     asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};\n" ::"r"(addr), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w)
                  : "memory");
@@ -131,13 +139,55 @@ __device__ __forceinline__ void rr_store(float* __restrict__ p, const float2 (&x
     }
 }
 
-// halo row of one field in shared memory: units of two pairs (one pair for H = 1),
-// unit q of lane l at byte (q * 32 + l) * unit size, conflict-free for the warp
 template <int H>
+__device__ __forceinline__ void rr_load(const double* __restrict__ p, double2 (&x)[H]) {
+    if constexpr (H == 1) {
+        x[0] = reinterpret_cast<const double2*>(p)[0];
+    } else {
+#pragma unroll
+        for (int q = 0; q < H / 2; ++q) {
+            const double2 a = reinterpret_cast<const double2*>(p)[q], b = reinterpret_cast<const double2*>(p + H)[q];
+            x[2 * q] = make_double2(a.x, b.x);
+            x[2 * q + 1] = make_double2(a.y, b.y);
+        }
+    }
+}
+template <int H>
+__device__ __forceinline__ void rr_store(double* __restrict__ p, const double2 (&x)[H]) {
+    if constexpr (H == 1) {
+        reinterpret_cast<double2*>(p)[0] = x[0];
+    } else {
+#pragma unroll
+        for (int q = 0; q < H / 2; ++q) {
+            reinterpret_cast<double2*>(p)[q] = make_double2(x[2 * q].x, x[2 * q + 1].x);
+            reinterpret_cast<double2*>(p + H)[q] = make_double2(x[2 * q].y, x[2 * q + 1].y);
+        }
+    }
+}
+
+// halo row of one field in shared memory: units of two pairs (one pair for H = 1),
+// unit q of lane l at byte (q * 32 + l) * unit size, conflict-free for the warp; one pair
+// of doubles per unit
+template <int H, typename P = float2>
 struct RRUnit {
     static constexpr int kCount = H >= 2 ? H / 2 : 1;
     static constexpr uint32_t kBytes = H >= 2 ? 16 : 8;
 };
+template <int H>
+struct RRUnit<H, double2> {
+    static constexpr int kCount = H;
+    static constexpr uint32_t kBytes = 16;
+};
+template <int H>
+__device__ __forceinline__ auto rr_unit(const float2 (&p)[H], int q) {
+    if constexpr (H >= 2) {
+        return make_float4(p[2 * q].x, p[2 * q].y, p[2 * q + 1].x, p[2 * q + 1].y);
+    } else {
+        return p[0];
+    }
+}
+template <int H>
+__device__ __forceinline__ double2 rr_unit(const double2 (&p)[H], int q) { return p[q]; }
 
 template <int H>
 __device__ __forceinline__ void rr_read_halo(const unsigned char* base, int lane, float2 (&x)[H]) {
@@ -153,35 +203,34 @@ __device__ __forceinline__ void rr_read_halo(const unsigned char* base, int lane
     }
 }
 
+template <int H>
+__device__ __forceinline__ void rr_read_halo(const unsigned char* base, int lane, double2 (&x)[H]) {
+#pragma unroll
+    for (int q = 0; q < H; ++q) x[q] = reinterpret_cast<const double2*>(base)[q * 32 + lane];
+}
+
 // sends one row (both fields) into the destination warp's halo slot: st.async with
 // a complete_tx on the destination's mbarrier when it lives in another CTA, else
 // st.shared and one mbarrier arrive per lane.  dst_u / dst_v / bar are addresses
 // in the destination CTA's shared-memory layout.
-template <int H>
-__device__ __forceinline__ void rr_send(const float2 (&pu)[H], const float2 (&pv)[H], uint32_t dst_u, uint32_t dst_v,
+template <int H, typename P>
+__device__ __forceinline__ void rr_send(const P (&pu)[H], const P (&pv)[H], uint32_t dst_u, uint32_t dst_v,
                                         uint32_t bar, bool remote, uint32_t rank, int lane) {
-    constexpr uint32_t UB = RRUnit<H>::kBytes;
-    auto unit = [](const float2 (&p)[H], int q) {
-        if constexpr (H >= 2) {
-            return make_float4(p[2 * q].x, p[2 * q].y, p[2 * q + 1].x, p[2 * q + 1].y);
-        } else {
-            return p[0];
-        }
-    };
+    using U = RRUnit<H, P>;
     if (remote) {
         const uint32_t ru = rr_mapa(dst_u, rank), rv = rr_mapa(dst_v, rank), rb = rr_mapa(bar, rank);
 #pragma unroll
-        for (int q = 0; q < RRUnit<H>::kCount; ++q) {
-            const uint32_t off = (uint32_t)(q * 32 + lane) * UB;
-            rr_st_async(ru + off, unit(pu, q), rb);
-            rr_st_async(rv + off, unit(pv, q), rb);
+        for (int q = 0; q < U::kCount; ++q) {
+            const uint32_t off = (uint32_t)(q * 32 + lane) * U::kBytes;
+            rr_st_async(ru + off, rr_unit<H>(pu, q), rb);
+            rr_st_async(rv + off, rr_unit<H>(pv, q), rb);
         }
     } else {
 #pragma unroll
-        for (int q = 0; q < RRUnit<H>::kCount; ++q) {
-            const uint32_t off = (uint32_t)(q * 32 + lane) * UB;
-            rr_st_local(dst_u + off, unit(pu, q));
-            rr_st_local(dst_v + off, unit(pv, q));
+        for (int q = 0; q < U::kCount; ++q) {
+            const uint32_t off = (uint32_t)(q * 32 + lane) * U::kBytes;
+            rr_st_local(dst_u + off, rr_unit<H>(pu, q));
+            rr_st_local(dst_v + off, rr_unit<H>(pv, q));
         }
         rr_arrive(bar);
     }
@@ -192,25 +241,25 @@ __device__ __forceinline__ void rr_send(const float2 (&pu)[H], const float2 (&pv
 // are added one by one, which costs the FP32 pipe as much as a packed addition (packed
 // operations take two cycles) and needs no moves into a pair: 256^2 on four clusters 0.586
 // -> 0.515 us per step, together with waiting before asking for an earlier failure.
-template <int H, int DRIFT>
-__device__ __forceinline__ void rr_horizontal(const float2 (&x)[H], float2 (&h)[H], float2 (&d)[H], int lane) {
-    const float l = __shfl_sync(0xffffffffu, x[H - 1].y, (lane + 31) & 31);
-    const float r = __shfl_sync(0xffffffffu, x[0].x, (lane + 1) & 31);
+template <int H, int DRIFT, typename P>
+__device__ __forceinline__ void rr_horizontal(const P (&x)[H], P (&h)[H], P (&d)[H], int lane) {
+    const auto l = __shfl_sync(0xffffffffu, x[H - 1].y, (lane + 31) & 31);
+    const auto r = __shfl_sync(0xffffffffu, x[0].x, (lane + 1) & 31);
 #pragma unroll
     for (int j = 0; j < H; ++j) {
-        const float2 L = j == 0 ? make_float2(l, x[H - 1].x) : x[j == 0 ? 0 : j - 1];
-        const float2 R = j == H - 1 ? make_float2(x[0].y, r) : x[j == H - 1 ? 0 : j + 1];
-        h[j] = j == 0 || j == H - 1 ? make_float2(L.x + R.x, L.y + R.y) : add2(L, R);
-        if (DRIFT) d[j] = j == 0 || j == H - 1 ? make_float2(L.x - R.x, L.y - R.y) : sub2(L, R);
+        const P L = j == 0 ? P{l, x[H - 1].x} : x[j == 0 ? 0 : j - 1];
+        const P R = j == H - 1 ? P{x[0].y, r} : x[j == H - 1 ? 0 : j + 1];
+        h[j] = j == 0 || j == H - 1 ? P{L.x + R.x, L.y + R.y} : add2(L, R);
+        if (DRIFT) d[j] = j == 0 || j == H - 1 ? P{L.x - R.x, L.y - R.y} : sub2(L, R);
     }
 }
 
 // next state of one row from the rows above (U), at (C) and below (D)
-template <int H, int DRIFT>
-__device__ __forceinline__ void rr_row(const GSCoef2& k, const float2 (&uU)[H], const float2 (&uC)[H],
-                                       const float2 (&uD)[H], const float2 (&vU)[H], const float2 (&vC)[H],
-                                       const float2 (&vD)[H], float2 (&un)[H], float2 (&vn)[H], int lane) {
-    float2 uh[H], ud[H], vh[H], vd[H];
+template <int H, int DRIFT, typename T, typename P>
+__device__ __forceinline__ void rr_row(const GSCoefP<T>& k, const P (&uU)[H], const P (&uC)[H], const P (&uD)[H],
+                                       const P (&vU)[H], const P (&vC)[H], const P (&vD)[H], P (&un)[H], P (&vn)[H],
+                                       int lane) {
+    P uh[H], ud[H], vh[H], vd[H];
     rr_horizontal<H, DRIFT>(uC, uh, ud, lane);
     rr_horizontal<H, DRIFT>(vC, vh, vd, lane);
 #pragma unroll
@@ -218,11 +267,11 @@ __device__ __forceinline__ void rr_row(const GSCoef2& k, const float2 (&uU)[H], 
         gs_update2s<DRIFT>(k, uh[j], ud[j], uU[j], uC[j], uD[j], vh[j], vd[j], vU[j], vC[j], vD[j], &un[j], &vn[j]);
 }
 
-template <int N, int WPC>
+template <int N, int WPC, typename T = float>
 struct RRShape {
     static constexpr int R = N / (kRRCluster * WPC);   // rows per warp
     static constexpr int H = N / 64;                    // column pairs per lane
-    static constexpr uint32_t kRow = 4u * N;            // bytes of one halo row of one field
+    static constexpr uint32_t kRow = sizeof(T) * N;            // bytes of one halo row of one field
     // [warp][parity][side above/below][field u/v] halo rows, then [warp][parity]
     // mbarriers, then the CTA's failure flag
     static constexpr uint32_t kHalo = (uint32_t)WPC * 8u * kRow;
@@ -231,9 +280,9 @@ struct RRShape {
     static_assert(R >= 1 && R * kRRCluster * WPC == N && H >= 1 && 64 * H == N, "lattice split");
 };
 
-template <int N, int WPC>
+template <int N, int WPC, typename T = float>
 struct RRCtx {
-    using S = RRShape<N, WPC>;
+    using S = RRShape<N, WPC, T>;
     uint32_t sbase;
     const unsigned char* smem;
     int lane, w;
@@ -251,18 +300,18 @@ struct RRCtx {
 // one step X -> Y of the warp's rows in registers (s: the step index of X; send:
 // whether Y's edge rows go out, i.e. not after the last step).  The edge rows are
 // computed and sent first; the interior rows are computed while the sends travel.
-template <int N, int WPC, int DRIFT>
-__device__ __forceinline__ void rr_step(const RRCtx<N, WPC>& c, const GSCoef2& k,
-                                        const float2 (&xu)[RRShape<N, WPC>::R][RRShape<N, WPC>::H],
-                                        const float2 (&xv)[RRShape<N, WPC>::R][RRShape<N, WPC>::H],
-                                        float2 (&yu)[RRShape<N, WPC>::R][RRShape<N, WPC>::H],
-                                        float2 (&yv)[RRShape<N, WPC>::R][RRShape<N, WPC>::H], int s, bool send) {
-    constexpr int R = RRShape<N, WPC>::R, H = RRShape<N, WPC>::H;
+template <int N, int WPC, int DRIFT, typename T, typename P = typename GSPair<T>::type>
+__device__ __forceinline__ void rr_step(const RRCtx<N, WPC, T>& c, const GSCoefP<T>& k,
+                                        const P (&xu)[RRShape<N, WPC, T>::R][RRShape<N, WPC, T>::H],
+                                        const P (&xv)[RRShape<N, WPC, T>::R][RRShape<N, WPC, T>::H],
+                                        P (&yu)[RRShape<N, WPC, T>::R][RRShape<N, WPC, T>::H],
+                                        P (&yv)[RRShape<N, WPC, T>::R][RRShape<N, WPC, T>::H], int s, bool send) {
+    constexpr int R = RRShape<N, WPC, T>::R, H = RRShape<N, WPC, T>::H;
     const int par = s & 1;
     rr_wait(c.bar(c.w, par), (uint32_t)(s >> 1) & 1u, c.failed);
     __syncwarp();
     if (c.lane == 0) rr_arm(c.bar(c.w, par), c.tx);   // the phase of step s + 2
-    float2 au[H], av[H], bu[H], bv[H];
+    P au[H], av[H], bu[H], bv[H];
     rr_read_halo<H>(c.smem + (c.slot(c.w, par, 0, 0) - c.sbase), c.lane, au);
     rr_read_halo<H>(c.smem + (c.slot(c.w, par, 0, 1) - c.sbase), c.lane, av);
     rr_read_halo<H>(c.smem + (c.slot(c.w, par, 1, 0) - c.sbase), c.lane, bu);
@@ -286,12 +335,12 @@ __device__ __forceinline__ void rr_step(const RRCtx<N, WPC>& c, const GSCoef2& k
         rr_row<H, DRIFT>(k, xu[r - 1], xu[r], xu[r + 1], xv[r - 1], xv[r], xv[r + 1], yu[r], yv[r], c.lane);
 }
 
-template <int N, int WPC, int DRIFT>
+template <int N, int WPC, int DRIFT, typename T, typename P = typename GSPair<T>::type>
 __global__ void __launch_bounds__(32 * WPC, 1)
-    k_gs_forward_rr(GSArgs<float> a, const float* __restrict__ u0, const float* __restrict__ v0,
-                    float* __restrict__ uo, float* __restrict__ vo, float* __restrict__ trace, int trace_every,
-                    const GSArgs<float>* __restrict__ batch_args) {
-    using S = RRShape<N, WPC>;
+    k_gs_forward_rr(GSArgs<T> a, const T* __restrict__ u0, const T* __restrict__ v0,
+                    T* __restrict__ uo, T* __restrict__ vo, T* __restrict__ trace, int trace_every,
+                    const GSArgs<T>* __restrict__ batch_args) {
+    using S = RRShape<N, WPC, T>;
     constexpr int R = S::R, H = S::H;
     constexpr int NN = N * N;
     // a batched launch runs one lattice per cluster: member m = cluster index, with
@@ -304,7 +353,7 @@ __global__ void __launch_bounds__(32 * WPC, 1)
         trace = nullptr;
     }
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    RRCtx<N, WPC> c;
+    RRCtx<N, WPC, T> c;
     c.smem = smem_raw;
     c.sbase = smem_u32(smem_raw);
     c.lane = threadIdx.x & 31;
@@ -321,7 +370,7 @@ __global__ void __launch_bounds__(32 * WPC, 1)
     c.tx = (uint32_t)nremote * 2u * S::kRow;
     const int row0 = ((int)rank * WPC + c.w) * R;
     const int col0 = c.lane * 2 * H;
-    const GSCoef2 k(a);
+    const GSCoefP<T> k(a);
 
     if (c.lane == 0) {
         // arrivals per phase: the own arm + 32 lanes of every producer warp in this CTA
@@ -330,7 +379,7 @@ __global__ void __launch_bounds__(32 * WPC, 1)
         fence_mbar_init();
     }
     if (threadIdx.x == 0) *c.failed = 0;
-    float2 xu[R][H], xv[R][H], yu[R][H], yv[R][H];
+    P xu[R][H], xv[R][H], yu[R][H], yv[R][H];
 #pragma unroll
     for (int r = 0; r < R; ++r) {
         rr_load<H>(u0 + (size_t)(row0 + r) * N + col0, xu[r]);
@@ -351,9 +400,9 @@ __global__ void __launch_bounds__(32 * WPC, 1)
         rr_send<H>(xu[R - 1], xv[R - 1], c.slot(c.dn_w, 0, 0, 0), c.slot(c.dn_w, 0, 0, 1), c.bar(c.dn_w, 0),
                    c.dn_remote, c.dn_rank, c.lane);
     }
-    auto put_trace = [&](int s, const float2 (&pu)[R][H], const float2 (&pv)[R][H]) {
+    auto put_trace = [&](int s, const P (&pu)[R][H], const P (&pv)[R][H]) {
         if (trace != nullptr && s % every == 0) {
-            float* du = trace + (size_t)(2 * (s / every)) * NN;
+            T* du = trace + (size_t)(2 * (s / every)) * NN;
 #pragma unroll
             for (int r = 0; r < R; ++r) {
                 rr_store<H>(du + (size_t)(row0 + r) * N + col0, pu[r]);
@@ -364,28 +413,28 @@ __global__ void __launch_bounds__(32 * WPC, 1)
     int s = 0;
     for (; s + 2 <= steps; s += 2) {      // two steps per iteration: X -> Y -> X without copies
         put_trace(s, xu, xv);
-        rr_step<N, WPC, DRIFT>(c, k, xu, xv, yu, yv, s, true);
+        rr_step<N, WPC, DRIFT, T>(c, k, xu, xv, yu, yv, s, true);
         put_trace(s + 1, yu, yv);
-        rr_step<N, WPC, DRIFT>(c, k, yu, yv, xu, xv, s + 1, s + 2 < steps);
+        rr_step<N, WPC, DRIFT, T>(c, k, yu, yv, xu, xv, s + 1, s + 2 < steps);
     }
     const bool odd = s < steps;
     if (odd) {
         put_trace(s, xu, xv);
-        rr_step<N, WPC, DRIFT>(c, k, xu, xv, yu, yv, s, false);
+        rr_step<N, WPC, DRIFT, T>(c, k, xu, xv, yu, yv, s, false);
     }
     __syncthreads();
     cluster_arrive();     // no CTA leaves while a neighbour may still address its shared memory
     cluster_wait();
     const bool bad = *c.failed != 0;
     if (bad && threadIdx.x == 0) atomicOr(&g_gs_fwd_err, 1);
-    const float nan = __int_as_float(0x7fc00000);
+    const T nan = (T)__int_as_float(0x7fc00000);
 #pragma unroll
     for (int r = 0; r < R; ++r) {
-        float2 pu[H], pv[H];
+        P pu[H], pv[H];
 #pragma unroll
         for (int j = 0; j < H; ++j) {
-            pu[j] = bad ? make_float2(nan, nan) : (odd ? yu[r][j] : xu[r][j]);
-            pv[j] = bad ? make_float2(nan, nan) : (odd ? yv[r][j] : xv[r][j]);
+            pu[j] = bad ? P{nan, nan} : (odd ? yu[r][j] : xu[r][j]);
+            pv[j] = bad ? P{nan, nan} : (odd ? yv[r][j] : xv[r][j]);
         }
         rr_store<H>(uo + (size_t)(row0 + r) * N + col0, pu);
         rr_store<H>(vo + (size_t)(row0 + r) * N + col0, pv);
@@ -406,9 +455,9 @@ __global__ void __launch_bounds__(32 * WPC, 1)
 // halo rows).  The partial sums are formed per lane and step in float and summed
 // in double.
 
-template <int N, int WPC>
+template <int N, int WPC, typename T = float>
 struct RRAdjShape {
-    using F = RRShape<N, WPC>;
+    using F = RRShape<N, WPC, T>;
     static constexpr int R = F::R, H = F::H;
     static constexpr int RC = WPC * R;                      // rows per CTA
     static constexpr int NB = 4;                            // state buffers in the ring
@@ -416,26 +465,26 @@ struct RRAdjShape {
     static constexpr uint32_t kPipe = F::kHalo + (uint32_t)WPC * 16u;   // full[NB], empty[NB]
     static constexpr uint32_t kFlag = kPipe + 16u * NB;
     static constexpr uint32_t kState = (kFlag + 16u + 127u) / 128u * 128u;   // [buf][field][RC][N]
-    static constexpr uint32_t kPlane = (uint32_t)RC * 4u * N;
+    static constexpr uint32_t kPlane = (uint32_t)RC * sizeof(T) * N;
     static constexpr uint32_t kSmem = kState + 2u * NB * kPlane;
     static_assert(kSmem <= 227u * 1024u, "adjoint shared memory exceeds a B200 CTA's");
 };
 
-template <int H, int DRIFT>
-__device__ __forceinline__ void rr_adj_row(const GSCoef2& k, const float2 (&aU)[H], const float2 (&aC)[H],
-                                           const float2 (&aD)[H], const float2 (&bU)[H], const float2 (&bC)[H],
-                                           const float2 (&bD)[H], const float2 (&uC)[H], const float2 (&vC)[H],
-                                           float2 (&an)[H], float2 (&bn)[H], float2 t[6], int lane) {
+template <int H, int DRIFT, typename T, typename P>
+__device__ __forceinline__ void rr_adj_row(const GSCoefP<T>& k, const P (&aU)[H], const P (&aC)[H],
+                                           const P (&aD)[H], const P (&bU)[H], const P (&bC)[H],
+                                           const P (&bD)[H], const P (&uC)[H], const P (&vC)[H],
+                                           P (&an)[H], P (&bn)[H], P t[6], int lane) {
     const int lft = (lane + 31) & 31, rgt = (lane + 1) & 31;
-    const float al = __shfl_sync(0xffffffffu, aC[H - 1].y, lft), ar = __shfl_sync(0xffffffffu, aC[0].x, rgt);
-    const float bl = __shfl_sync(0xffffffffu, bC[H - 1].y, lft), br = __shfl_sync(0xffffffffu, bC[0].x, rgt);
+    const T al = __shfl_sync(0xffffffffu, aC[H - 1].y, lft), ar = __shfl_sync(0xffffffffu, aC[0].x, rgt);
+    const T bl = __shfl_sync(0xffffffffu, bC[H - 1].y, lft), br = __shfl_sync(0xffffffffu, bC[0].x, rgt);
 #pragma unroll
     for (int j = 0; j < H; ++j) {
         const int jl = j == 0 ? 0 : j - 1, jr = j == H - 1 ? 0 : j + 1;
-        const float2 aL = j == 0 ? make_float2(al, aC[H - 1].x) : aC[jl];
-        const float2 aR = j == H - 1 ? make_float2(aC[0].y, ar) : aC[jr];
-        const float2 bL = j == 0 ? make_float2(bl, bC[H - 1].x) : bC[jl];
-        const float2 bR = j == H - 1 ? make_float2(bC[0].y, br) : bC[jr];
+        const P aL = j == 0 ? P{al, aC[H - 1].x} : aC[jl];
+        const P aR = j == H - 1 ? P{aC[0].y, ar} : aC[jr];
+        const P bL = j == 0 ? P{bl, bC[H - 1].x} : bC[jl];
+        const P bR = j == H - 1 ? P{bC[0].y, br} : bC[jr];
         gs_adj_update2s<DRIFT>(k, aL, aR, aU[j], aC[j], aD[j], bL, bR, bU[j], bC[j], bD[j], uC[j], vC[j], &an[j],
                                &bn[j], t);
     }
@@ -444,10 +493,10 @@ __device__ __forceinline__ void rr_adj_row(const GSCoef2& k, const float2 (&aU)[
 // issues the TMA copies of the forward state of adjoint step q (stored state
 // len - 1 - q) into ring buffer q % NB, after all warps released that buffer's
 // previous use (step q - NB); one thread
-template <int N, int WPC>
-__device__ __forceinline__ void rr_adj_issue(const RRCtx<N, WPC>& c, const float* __restrict__ states, int len, int q,
+template <int N, int WPC, typename T>
+__device__ __forceinline__ void rr_adj_issue(const RRCtx<N, WPC, T>& c, const T* __restrict__ states, int len, int q,
                                              int rc0) {
-    using S = RRAdjShape<N, WPC>;
+    using S = RRAdjShape<N, WPC, T>;
     constexpr int NN = N * N;
     const int b = q % S::NB, j = len - 1 - q;
     uint64_t* full = reinterpret_cast<uint64_t*>(const_cast<unsigned char*>(c.smem) + S::kPipe) + b;
@@ -455,8 +504,8 @@ __device__ __forceinline__ void rr_adj_issue(const RRCtx<N, WPC>& c, const float
     fence_proxy_async();
     mbar_expect_tx(full, 2u * S::kPlane);
     for (int f = 0; f < 2; ++f) {
-        const float* src = states + (size_t)(2 * j + f) * NN + (size_t)rc0 * N;
-        float* dst = reinterpret_cast<float*>(const_cast<unsigned char*>(c.smem) + S::kState +
+        const T* src = states + (size_t)(2 * j + f) * NN + (size_t)rc0 * N;
+        T* dst = reinterpret_cast<T*>(const_cast<unsigned char*>(c.smem) + S::kState +
                                               (uint32_t)(2 * b + f) * S::kPlane);
         bulk_g2s(dst, src, S::kPlane, full);
     }
@@ -464,14 +513,14 @@ __device__ __forceinline__ void rr_adj_issue(const RRCtx<N, WPC>& c, const float
 
 // one transposed step X -> Y of the warp's adjoint rows; the forward state of the
 // step is buffer s % NB of the state ring
-template <int N, int WPC, int DRIFT>
-__device__ __forceinline__ void rr_adj_step(const RRCtx<N, WPC>& c, const GSCoef2& k,
-                                            const float2 (&xa)[RRShape<N, WPC>::R][RRShape<N, WPC>::H],
-                                            const float2 (&xb)[RRShape<N, WPC>::R][RRShape<N, WPC>::H],
-                                            float2 (&ya)[RRShape<N, WPC>::R][RRShape<N, WPC>::H],
-                                            float2 (&yb)[RRShape<N, WPC>::R][RRShape<N, WPC>::H], int s, bool send,
-                                            float2 t[6]) {
-    using S = RRAdjShape<N, WPC>;
+template <int N, int WPC, int DRIFT, typename T, typename P = typename GSPair<T>::type>
+__device__ __forceinline__ void rr_adj_step(const RRCtx<N, WPC, T>& c, const GSCoefP<T>& k,
+                                            const P (&xa)[RRShape<N, WPC, T>::R][RRShape<N, WPC, T>::H],
+                                            const P (&xb)[RRShape<N, WPC, T>::R][RRShape<N, WPC, T>::H],
+                                            P (&ya)[RRShape<N, WPC, T>::R][RRShape<N, WPC, T>::H],
+                                            P (&yb)[RRShape<N, WPC, T>::R][RRShape<N, WPC, T>::H], int s, bool send,
+                                            P t[6]) {
+    using S = RRAdjShape<N, WPC, T>;
     constexpr int R = S::R, H = S::H;
     const int par = s & 1, sb = s % S::NB;
     const uint32_t full = c.sbase + S::kPipe + 8u * sb;
@@ -480,16 +529,16 @@ __device__ __forceinline__ void rr_adj_step(const RRCtx<N, WPC>& c, const GSCoef
     rr_wait(c.bar(c.w, par), (uint32_t)(s >> 1) & 1u, c.failed);   // the adjoint halo rows
     __syncwarp();
     if (c.lane == 0) rr_arm(c.bar(c.w, par), c.tx);
-    float2 ha[H], hb[H], la[H], lb[H];
+    P ha[H], hb[H], la[H], lb[H];
     rr_read_halo<H>(c.smem + (c.slot(c.w, par, 0, 0) - c.sbase), c.lane, ha);
     rr_read_halo<H>(c.smem + (c.slot(c.w, par, 0, 1) - c.sbase), c.lane, hb);
     rr_read_halo<H>(c.smem + (c.slot(c.w, par, 1, 0) - c.sbase), c.lane, la);
     rr_read_halo<H>(c.smem + (c.slot(c.w, par, 1, 1) - c.sbase), c.lane, lb);
     // the forward state at the warp's rows (shared-memory rows w R .. w R + R - 1)
-    const float* Us = reinterpret_cast<const float*>(c.smem + S::kState + (uint32_t)(2 * sb) * S::kPlane);
-    const float* Vs = reinterpret_cast<const float*>(c.smem + S::kState + (uint32_t)(2 * sb + 1) * S::kPlane);
+    const T* Us = reinterpret_cast<const T*>(c.smem + S::kState + (uint32_t)(2 * sb) * S::kPlane);
+    const T* Vs = reinterpret_cast<const T*>(c.smem + S::kState + (uint32_t)(2 * sb + 1) * S::kPlane);
     const int col0 = c.lane * 2 * H;
-    float2 su[R][H], sv[R][H];
+    P su[R][H], sv[R][H];
 #pragma unroll
     for (int r = 0; r < R; ++r) {
         rr_load<H>(Us + (c.w * R + r) * N + col0, su[r]);
@@ -517,17 +566,17 @@ __device__ __forceinline__ void rr_adj_step(const RRCtx<N, WPC>& c, const GSCoef
     if (c.lane == 0) rr_arrive(empty);                       // this warp is done with the state buffer
 }
 
-template <int N, int WPC, int DRIFT>
+template <int N, int WPC, int DRIFT, typename T, typename P = typename GSPair<T>::type>
 __global__ void __launch_bounds__(32 * WPC, 1)
-    k_gs_adjoint_rr(GSArgs<float> a, const float* __restrict__ states, int len, const float* __restrict__ lu_in,
-                    const float* __restrict__ lv_in, float* __restrict__ lu_out, float* __restrict__ lv_out,
+    k_gs_adjoint_rr(GSArgs<T> a, const T* __restrict__ states, int len, const T* __restrict__ lu_in,
+                    const T* __restrict__ lv_in, T* __restrict__ lu_out, T* __restrict__ lv_out,
                     double* __restrict__ grad, int* __restrict__ err) {
-    using S = RRAdjShape<N, WPC>;
+    using S = RRAdjShape<N, WPC, T>;
     constexpr int R = S::R, H = S::H, RC = S::RC;
     constexpr int NN = N * N;
     extern __shared__ __align__(128) unsigned char smem_raw[];
     __shared__ double red[6][32];
-    RRCtx<N, WPC> c;
+    RRCtx<N, WPC, T> c;
     c.smem = smem_raw;
     c.sbase = smem_u32(smem_raw);
     c.lane = threadIdx.x & 31;
@@ -541,12 +590,12 @@ __global__ void __launch_bounds__(32 * WPC, 1)
     c.dn_w = c.dn_remote ? 0 : c.w + 1;
     c.failed = reinterpret_cast<volatile int*>(smem_raw + S::kFlag);
     const int nremote = (int)c.up_remote + (int)c.dn_remote;
-    c.tx = (uint32_t)nremote * 2u * RRShape<N, WPC>::kRow;
+    c.tx = (uint32_t)nremote * 2u * RRShape<N, WPC, T>::kRow;
     uint64_t* pipe = reinterpret_cast<uint64_t*>(smem_raw + S::kPipe);   // full[0..NB-1], empty[0..NB-1]
     const int rc0 = (int)rank * RC;
     const int row0 = rc0 + c.w * R;
     const int col0 = c.lane * 2 * H;
-    const GSCoef2 k(a);
+    const GSCoefP<T> k(a);
 
     const bool issuer = threadIdx.x == 0;
     if (issuer) {
@@ -562,7 +611,7 @@ __global__ void __launch_bounds__(32 * WPC, 1)
         mbar_init(reinterpret_cast<uint64_t*>(smem_raw + (c.bar(c.w, 1) - c.sbase)), 1 + 32 * (2 - nremote));
         fence_mbar_init();
     }
-    float2 xa[R][H], xb[R][H], ya[R][H], yb[R][H];
+    P xa[R][H], xb[R][H], ya[R][H], yb[R][H];
 #pragma unroll
     for (int r = 0; r < R; ++r) {
         rr_load<H>(lu_in + (size_t)(row0 + r) * N + col0, xa[r]);
@@ -573,7 +622,7 @@ __global__ void __launch_bounds__(32 * WPC, 1)
     cluster_wait();
     double g[6] = {0, 0, 0, 0, 0, 0};
     if (issuer)
-        for (int q = 0; q < S::kAhead && q < len; ++q) rr_adj_issue<N, WPC>(c, states, len, q, rc0);
+        for (int q = 0; q < S::kAhead && q < len; ++q) rr_adj_issue<N, WPC, T>(c, states, len, q, rc0);
     if (len > 0) {
         if (c.lane == 0) {
             rr_arm(c.bar(c.w, 0), c.tx);
@@ -585,25 +634,25 @@ __global__ void __launch_bounds__(32 * WPC, 1)
                    c.dn_remote, c.dn_rank, c.lane);
     }
     // gradient partial sums: float over the two steps of an iteration, then double
-    auto flush = [&](float2 (&t)[6]) {
+    auto flush = [&](P (&t)[6]) {
 #pragma unroll
         for (int q = 0; q < 6; ++q) {
             g[q] += (double)t[q].x + (double)t[q].y;
-            t[q] = f2(0.f);
+            t[q] = f2(T(0));
         }
     };
-    float2 t[6] = {f2(0.f), f2(0.f), f2(0.f), f2(0.f), f2(0.f), f2(0.f)};
+    P t[6] = {f2(T(0)), f2(T(0)), f2(T(0)), f2(T(0)), f2(T(0)), f2(T(0))};
     int s = 0;
     for (; s + 2 <= len; s += 2) {
-        if (issuer && s + S::kAhead < len) rr_adj_issue<N, WPC>(c, states, len, s + S::kAhead, rc0);
-        rr_adj_step<N, WPC, DRIFT>(c, k, xa, xb, ya, yb, s, true, t);
-        if (issuer && s + 1 + S::kAhead < len) rr_adj_issue<N, WPC>(c, states, len, s + 1 + S::kAhead, rc0);
-        rr_adj_step<N, WPC, DRIFT>(c, k, ya, yb, xa, xb, s + 1, s + 2 < len, t);
+        if (issuer && s + S::kAhead < len) rr_adj_issue<N, WPC, T>(c, states, len, s + S::kAhead, rc0);
+        rr_adj_step<N, WPC, DRIFT, T>(c, k, xa, xb, ya, yb, s, true, t);
+        if (issuer && s + 1 + S::kAhead < len) rr_adj_issue<N, WPC, T>(c, states, len, s + 1 + S::kAhead, rc0);
+        rr_adj_step<N, WPC, DRIFT, T>(c, k, ya, yb, xa, xb, s + 1, s + 2 < len, t);
         flush(t);
     }
     const bool odd = s < len;
     if (odd) {
-        rr_adj_step<N, WPC, DRIFT>(c, k, xa, xb, ya, yb, s, false, t);
+        rr_adj_step<N, WPC, DRIFT, T>(c, k, xa, xb, ya, yb, s, false, t);
         flush(t);
     }
     g[4] = -g[4];      // gs_adj_update2s accumulates the drift sums negated
@@ -613,14 +662,14 @@ __global__ void __launch_bounds__(32 * WPC, 1)
     cluster_wait();
     const bool bad = *c.failed != 0;
     if (bad && threadIdx.x == 0) atomicOr(err, 1);
-    const float nan = __int_as_float(0x7fc00000);
+    const T nan = (T)__int_as_float(0x7fc00000);
 #pragma unroll
     for (int r = 0; r < R; ++r) {
-        float2 pa[H], pb[H];
+        P pa[H], pb[H];
 #pragma unroll
         for (int j = 0; j < H; ++j) {
-            pa[j] = bad ? make_float2(nan, nan) : (odd ? ya[r][j] : xa[r][j]);
-            pb[j] = bad ? make_float2(nan, nan) : (odd ? yb[r][j] : xb[r][j]);
+            pa[j] = bad ? P{nan, nan} : (odd ? ya[r][j] : xa[r][j]);
+            pb[j] = bad ? P{nan, nan} : (odd ? yb[r][j] : xb[r][j]);
         }
         rr_store<H>(lu_out + (size_t)(row0 + r) * N + col0, pa);
         rr_store<H>(lv_out + (size_t)(row0 + r) * N + col0, pb);

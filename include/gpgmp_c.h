@@ -269,7 +269,7 @@ typedef struct gpgmp_gs_params {
     int32_t n;                  /* lattice side; a multiple of the cluster size */
     int32_t steps;
     double  F, k, Du, Dv, vx, vy, dt;
-    int32_t checkpoint_every;   /* <= 0: 100 in float32, 25 in float64 */
+    int32_t checkpoint_every;   /* <= 0: 100 in float32; in float64 25 at n = 256, up to 100 on smaller lattices */
     int32_t cluster;            /* CTAs per thread-block cluster, 0 = automatic */
     int32_t variant;            /* kernel family (float32): 0 automatic = for n = 256 the
                                    multi-cluster kernel 41 where the device holds its four clusters at
@@ -281,7 +281,8 @@ typedef struct gpgmp_gs_params {
                                    i = 0 (2, 8), 1 (4, 8), 2 (4, 16), 3 (8, 8), 4 (8, 16),
                                    5 (4, 32), 6 (2, 32), a CUDA error where the device cannot hold
                                    all its clusters at once.  Every float32 family gives the same
-                                   bits.  float64 always uses 0 / 1 (column walk / per cell).  The
+                                   bits.  float64: 0 register-resident at n 64 and 128 on a 16-CTA
+                                   cluster, else the column walk (2); 1 per cell.  The
                                    adjoint runs the multi-cluster adjoint under 40 + i (the same
                                    lambda bits); under 0, where the forward is multi-cluster, it
                                    recomputes the segments on two clusters (40) and runs the

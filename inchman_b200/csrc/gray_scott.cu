@@ -22,6 +22,7 @@
 #include <cooperative_groups.h>
 #include <cstdint>
 #include <cstdio>
+#include <map>
 #include <mutex>
 #include <type_traits>
 #include <vector>
@@ -530,6 +531,7 @@ __global__ void __launch_bounds__(512, 1) k_gs_adjoint_cw(GSArgs<T> a, const T* 
 #include "gs_rr.cuh"
 #include "gs_rb.cuh"
 #include "gs_mc.cuh"
+#include "gs_tile.cuh"
 
 // register-resident forward kernel for an n x n float32 lattice with *wpc warps per
 // CTA (*wpc = 0: the default split, written back), or NULL where the lattice does
@@ -750,6 +752,79 @@ cudaError_t mc_forward(int i, const GSArgs<float>& a0, bool drift, const float* 
     return mc_run(i, 0, drift, args, 7, st);
 }
 
+// ---- tiled kernels (gs_tile.cuh) -------------------------------------------------
+// sides with kernels of their own: their arithmetic is gs_update's, the other sides'
+// k_gs_forward's
+bool gs_own_side(int n) { return n == 64 || n == 128 || n == 256 || n == 512; }
+
+// the sides that take the tiled kernel under the automatic choice: those without a
+// register-resident kernel
+constexpr int kTileVariant = 50;
+bool tile_side(int n, int elem_bytes) {
+    return elem_bytes == 8 ? n != 64 && n != 128 : !gs_own_side(n);
+}
+
+template <typename T>
+const void* tile_kernel(int n, bool drift) {
+    if (!gs_own_side(n)) return (const void*)k_gs_forward_tile<T, 1, 1>;     // the drift terms are always there
+    return drift ? (const void*)k_gs_forward_tile<T, 1, 0> : (const void*)k_gs_forward_tile<T, 0, 0>;
+}
+int tile_count(int n) { return (n + kTileCore - 1) / kTileCore; }
+
+// whether all CTAs of an n x n lattice can be resident at once (cached per device and kernel)
+cudaError_t tile_fits(const void* fn, int n, bool* fits) {
+    static std::map<std::pair<int, const void*>, int> cache;
+    static std::mutex mu;
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    std::lock_guard<std::mutex> lock(mu);
+    int& most = cache[{dev, fn}];
+    if (most == 0) {
+        int per_sm = 0, sms = 0;
+        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, 32 * kTileWarps, 0);
+        if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+        if (e != cudaSuccess) return e;
+        most = std::max(1, per_sm * sms);
+    }
+    *fits = tile_count(n) * tile_count(n) <= most;
+    return cudaSuccess;
+}
+
+// one tiled launch: the exchange buffer from the stream-ordered pool (private to the launch),
+// cleared on the stream, then the kernel with `args` and the buffer and tile counts
+template <typename T>
+cudaError_t tile_run(const void* fn, int n, int steps, void** args, int nargs, cudaStream_t st) {
+    const size_t bytes = steps > kTileGhost ? (size_t)n * n * 2 * 2 * sizeof(uint64_t) * (sizeof(T) / 4) : 0;
+    uint64_t* xb = nullptr;
+    cudaError_t e = cudaSuccess;
+    if (bytes) {
+        e = pool_alloc((void**)&xb, bytes, st);
+        if (e != cudaSuccess) return e;
+        e = cudaMemsetAsync(xb, 0, bytes, st);
+    }
+    if (e == cudaSuccess) {
+        int tiles = tile_count(n);
+        void* all[16];
+        for (int q = 0; q < nargs; ++q) all[q] = args[q];
+        all[nargs] = &xb;
+        all[nargs + 1] = &tiles;
+        all[nargs + 2] = &tiles;
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(tiles * tiles, 1, 1);
+        cfg.blockDim = dim3(32 * kTileWarps, 1, 1);
+        cfg.stream = st;
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeCooperative;
+        attr[0].val.cooperative = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        e = cudaLaunchKernelExC(&cfg, fn, all);
+    }
+    cudaError_t e2 = pool_free(xb, st);
+    return e != cudaSuccess ? e : e2;
+}
+
 // register-resident adjoint kernel with wpc warps per CTA
 const void* rr_adj_kernel(int n, int* wpc, bool drift, size_t* smem) {
 #define GS_RRA_CASE(N_, W_)                                                                        \
@@ -880,6 +955,14 @@ cudaError_t gs_forward(const GSParams& p, const T* u0, const T* v0, T* u, T* v, 
     GSArgs<T> a{p.n, p.steps, (T)p.F, (T)p.k, (T)p.Du, (T)p.Dv, (T)p.vx, (T)p.vy, (T)p.dt};
     int every = trace_every > 0 ? trace_every : 1;
     void* args[] = {&a, (void*)&u0, (void*)&v0, &u, &v, &trace, &every};
+    if (p.variant == kTileVariant || (p.variant == 0 && p.cluster <= 0 && tile_side(p.n, (int)sizeof(T)))) {
+        const void* fn = tile_kernel<T>(p.n, p.vx != 0.0 || p.vy != 0.0);
+        bool fits = false;
+        cudaError_t e = tile_fits(fn, p.n, &fits);
+        if (e != cudaSuccess) return e;
+        if (fits) return tile_run<T>(fn, p.n, p.steps, args, 7, st);
+        if (p.variant != 0) return cudaErrorInvalidConfiguration;
+    }
     if constexpr (std::is_same<T, float>::value) {
         const bool drift = p.vx != 0.0 || p.vy != 0.0;
         if (p.variant >= kMCVariant && p.variant < kMCVariant + kMCConfigs) {
@@ -1033,6 +1116,15 @@ cudaError_t gs_auto_variant(int n, bool drift, int* variant) {
         if (e != cudaSuccess) return e;
         if (fits) {
             *variant = kMCVariant + kMCDefault;
+            return cudaSuccess;
+        }
+    }
+    if (cl > 0 && tile_side(n, 4)) {
+        bool fits = false;
+        cudaError_t e = tile_fits(tile_kernel<float>(n, drift), n, &fits);
+        if (e != cudaSuccess) return e;
+        if (fits) {
+            *variant = kTileVariant;
             return cudaSuccess;
         }
     }

@@ -274,15 +274,19 @@ typedef struct gpgmp_gs_params {
     int32_t variant;            /* kernel family (float32): 0 automatic = for n = 256 the
                                    multi-cluster kernel 41 where the device holds its four clusters at
                                    once, else register-resident where the lattice allows (n 64, 128,
-                                   256 on a 16-CTA cluster), else the shared-memory column walk;
+                                   256 on a 16-CTA cluster), else (cluster = 0) the tiled kernel 50
+                                   where the device holds all its tiles at once, else the
+                                   shared-memory column walk or 1;
                                    1 one cell per iteration; 2 shared-memory column walk;
                                    3 register-resident; 10 + w register-resident with w warps per
                                    CTA; 40 + i multi-cluster (n = 256; clusters, ghost rows):
                                    i = 0 (2, 8), 1 (4, 8), 2 (4, 16), 3 (8, 8), 4 (8, 16),
                                    5 (4, 32), 6 (2, 32), a CUDA error where the device cannot hold
-                                   all its clusters at once.  Every float32 family gives the same
-                                   bits.  float64: 0 register-resident at n 64 and 128 on a 16-CTA
-                                   cluster, else the column walk (2); 1 per cell.  The
+                                   all its clusters at once; 50 tiled, any n, a CUDA error where
+                                   the device cannot hold all its tiles at once.  Every float32
+                                   family gives the same bits (on sides other than 64, 128, 256,
+                                   512 those of 1).  float64: 0 register-resident at n 64 and 128
+                                   on a 16-CTA cluster, else 50 as above; 1; 2; 50.  The
                                    adjoint runs the multi-cluster adjoint under 40 + i (the same
                                    lambda bits); under 0, where the forward is multi-cluster, it
                                    recomputes the segments on two clusters (40) and runs the

@@ -40,113 +40,282 @@ constexpr int kScanTile = kScanThreads * kScanItems;   // 16384
 // ---- exclusive scan ------------------------------------------------------------
 // scratch: [0] tile counter, [1] error word, then one status word per tile:
 // (flag << 32) | value, flag 0 = not ready, 1 = tile aggregate, 2 = inclusive prefix.
-// A tile is 512 threads x 32 consecutive values (16384: fewer tiles, a shorter
-// look-back chain).  Every tile moves through shared memory, one uint4 of padding per
-// eight so that a thread's 128-byte row reads and writes without bank conflicts: a
-// full tile whose pointers are 16-byte aligned (vec) with warp-contiguous 16-byte loads
-// and stores (every HBM request coalesced), a partial tile or unaligned pointers with
-// coalesced element loads and stores.  A thread sums its row from shared memory, and
-// after the look-back writes its row's exclusive prefixes back in place: the values
-// never sit in registers, so three CTAs fit on an SM (shared memory is the limit)
-// instead of two (registers were), and more loads are in flight while tiles wait in
-// the look-back.
-constexpr int kScanQuads = kScanTile / 4;                 // uint4 per tile
-__device__ __forceinline__ int scan_pad(int i4) { return i4 + (i4 >> 3); }
-// word index of value i of the tile in the padded layout
-__device__ __forceinline__ int scan_word(int i) { return 4 * scan_pad(i >> 2) + (i & 3); }
+// A tile is 16384 values, 1024 consecutive ones per warp, which a warp holds in registers as
+// eight rows of 32 16-byte quads: every load and store is one coalesced 512-byte row, and
+// the exclusive sums come from shuffles over the eight rows at once, so nothing but the
+// warps' totals passes through shared memory (partial tiles and unaligned pointers take
+// element loads in the same places).
+// A scan of one tile needs neither the counter nor status words (tiles == 1): it clears the
+// error word itself and the scratch is not cleared before.
+// A warp's 128 ROWS values in registers, as rows of 32 quads, and their exclusive sums.
+template <int ROWS>
+struct ScanTile {
+    static constexpr int kValues = 128 * ROWS;
+    uint4 v[ROWS];
+    uint32_t ex[ROWS];           // sum of the warp's values before the lane's quad of row j
+    // row: 128 words of shared memory of the warp's own, for the element loads and stores
+    __device__ __forceinline__ void load(const uint32_t* __restrict__ in, int64_t wbase, int64_t n, int vec, int lane,
+                                         uint32_t* row) {
+        if (vec && wbase + kValues <= n) {      // the same in every lane
+            const uint4* src = reinterpret_cast<const uint4*>(in + wbase) + lane;
+#pragma unroll
+            for (int j = 0; j < ROWS; ++j) v[j] = src[j * 32];
+            return;
+        }
+        const auto at = [&](int64_t i) { return i < n ? in[i] : 0u; };
+#pragma unroll
+        for (int j = 0; j < ROWS; ++j) {
+            const int64_t i = wbase + j * 128 + lane;
+            v[j] = make_uint4(at(i), at(i + 32), at(i + 64), at(i + 96));
+        }
+#pragma unroll
+        for (int j = 0; j < ROWS; ++j) {
+            row[lane] = v[j].x;
+            row[lane + 32] = v[j].y;
+            row[lane + 64] = v[j].z;
+            row[lane + 96] = v[j].w;
+            __syncwarp();
+            v[j] = reinterpret_cast<const uint4*>(row)[lane];
+            __syncwarp();
+        }
+    }
+    // returns the warp's total
+    __device__ __forceinline__ uint32_t sum(int lane) {
+#pragma unroll
+        for (int j = 0; j < ROWS; ++j) ex[j] = (v[j].x + v[j].y) + (v[j].z + v[j].w);
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+#pragma unroll
+            for (int j = 0; j < ROWS; ++j) {
+                const uint32_t t = __shfl_up_sync(0xffffffffu, ex[j], o);
+                if (lane >= o) ex[j] += t;
+            }
+        }
+        uint32_t total = 0;
+#pragma unroll
+        for (int j = 0; j < ROWS; ++j) {
+            const uint32_t row = __shfl_sync(0xffffffffu, ex[j], 31);
+            ex[j] += total - ((v[j].x + v[j].y) + (v[j].z + v[j].w));
+            total += row;
+        }
+        return total;
+    }
+    __device__ __forceinline__ void store(uint32_t* __restrict__ out, int64_t wbase, int64_t n, int vec, int lane,
+                                          uint32_t base, uint32_t* row) const {
+        const bool full = vec && wbase + kValues <= n;
+        uint4* dst = reinterpret_cast<uint4*>(out + wbase) + lane;
+#pragma unroll
+        for (int j = 0; j < ROWS; ++j) {
+            uint4 w;
+            w.x = base + ex[j];
+            w.y = w.x + v[j].x;
+            w.z = w.y + v[j].y;
+            w.w = w.z + v[j].z;
+            if (full) {
+                dst[j * 32] = w;
+                continue;
+            }
+            reinterpret_cast<uint4*>(row)[lane] = w;
+            __syncwarp();
+#pragma unroll
+            for (int c = 0; c < 128; c += 32) {
+                const int64_t i = wbase + j * 128 + c + lane;
+                if (i < n) out[i] = row[c + lane];
+            }
+            __syncwarp();
+        }
+    }
+};
 
-__global__ void __launch_bounds__(kScanThreads, 3) k_scan_exclusive(const uint32_t* __restrict__ in,
+// exclusive sums of W warps' totals (called by one warp): returns lane w's warp's, *sum all
+template <int W>
+__device__ __forceinline__ uint32_t scan_warps(uint32_t mine, int lane, uint32_t* sum) {
+    uint32_t incl = mine;
+#pragma unroll
+    for (int o = 1; o < W; o <<= 1) {
+        const uint32_t t = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += t;
+    }
+    *sum = __shfl_sync(0xffffffffu, incl, W - 1);
+    return incl - mine;
+}
+
+constexpr int kScanWarps = kScanThreads / 32;
+__global__ void __launch_bounds__(kScanThreads, 2) k_scan_exclusive(const uint32_t* __restrict__ in,
                                                                     uint32_t* __restrict__ out, int64_t n,
-                                                                    uint64_t* __restrict__ scratch, int vec) {
-    extern __shared__ uint4 s_io[];   // kScanQuads + kScanQuads / 8 (dynamic: 72 KB)
-    uint32_t* s_w32 = reinterpret_cast<uint32_t*>(s_io);
+                                                                    uint64_t* __restrict__ scratch, int vec,
+                                                                    uint32_t tiles) {
     __shared__ uint32_t s_tile;
-    __shared__ uint32_t s_warp[kScanThreads / 32];
-    __shared__ uint32_t s_prefix;
+    __shared__ uint32_t s_warp[kScanWarps], s_base[kScanWarps];
+    __shared__ __align__(16) uint32_t s_row[kScanWarps][128];
     unsigned int* counter = reinterpret_cast<unsigned int*>(scratch);
     int* err = reinterpret_cast<int*>(scratch) + 2;
     uint64_t* status = scratch + 2;
-    if (threadIdx.x == 0) s_tile = atomicAdd(counter, 1u);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (threadIdx.x == 0) {
+        s_tile = tiles > 1 ? atomicAdd(counter, 1u) : 0u;
+        if (tiles == 1) *err = 0;
+    }
     __syncthreads();
     const uint32_t tile = s_tile;
-    const int64_t tbase = (int64_t)tile * kScanTile;
-    const bool full = vec && tbase + kScanTile <= n;    // the same in every thread of the block
-    if (full) {
-        const uint4* src = reinterpret_cast<const uint4*>(in + tbase);
-#pragma unroll
-        for (int q = 0; q < kScanItems / 4; ++q) {
-            const int i4 = q * kScanThreads + threadIdx.x;
-            s_io[scan_pad(i4)] = src[i4];
-        }
-    } else {
-        for (int q = 0; q < kScanItems; ++q) {
-            const int i = q * kScanThreads + threadIdx.x;
-            s_w32[scan_word(i)] = tbase + i < n ? in[tbase + i] : 0u;
-        }
+    const int64_t wbase = (int64_t)tile * kScanTile + warp * (32 * kScanItems);
+    ScanTile<kScanItems / 4> t;
+    t.load(in, wbase, n, vec, lane, s_row[warp]);
+    const uint32_t total = t.sum(lane);
+    if (lane == 0) s_warp[warp] = total;
+    __syncthreads();
+    if (warp == 0) {
+        uint32_t aggregate;
+        const uint32_t ex = scan_warps<kScanWarps>(lane < kScanWarps ? s_warp[lane] : 0u, lane, &aggregate);
+        const uint32_t prefix = tiles > 1 ? warp_lookback_u32(status, tile, aggregate, err) : 0u;
+        if (lane < kScanWarps) s_base[lane] = prefix + ex;
     }
     __syncthreads();
-    // the thread's row: values threadIdx.x * 32 .. + 31 of the tile
-    const int row = threadIdx.x * (kScanItems / 4);
-    uint32_t sum = 0;
-#pragma unroll
-    for (int q = 0; q < kScanItems / 4; ++q) {
-        const uint4 w = s_io[scan_pad(row + q)];
-        sum += w.x + w.y + w.z + w.w;
-    }
-    // block exclusive scan of the thread sums
+    t.store(out, wbase, n, vec, lane, s_base[warp], s_row[warp]);
+}
+
+// Large scans: one CTA per SM, all of them resident (cooperative launch), in rounds of one
+// tile per CTA.  A CTA publishes its tile's sum and reads every CTA's of the round: the sums
+// before its own give its prefix, all of them the carry into the next round, so there is no
+// chain of look-backs.  A sum takes 2 to 4 us to reach the other SMs while memory is busy,
+// longer than a tile's share of the bandwidth (3 us), so a CTA keeps three tiles in shared
+// memory: one loading (bulk copy), one whose sum is published, one whose round is complete
+// and which is written.  2^27 values: 214 us, 5.0 TB/s (306 us with every tile staged in
+// shared memory by its own CTA and chained look-backs; 459 us in rounds without the third
+// tile; HBM's floor is 166).
+constexpr int kStreamThreads = 1024, kStreamWarps = kStreamThreads / 32, kStreamStages = 3;
+constexpr int kStreamRows = kScanTile / (128 * kStreamWarps);
+constexpr int kStreamSmem = kStreamStages * kScanTile * (int)sizeof(uint32_t);
+__device__ __forceinline__ uint32_t scan_smem(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+
+__global__ void __launch_bounds__(kStreamThreads, 1) k_scan_stream(const uint32_t* __restrict__ in,
+                                                                   uint32_t* __restrict__ out, int64_t n,
+                                                                   uint64_t* __restrict__ scratch, uint32_t tiles) {
+    extern __shared__ __align__(128) uint32_t s_ring[];      // [stage][kScanTile]
+    __shared__ __align__(8) uint64_t s_full[kStreamStages];
+    __shared__ uint32_t s_warp[kStreamWarps], s_base[kStreamWarps];
+    __shared__ __align__(16) uint32_t s_row[kStreamWarps][128];
+    int* err = reinterpret_cast<int*>(scratch) + 2;
+    uint64_t* status = scratch + 2;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    uint32_t incl = sum;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        uint32_t t = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= o) incl += t;
-    }
-    if (lane == 31) s_warp[warp] = incl;
-    __syncthreads();
-    if (warp == 0) {
-        uint32_t w = lane < kScanThreads / 32 ? s_warp[lane] : 0u;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            uint32_t t = __shfl_up_sync(0xffffffffu, w, o);
-            if (lane >= o) w += t;
+    const uint32_t G = gridDim.x, rank = blockIdx.x;
+    const uint32_t mine = rank < tiles ? (tiles - rank + G - 1) / G : 0;      // tiles rank, rank + G, ...
+    const auto first = [&](uint32_t i) { return ((int64_t)i * G + rank) * kScanTile; };
+    const auto whole = [&](uint32_t i) { return first(i) + kScanTile <= n; };  // all but the last tile of all
+    const auto issue = [&](uint32_t i) {
+        const uint32_t bar = scan_smem(&s_full[i % kStreamStages]);
+        constexpr uint32_t bytes = kScanTile * sizeof(uint32_t);
+        asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(bar), "r"(bytes) : "memory");
+        asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n" ::"r"(
+                         scan_smem(s_ring + (i % kStreamStages) * kScanTile)),
+                     "l"(in + first(i)), "r"(bytes), "r"(bar)
+                     : "memory");
+    };
+    const auto wait = [&](uint32_t i) {
+        const uint32_t bar = scan_smem(&s_full[i % kStreamStages]), parity = (i / kStreamStages) & 1u;
+        for (uint32_t spins = 0;; ++spins) {
+            uint32_t ok;
+            asm volatile(
+                "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
+                : "=r"(ok)
+                : "r"(bar), "r"(parity)
+                : "memory");
+            if (ok) return;
+            if (spins == kSpinLimit) {
+                atomicExch(err, 1);
+                return;
+            }
         }
-        if (lane < kScanThreads / 32) s_warp[lane] = w;   // inclusive over warps
-    }
-    __syncthreads();
-    const uint32_t warp_excl = warp == 0 ? 0u : s_warp[warp - 1];
-    const uint32_t thread_excl = warp_excl + incl - sum;
-    const uint32_t aggregate = s_warp[kScanThreads / 32 - 1];
-    // decoupled look-back by warp 0
-    if (warp == 0) {
-        const uint32_t exclusive = warp_lookback_u32(status, tile, aggregate, err);
-        if (lane == 0) s_prefix = exclusive;
-    }
-    __syncthreads();
-    // the row's exclusive prefixes, in place
-    uint32_t run = s_prefix + thread_excl;
+    };
+    ScanTile<kStreamRows> t;
+    const auto read = [&](uint32_t i) {
+        const uint4* q = reinterpret_cast<const uint4*>(s_ring + (i % kStreamStages) * kScanTile) +
+                         warp * (32 * kStreamRows) + lane;
 #pragma unroll
-    for (int q = 0; q < kScanItems / 4; ++q) {
-        const uint4 v = s_io[scan_pad(row + q)];
-        uint4 w;
-        w.x = run; run += v.x;
-        w.y = run; run += v.y;
-        w.z = run; run += v.z;
-        w.w = run; run += v.w;
-        s_io[scan_pad(row + q)] = w;
+        for (int j = 0; j < kStreamRows; ++j) t.v[j] = q[j * 32];
+    };
+    // the sums of tile i's warps into s_warp (the caller syncs)
+    const auto sums = [&](uint32_t i) {
+        if (whole(i)) {
+            wait(i);
+        } else {
+            uint32_t* q = s_ring + (i % kStreamStages) * kScanTile;
+            for (int k = threadIdx.x; k < kScanTile; k += kStreamThreads) q[k] = first(i) + k < n ? in[first(i) + k] : 0u;
+            __syncthreads();       // the same in every thread of the block
+        }
+        read(i);
+        uint32_t x = 0;
+#pragma unroll
+        for (int j = 0; j < kStreamRows; ++j) x += (t.v[j].x + t.v[j].y) + (t.v[j].z + t.v[j].w);
+        x = __reduce_add_sync(0xffffffffu, x);
+        if (lane == 0) s_warp[warp] = x;
+    };
+    if (threadIdx.x == 0) {
+        for (int b = 0; b < kStreamStages; ++b)
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(scan_smem(&s_full[b])) : "memory");
+        asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+        for (uint32_t i = 0; i < kStreamStages && i < mine; ++i)
+            if (whole(i)) issue(i);
     }
     __syncthreads();
-    if (full) {
-        uint4* dst = reinterpret_cast<uint4*>(out + tbase);
+    uint32_t carry = 0, ex = 0;       // warp 0: the sum of all earlier rounds; the tile's sums before each warp
+    if (mine > 0) {
+        sums(0);
+        __syncthreads();
+        if (warp == 0) {
+            uint32_t aggregate;
+            ex = scan_warps<kStreamWarps>(s_warp[lane], lane, &aggregate);
+            if (lane == 0) st_relaxed_u64(&status[rank], kScanFlagA | aggregate);
+        }
+        __syncthreads();
+    }
+    for (uint32_t i = 0; i < mine; ++i) {
+        if (i + 1 < mine) sums(i + 1);
+        __syncthreads();
+        if (warp == 0) {
+            uint32_t ex_next = 0;
+            if (i + 1 < mine) {
+                uint32_t aggregate;
+                ex_next = scan_warps<kStreamWarps>(s_warp[lane], lane, &aggregate);
+                if (lane == 0) st_relaxed_u64(&status[(i + 1) * G + rank], kScanFlagA | aggregate);
+            }
+            const uint32_t r0 = i * G;
+            uint32_t before = 0, all = 0, spins = 0;
+            for (uint32_t q0 = 0; q0 < G; q0 += 32 * 5) {
+                uint64_t w[5];
+                bool ready;
+                do {
+                    ready = true;
 #pragma unroll
-        for (int q = 0; q < kScanItems / 4; ++q) {
-            const int i4 = q * kScanThreads + threadIdx.x;
-            dst[i4] = s_io[scan_pad(i4)];
+                    for (int u = 0; u < 5; ++u) {
+                        const uint32_t q = q0 + 32 * u + lane;
+                        w[u] = q < G && r0 + q < tiles ? ld_volatile_u64(&status[r0 + q]) : kScanFlagA;
+                        ready = ready && (w[u] >> 32) != 0;
+                    }
+                    if (!ready && ++spins > kSpinLimit) {
+                        atomicExch(err, 1);
+                        ready = true;
+                    }
+                } while (!__all_sync(0xffffffffu, ready));
+#pragma unroll
+                for (int u = 0; u < 5; ++u) {
+                    all += (uint32_t)w[u];
+                    if (q0 + 32 * u + lane < rank) before += (uint32_t)w[u];
+                }
+            }
+            before = __reduce_add_sync(0xffffffffu, before);
+            all = __reduce_add_sync(0xffffffffu, all);
+            s_base[lane] = carry + before + ex;
+            carry += all;
+            ex = ex_next;
         }
-    } else {
-        for (int q = 0; q < kScanItems; ++q) {
-            const int i = q * kScanThreads + threadIdx.x;
-            if (tbase + i < n) out[tbase + i] = s_w32[scan_word(i)];
-        }
+        __syncthreads();
+        read(i);
+        t.sum(lane);
+        t.store(out, first(i) + warp * t.kValues, n, 1, lane, s_base[warp], s_row[warp]);
+        __syncthreads();
+        if (threadIdx.x == 0 && i + kStreamStages < mine && whole(i + kStreamStages)) issue(i + kStreamStages);
     }
 }
 
@@ -582,16 +751,60 @@ size_t scan_scratch_bytes(int64_t n) {
     return (size_t)(2 + tiles) * sizeof(uint64_t);
 }
 
+// Scans of more than one tile per SM stream (us, look-back -> stream: 2^22 values 14.7 ->
+// 13.7, 2^24 47 -> 35, 2^27 325 -> 214; below, both wait for the launch), where the pointers
+// are 16-byte aligned as the bulk copies want them.  *sms: the device's SMs if each holds the
+// kernel's one CTA, else 0; cached per device.
+constexpr int64_t kStreamMinTiles = 64;
+static cudaError_t stream_sms(int* sms) {
+    static std::mutex mu;
+    static int cache[64];        // 0: not asked yet, -1: the kernel does not fit
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    *sms = 0;
+    if (dev < 0 || dev >= 64) return cudaSuccess;
+    std::lock_guard<std::mutex> lock(mu);
+    if (cache[dev] == 0) {
+        int per_sm = 0, n = 0;
+        e = cudaFuncSetAttribute(k_scan_stream, cudaFuncAttributeMaxDynamicSharedMemorySize, kStreamSmem);
+        if (e == cudaSuccess)
+            e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_scan_stream, kStreamThreads, kStreamSmem);
+        if (e == cudaSuccess) e = cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
+        if (e != cudaSuccess) return e;
+        cache[dev] = per_sm >= 1 ? n : -1;
+    }
+    *sms = cache[dev] > 0 ? cache[dev] : 0;
+    return cudaSuccess;
+}
+
 cudaError_t scan_exclusive_u32(const uint32_t* in, uint32_t* out, int64_t n, void* scratch, cudaStream_t st) {
     if (n <= 0) return cudaSuccess;
     const int64_t tiles = (n + kScanTile - 1) / kScanTile;
-    cudaError_t e = cudaMemsetAsync(scratch, 0, scan_scratch_bytes(n), st);
-    if (e != cudaSuccess) return e;
+    if (tiles > 1) {
+        cudaError_t e = cudaMemsetAsync(scratch, 0, scan_scratch_bytes(n), st);
+        if (e != cudaSuccess) return e;
+    }
     const int vec = (((uintptr_t)in | (uintptr_t)out) & 15u) == 0 ? 1 : 0;
-    const int smem = (int)(sizeof(uint4) * (kScanQuads + kScanQuads / 8));
-    e = cudaFuncSetAttribute(k_scan_exclusive, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) return e;
-    k_scan_exclusive<<<(unsigned)tiles, kScanThreads, smem, st>>>(in, out, n, (uint64_t*)scratch, vec);
+    int sms = 0;
+    if (vec && tiles > kStreamMinTiles) {
+        cudaError_t e = stream_sms(&sms);
+        if (e != cudaSuccess) return e;
+    }
+    if (tiles > sms && sms > 0) {
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(sms, 1, 1);
+        cfg.blockDim = dim3(kStreamThreads, 1, 1);
+        cfg.dynamicSmemBytes = kStreamSmem;
+        cfg.stream = st;
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeCooperative;
+        attr[0].val.cooperative = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        return cudaLaunchKernelEx(&cfg, k_scan_stream, in, out, n, (uint64_t*)scratch, (uint32_t)tiles);
+    }
+    k_scan_exclusive<<<(unsigned)tiles, kScanThreads, 0, st>>>(in, out, n, (uint64_t*)scratch, vec, (uint32_t)tiles);
     return cudaGetLastError();
 }
 

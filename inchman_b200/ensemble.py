@@ -44,9 +44,15 @@ _SIGS = {
 _lib.SIGNATURES.update(_SIGS)
 
 
+_FNS = {}
+
+
 def _fn(name):
-    f = getattr(_lib.lib(), name)
-    f.restype, f.argtypes = _SIGS[name]
+    f = _FNS.get(name)
+    if f is None:          # the signature is set once: it costs more than a small call
+        f = getattr(_lib.lib(), name)
+        f.restype, f.argtypes = _SIGS[name]
+        _FNS[name] = f
     return f
 
 

@@ -45,11 +45,15 @@ _SIGS = {
 _lib.SIGNATURES.update(_SIGS)
 
 
+_FNS = {}
+
+
 def _fn(name):
-    L = _lib.lib()
-    f = getattr(L, name)
-    res, args = _SIGS[name]
-    f.restype, f.argtypes = res, args
+    f = _FNS.get(name)
+    if f is None:          # the signature is set once: it costs more than a small call
+        f = getattr(_lib.lib(), name)
+        f.restype, f.argtypes = _SIGS[name]
+        _FNS[name] = f
     return f
 
 

@@ -44,9 +44,15 @@ _SIGS = {
 _lib.SIGNATURES.update(_SIGS)
 
 
+_FNS = {}
+
+
 def _fn(name):
-    f = getattr(_lib.lib(), name)
-    f.restype, f.argtypes = _SIGS[name]
+    f = _FNS.get(name)
+    if f is None:          # the signature is set once: it costs more than a small call
+        f = getattr(_lib.lib(), name)
+        f.restype, f.argtypes = _SIGS[name]
+        _FNS[name] = f
     return f
 
 
@@ -56,11 +62,12 @@ def _call(name, *args):
 
 def _stream():
     import torch
-    return C.c_void_p(torch.cuda.current_stream().cuda_stream)
+    raw = getattr(torch._C, "_cuda_getCurrentRawStream", None)     # a third of a small call otherwise
+    return raw(torch.cuda.current_device()) if raw else torch.cuda.current_stream().cuda_stream
 
 
 def _ptr(t):
-    return C.c_void_p(t.data_ptr()) if t is not None else None
+    return t.data_ptr() if t is not None else None
 
 
 def scan_scratch(n: int, device="cuda"):

@@ -705,6 +705,132 @@ __global__ void __launch_bounds__(SortShape<RB>::kThreads, SortShape<RB>::kMinBl
     }
 }
 
+// ---- small lists ----------------------------------------------------------------
+// Up to 8192 pairs in one CTA: LSD passes of 5-bit digits between registers and shared
+// memory, so that a sort of a short list is one launch instead of a clear, a histogram and a
+// kernel per 8-bit digit, whose latencies add up (4096 pairs, 10-bit keys: 23 us a call, now 12,
+// 9 of them the kernel).
+// A warp owns 32 ITEMS consecutive pairs; five ballots give each lane the lanes that share
+// its item's digit and the count of the digit whose number it bears, so a lane keeps one
+// digit's running count in a register.  The counts of all warps (32 x 32, digit-major) are
+// scanned once per pass.
+constexpr int kSmallThreads = 1024, kSmallMax = 8 * kSmallThreads;
+template <int ITEMS>
+__global__ void __launch_bounds__(kSmallThreads) k_sort_small(const uint32_t* __restrict__ kin,
+                                                              const uint32_t* __restrict__ vin,
+                                                              uint32_t* __restrict__ kout, uint32_t* __restrict__ vout,
+                                                              int n, int key_bits, int* __restrict__ err) {
+    extern __shared__ uint32_t s_pairs[];                     // keys, then values
+    __shared__ uint32_t s_count[32 * 32], s_warp[32];
+    uint32_t* s_k = s_pairs;
+    uint32_t* s_v = s_pairs + ITEMS * kSmallThreads;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int base = warp * 32 * ITEMS + lane;
+    if (threadIdx.x == 0) *err = 0;
+    uint32_t key[ITEMS], val[ITEMS], pos[ITEMS];
+#pragma unroll
+    for (int j = 0; j < ITEMS; ++j) {
+        const int i = base + 32 * j;
+        key[j] = i < n ? kin[i] : 0xffffffffu;      // past the end: digit 31 of every pass, after the rest
+        val[j] = i < n ? vin[i] : 0u;
+    }
+    for (int shift = 0; shift < key_bits; shift += 5) {
+        const uint32_t mask = key_bits - shift >= 5 ? 31u : (1u << (key_bits - shift)) - 1u;
+        uint32_t mine = 0;                          // pairs of digit `lane` so far in this warp
+#pragma unroll
+        for (int j = 0; j < ITEMS; ++j) {
+            const uint32_t d = base + 32 * j < n || shift > 0 ? (key[j] >> shift) & mask : mask;
+            uint32_t peers = 0xffffffffu, own = 0xffffffffu;
+#pragma unroll
+            for (int b = 0; b < 5; ++b) {
+                const uint32_t bal = __ballot_sync(0xffffffffu, (d >> b) & 1u);
+                peers &= (d >> b) & 1u ? bal : ~bal;
+                own &= (lane >> b) & 1 ? bal : ~bal;
+            }
+            pos[j] = __shfl_sync(0xffffffffu, mine, (int)d) + __popc(peers & ((1u << lane) - 1u));
+            mine += __popc(own);
+        }
+        s_count[lane * 32 + warp] = mine;
+        __syncthreads();
+        // exclusive scan in (digit, warp) order: thread 32 d + w holds digit d of warp w
+        const uint32_t c = s_count[threadIdx.x];
+        uint32_t incl = c;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t t = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += t;
+        }
+        if (lane == 31) s_warp[warp] = incl;
+        __syncthreads();
+        uint32_t before = lane < warp ? s_warp[lane] : 0u;
+        before = __reduce_add_sync(0xffffffffu, before);
+        s_count[threadIdx.x] = before + incl - c;
+        __syncthreads();
+        const uint32_t start = s_count[lane * 32 + warp];      // of digit `lane` in this warp
+#pragma unroll
+        for (int j = 0; j < ITEMS; ++j) {
+            const uint32_t d = base + 32 * j < n || shift > 0 ? (key[j] >> shift) & mask : mask;
+            const uint32_t p = pos[j] + __shfl_sync(0xffffffffu, start, (int)d);
+            s_k[p] = key[j];
+            s_v[p] = val[j];
+        }
+        __syncthreads();
+#pragma unroll
+        for (int j = 0; j < ITEMS; ++j) {
+            key[j] = s_k[base + 32 * j];
+            val[j] = s_v[base + 32 * j];
+        }
+    }
+#pragma unroll
+    for (int j = 0; j < ITEMS; ++j) {
+        const int i = base + 32 * j;
+        if (i < n) {
+            kout[i] = key[j];
+            vout[i] = val[j];
+        }
+    }
+}
+
+// Cell starts and counts of a short list over few cells in one CTA: a histogram in shared
+// memory and its scan, instead of two clears, a histogram and a scan.
+constexpr int64_t kSmallCells = 16384, kSmallKeys = 32768;
+__global__ void __launch_bounds__(kSmallThreads) k_cells_small(const uint32_t* __restrict__ keys, int n, int ncells,
+                                                               uint32_t* __restrict__ start,
+                                                               uint32_t* __restrict__ count, int* __restrict__ err) {
+    extern __shared__ uint32_t s_cells[];          // kSmallThreads * per words
+    __shared__ uint32_t s_warp[32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int per = (ncells + kSmallThreads - 1) / kSmallThreads;
+    if (threadIdx.x == 0) *err = 0;
+    for (int c = threadIdx.x; c < per * kSmallThreads; c += kSmallThreads) s_cells[c] = 0;
+    __syncthreads();
+    for (int i = threadIdx.x; i < n; i += kSmallThreads) {
+        const uint32_t k = keys[i];
+        if (k < (uint32_t)ncells) atomicAdd(&s_cells[k], 1u);
+    }
+    __syncthreads();
+    for (int c = threadIdx.x; c < ncells; c += kSmallThreads) count[c] = s_cells[c];
+    uint32_t sum = 0;
+    for (int q = 0; q < per; ++q) sum += s_cells[threadIdx.x * per + q];
+    uint32_t incl = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t t = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += t;
+    }
+    if (lane == 31) s_warp[warp] = incl;
+    __syncthreads();
+    uint32_t run = __reduce_add_sync(0xffffffffu, lane < warp ? s_warp[lane] : 0u) + incl - sum;
+    for (int q = 0; q < per; ++q) {
+        const int c = threadIdx.x * per + q;
+        const uint32_t k = s_cells[c];
+        s_cells[c] = run;
+        run += k;
+    }
+    __syncthreads();
+    for (int c = threadIdx.x; c < ncells; c += kSmallThreads) start[c] = s_cells[c];
+}
+
 // Counts per cell.  Equal neighbours within a warp are added as one run (the keys come
 // sorted, so a warp holds a few runs): the last lane of each run adds its length.
 __global__ void k_histogram_cells(const uint32_t* __restrict__ keys, int64_t n, uint32_t ncells,
@@ -888,12 +1014,31 @@ cudaError_t radix_sort_finish(const uint32_t* kin, const uint32_t* vin, uint32_t
     return cudaSuccess;
 }
 
+static cudaError_t sort_small(const uint32_t* kin, const uint32_t* vin, uint32_t* kout, uint32_t* vout, int n,
+                              int key_bits, int* err, cudaStream_t st) {
+    const auto launch = [&](auto kernel, int items) -> cudaError_t {
+        const int smem = 2 * items * kSmallThreads * (int)sizeof(uint32_t);
+        if (smem > 48 * 1024) {
+            cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+            if (e != cudaSuccess) return e;
+        }
+        kernel<<<1, kSmallThreads, smem, st>>>(kin, vin, kout, vout, n, key_bits, err);
+        return cudaGetLastError();
+    };
+    if (n <= kSmallThreads) return launch(k_sort_small<1>, 1);
+    if (n <= 2 * kSmallThreads) return launch(k_sort_small<2>, 2);
+    if (n <= 4 * kSmallThreads) return launch(k_sort_small<4>, 4);
+    return launch(k_sort_small<8>, 8);
+}
+
 cudaError_t radix_sort_pairs_u32(const uint32_t* kin, const uint32_t* vin, uint32_t* kout, uint32_t* vout, int64_t n,
                                  int key_bits, void* scratch, cudaStream_t st, uint32_t* cell_count, int64_t ncells) {
     if (n <= 0) return cudaSuccess;
+    const SortLayout L = sort_layout(n, key_bits);
+    if (n <= kSmallMax && !cell_count)
+        return sort_small(kin, vin, kout, vout, (int)n, key_bits, (int*)((char*)scratch + L.off_counters) + 4, st);
     cudaError_t e = radix_sort_begin(n, key_bits, scratch, st);
     if (e != cudaSuccess) return e;
-    const SortLayout L = sort_layout(n, key_bits);
     uint32_t* hist = radix_sort_hist(n, key_bits, scratch);
     // about 16 keys per thread, at most two CTAs per SM
     int64_t hb = (n + (int64_t)kHistThreads * 16 - 1) / ((int64_t)kHistThreads * 16);
@@ -915,6 +1060,16 @@ cudaError_t cell_counts_u32(const uint32_t* sorted_keys, int64_t n, int64_t ncel
 
 cudaError_t cell_offsets_u32(const uint32_t* sorted_keys, int64_t n, int64_t ncells, uint32_t* start, uint32_t* count,
                              void* scan_scratch, cudaStream_t st) {
+    if (n <= kSmallKeys && ncells <= kSmallCells) {
+        const int smem = (int)((ncells + kSmallThreads - 1) / kSmallThreads * kSmallThreads * sizeof(uint32_t));
+        if (smem > 48 * 1024) {
+            cudaError_t e = cudaFuncSetAttribute(k_cells_small, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+            if (e != cudaSuccess) return e;
+        }
+        k_cells_small<<<1, kSmallThreads, smem, st>>>(sorted_keys, (int)n, (int)ncells, start, count,
+                                                      (int*)scan_scratch + 2);
+        return cudaGetLastError();
+    }
     cudaError_t e = cell_counts_u32(sorted_keys, n, ncells, count, st);
     if (e != cudaSuccess) return e;
     return scan_exclusive_u32(count, start, ncells, scan_scratch, st);

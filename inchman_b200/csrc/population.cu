@@ -40,8 +40,12 @@ namespace gpgmp {
 namespace {
 
 constexpr int kPlanThreads = 512;
-constexpr int kPlanItems = 8;
-constexpr int kPlanTile = kPlanThreads * kPlanItems;   // 4096 cells
+// cells per thread of a plan tile: 1 while a tile per SM covers the grid, 2 while two do
+// (a small grid's cells are spread over the chip, and over the lanes that draw: 1024 cells
+// 13 us with 8, 6 with 1), 8 above
+inline int plan_items(int64_t ncells) {
+    return ncells <= 148 * kPlanThreads ? 1 : ncells <= 148 * 2 * 2 * kPlanThreads ? 2 : 8;
+}
 constexpr int kMoveThreads = 256;
 constexpr int kMoveUnroll = 4;   // independent loads in flight per thread
 constexpr uint32_t kMaskCell = 32;     // cells of at most this many individuals get a removal mask
@@ -121,11 +125,13 @@ __device__ __forceinline__ void warp_masks(const uint32_t* list, uint32_t* mask,
 // Cells are read and written warp-striped (item q of lane l of warp w is cell
 // tile_base + 256 w + 32 q + l for 8 items), so every access is one coalesced 128-byte row; the
 // scans run in that order: a warp scan per item row, carried across the rows.
+template <int kPlanItems>
 __global__ void __launch_bounds__(kPlanThreads, 2)
     k_pop_plan(const uint32_t* __restrict__ start, const uint32_t* __restrict__ count,
                const int32_t* __restrict__ goal, int64_t ncells, uint32_t seed, uint32_t step,
                uint32_t* __restrict__ new_start, uint32_t* __restrict__ birth_off, CellPlan* __restrict__ plan,
                PopHeader* __restrict__ head, uint64_t* __restrict__ status, int64_t tiles) {
+    constexpr int kPlanTile = kPlanThreads * kPlanItems;
     __shared__ uint32_t s_tile;
     __shared__ uint32_t s_warp[3][kPlanThreads / 32];
     __shared__ uint32_t s_prefix[3];
@@ -259,22 +265,27 @@ __global__ void __launch_bounds__(kMoveThreads, 6)
                const uint32_t* __restrict__ new_start, const uint32_t* __restrict__ birth_off,
                const CellPlan* __restrict__ plan, uint32_t* __restrict__ keys_out, uint32_t* __restrict__ ids_out,
                int64_t capacity_out, uint32_t* __restrict__ pool_out, int64_t pool_capacity,
-               PopHeader* __restrict__ head) {
-    if (head->lookback_err) return;
+               PopHeader* __restrict__ head, PopHeader* __restrict__ host, int roles) {
+    const int lookback_err = head->lookback_err;
     const int64_t B = head->totals[1], K = head->totals[2];
     int check = 0;
     if (B > n_pool) check = kPopShortPool;
     else if ((int64_t)head->goal_total > capacity_out) check = kPopListFull;
     else if (n_pool - B + K > pool_capacity) check = kPopPoolFull;
-    if (check) {
-        if (blockIdx.x == 0 && threadIdx.x == 0) head->check = check;
-        return;
+    if (blockIdx.x == 0 && threadIdx.x == 0) {     // for the host (which waits for the kernel)
+        PopHeader h = *head;
+        h.check = check;
+        *host = h;
     }
-    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-    const int64_t t0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (lookback_err || check) return;
+    // roles == 3: the three parts run on blocks of their own (a small list's parts are chains
+    // of a few dependent loads, not work: 4096 individuals 7.9 -> 6.1 us)
+    const int role = roles == 3 ? (int)(blockIdx.x % 3u) : -1;
+    const int64_t stride = (int64_t)(gridDim.x / roles) * blockDim.x;
+    const int64_t t0 = (blockIdx.x / roles) * (int64_t)blockDim.x + threadIdx.x;
     // every individual of a cell whose removals are in its mask (or that loses nobody),
     // kMoveUnroll at a time so that their loads are in flight together
-    int64_t i = t0;
+    int64_t i = role > 0 ? n : t0;
     for (; i + (kMoveUnroll - 1) * stride < n; i += kMoveUnroll * stride) {
         uint32_t c[kMoveUnroll], id[kMoveUnroll];
         CellPlan p[kMoveUnroll];
@@ -298,7 +309,7 @@ __global__ void __launch_bounds__(kMoveThreads, 6)
     }
     // cells that gain, and cells too large for a mask that lose; the counts of
     // kMoveUnroll cells are loaded together
-    for (int64_t c0 = t0; c0 < ncells; c0 += kMoveUnroll * stride) {
+    for (int64_t c0 = role >= 0 && role != 1 ? ncells : t0; c0 < ncells; c0 += kMoveUnroll * stride) {
         uint32_t is[kMoveUnroll], g[kMoveUnroll];
 #pragma unroll
         for (int u = 0; u < kMoveUnroll; ++u) {
@@ -338,7 +349,7 @@ __global__ void __launch_bounds__(kMoveThreads, 6)
     }
     // the unused rest of the old pool, after the removed ids
     const int64_t rest = n_pool - B;
-    int64_t t = t0;
+    int64_t t = role >= 0 && role != 2 ? rest : t0;
     for (; t + (kMoveUnroll - 1) * stride < rest; t += kMoveUnroll * stride) {
         uint32_t v[kMoveUnroll];
 #pragma unroll
@@ -358,7 +369,8 @@ size_t align256(size_t v) { return (v + 255) & ~(size_t)255; }
 
 PopLayout pop_layout(int64_t ncells) {
     PopLayout L;
-    L.tiles = (ncells + kPlanTile - 1) / kPlanTile;
+    const int64_t tile = (int64_t)kPlanThreads * plan_items(ncells);
+    L.tiles = (ncells + tile - 1) / tile;
     size_t o = 0;
     const size_t nc = (size_t)ncells;
     L.head = o; o = align256(o + sizeof(PopHeader));
@@ -371,8 +383,8 @@ PopLayout pop_layout(int64_t ncells) {
 }
 
 // one wave of the move kernel: the blocks that fit on the device at once (looked up
-// once per device), fewer for small work
-unsigned move_grid(int64_t work) {
+// once per device), fewer for small work; *roles: 3 where three times the blocks still fit
+unsigned move_grid(int64_t work, int* roles) {
     static std::atomic<int> resident[64];
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) dev = -1;
@@ -392,7 +404,8 @@ unsigned move_grid(int64_t work) {
     int64_t b = (work + kMoveThreads - 1) / kMoveThreads;
     if (b < 1) b = 1;
     if (b > wave) b = wave;
-    return (unsigned)b;
+    *roles = 3 * b <= wave ? 3 : 1;
+    return (unsigned)(b * *roles);
 }
 
 #define CK(expr)                                                                                           \
@@ -455,27 +468,32 @@ int population_maintain(const uint32_t* keys, const uint32_t* ids, int64_t n_act
     uint32_t* birth_off = (uint32_t*)(base + L.birth_off);
     CellPlan* plan = (CellPlan*)(base + L.plan);
     CK(cudaMemsetAsync(base, 0, L.status + 3 * sizeof(uint64_t) * (size_t)L.tiles, st));
-    k_pop_plan<<<(unsigned)L.tiles, kPlanThreads, 0, st>>>(cell_start, cell_count, goal, ncells, seed, step, new_start,
+    const int items = plan_items(ncells);
+    const auto plan_kernel = items == 1 ? k_pop_plan<1> : items == 2 ? k_pop_plan<2> : k_pop_plan<8>;
+    plan_kernel<<<(unsigned)L.tiles, kPlanThreads, 0, st>>>(cell_start, cell_count, goal, ncells, seed, step, new_start,
                                                             birth_off, plan, head, status, L.tiles);
     CK(cudaGetLastError());
-    int64_t work = n_active > ncells ? n_active : ncells;
-    if (n_pool > work) work = n_pool;
-    k_pop_move<<<move_grid(work), kMoveThreads, 0, st>>>(keys, ids, n_active, cell_count, goal, ncells, pool, n_pool,
-                                                         seed, step, new_start, birth_off, plan, keys_out, ids_out,
-                                                         cap_out, pool_out, cap_pool, head);
-    CK(cudaGetLastError());
-    // the header comes back into this thread's pinned copy (a plain async copy, no
-    // staging through a pageable buffer); a call returns only after its copy landed
+    // the move kernel writes the header to this thread's pinned copy in host memory (a copy
+    // command after it cost as much as the kernel on a small list); without pinned memory, to
+    // its own place in the scratch, which is then copied.  A call returns only after it landed.
     thread_local PinnedHeader t_pinned;
     if (!t_pinned.p && cudaMallocHost((void**)&t_pinned.p, sizeof(PopHeader)) != cudaSuccess) {
         cudaGetLastError();
         t_pinned.p = nullptr;
     }
-    PopHeader h_stack;
-    PopHeader* hp = t_pinned.p ? t_pinned.p : &h_stack;
-    CK(cudaMemcpyAsync(hp, head, sizeof(PopHeader), cudaMemcpyDeviceToHost, st));
+    int64_t work = n_active > ncells ? n_active : ncells;
+    if (n_pool > work) work = n_pool;
+    int roles = 1;
+    const unsigned blocks = move_grid(work, &roles);
+    k_pop_move<<<blocks, kMoveThreads, 0, st>>>(keys, ids, n_active, cell_count, goal, ncells, pool, n_pool,
+                                                         seed, step, new_start, birth_off, plan, keys_out, ids_out,
+                                                         cap_out, pool_out, cap_pool, head,
+                                                         t_pinned.p ? t_pinned.p : head, roles);
+    CK(cudaGetLastError());
+    PopHeader h;
+    if (!t_pinned.p) CK(cudaMemcpyAsync(&h, head, sizeof(PopHeader), cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
-    const PopHeader h = *hp;
+    if (t_pinned.p) std::memcpy(&h, t_pinned.p, sizeof(h));
     if (h.lookback_err) return set_error(GPGMP_ERR_TIMEOUT, "a scan's look-back wait gave up");
     const int64_t n_new = (int64_t)h.goal_total, B = h.totals[1], K = h.totals[2];
     if (h.check == kPopShortPool)

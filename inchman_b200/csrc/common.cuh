@@ -350,6 +350,16 @@ struct BinomialSetup {
         return kind == 2 ? n - k : k;
     }
 };
+// The same for one probability of a whole block, with the first powers in a table.
+struct BinomialTable : BinomialSetup<1> {
+    const float* table;      // (1 - q)^m for m < size, in shared memory
+    int size;
+    __device__ __forceinline__ float power(int m) const { return m < size ? table[m] : pow_int(sq[0], m); }
+    __device__ __forceinline__ int count(uint32_t draw, int n) const {
+        const int k = binomial_count(u01(draw), n, power(n), r);
+        return kind == 2 ? n - k : k;
+    }
+};
 template <int BITS>
 __device__ __forceinline__ int binomial(Stream& st, int n, const BinomialSetup<BITS>& b) {
     if (n <= 0 || b.kind == 0) return 0;

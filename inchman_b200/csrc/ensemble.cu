@@ -16,7 +16,9 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <functional>
 #include <mutex>
+#include <queue>
 #include <vector>
 #include <cuda_runtime.h>
 #include "host_common.h"
@@ -36,9 +38,30 @@ struct Ctrl {
 
 // the reaction structs and their dependency masks, or the packed tables
 constexpr size_t kEnsTables = (sizeof(gpgmp_reaction) + sizeof(uint32_t) * 4) * MAX_REACTIONS;
-static_assert(kEnsTables >= (sizeof(float4) + sizeof(uint4)) * MAX_REACTIONS + sizeof(float) * 1024 &&
-                  kEnsTables % 16 == 0,
-              "the packed tables and one slot per thread");
+static_assert(kEnsTables % 16 == 0, "alignment");
+
+constexpr int kEnsPowers = 512;      // (1 - q)^m of the jump draw, behind the packed tables
+static_assert(kEnsTables >= (sizeof(float4) + sizeof(uint4)) * MAX_REACTIONS + sizeof(float) * kEnsPowers +
+                                sizeof(float) * 1024,
+              "the packed tables, the powers and one slot per thread");
+
+__device__ __forceinline__ unsigned cluster_rank() {
+    unsigned r;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;\n" : "=r"(r));
+    return r;
+}
+__device__ __forceinline__ void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;\n" ::: "memory");
+}
+// *p of the shared memory of CTA `rank` of the cluster
+__device__ __forceinline__ int cluster_read(const int* p, unsigned rank) {
+    int v;
+    asm volatile("{\n .reg .b32 a;\n mapa.shared::cluster.u32 a, %1, %2;\n ld.shared::cluster.s32 %0, [a];\n}\n"
+                 : "=r"(v)
+                 : "r"((uint32_t)__cvta_generic_to_shared(p)), "r"(rank)
+                 : "memory");
+    return v;
+}
 
 struct EnsArgs {
     const gpgmp_instance* inst;
@@ -54,14 +77,19 @@ struct EnsArgs {
     int64_t* snap_time_off;  // per instance: first float of its snapshot times, or -1
     int32_t* status;
     int64_t* steps;
-    int32_t* lost;           // [slot][max_area * 4]
+    int32_t* lost;           // [CTA or cluster][2][max_area * 4]
+    int cluster;             // CTAs per instance
     int64_t lost_stride;
     unsigned int* queue;
     int n_inst;
     int max_species;
 };
 
-template <int NT>
+// CL: the instance's cells are shared by a cluster of CTAs (A.cluster of them); every CTA
+// steps the same clocks.  A thread keeps its cells for the whole run, so only the lost
+// counts of a species cross between threads: one barrier per jump, with the two halves of
+// the lost buffer in turn.
+template <int NT, bool CL>
 __global__ void __launch_bounds__(NT) k_ensemble(EnsArgs A) {
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ gpgmp_instance s_inst;
@@ -73,24 +101,46 @@ __global__ void __launch_bounds__(NT) k_ensemble(EnsArgs A) {
     uint32_t* deps = reinterpret_cast<uint32_t*>(smem + sizeof(gpgmp_reaction) * MAX_REACTIONS);
     float4* ent = reinterpret_cast<float4*>(smem);
     uint4* nets = reinterpret_cast<uint4*>(ent + MAX_REACTIONS);
+    float* powers = reinterpret_cast<float*>(nets + MAX_REACTIONS);
     int* xs = reinterpret_cast<int*>(smem + kEnsTables);
     float* hs = reinterpret_cast<float*>(xs + (size_t)A.max_species * NT);
     // the packed form's slot 0 of every thread lies in the part of the tables that it leaves free
     float* slots = reinterpret_cast<float*>(xs) - NT + threadIdx.x;
-    int32_t* lost = A.lost + (int64_t)blockIdx.x * A.lost_stride;
+    const unsigned csize = CL ? (unsigned)A.cluster : 1u, rank = CL ? cluster_rank() : 0u;
+    const int stride = (int)csize * NT;
+    // consecutive warps of cells on different CTAs
+    const int me = (int)(((threadIdx.x >> 5) * csize + rank) * 32 + (threadIdx.x & 31));
+    const auto sync = [&] {
+        if (CL)
+            cluster_sync();
+        else
+            __syncthreads();
+    };
+    int32_t* lost2 = A.lost + (int64_t)(blockIdx.x / csize) * A.lost_stride;
+    int half = 0;
     for (;;) {
-        if (threadIdx.x == 0) s_item = (int)atomicAdd(A.queue, 1u);
-        __syncthreads();
-        const int item = s_item;
+        if (rank == 0 && threadIdx.x == 0) s_item = (int)atomicAdd(A.queue, 1u);
+        sync();
+        const int item = CL ? cluster_read(&s_item, 0u) : s_item;
+        sync();
         if (item >= A.n_inst) break;
         const int id = A.order[item];
         if (threadIdx.x == 0) s_inst = A.inst[id];
         __syncthreads();
         const int W = s_inst.width, area = W * W, S = s_inst.num_species, R = s_inst.num_reactions;
+        // stay and jump probabilities (as gpgmp_solver_create computes them)
+        const float stay = (float)(1.0 - (double)s_inst.p0);
+        const float pi = (float)((1.0 - (double)stay) / 6.0);
+        BinomialTable jump;
+        jump.init(pi * 4.0f);
+        jump.table = powers;
+        jump.size = 0;
         const gpgmp_reaction* reactions = A.reactions + s_inst.reaction_offset;
         const int nnet = A.nnet[id];
         if (nnet > 0) {
             packed_tables<NT>(A.packed + s_inst.reaction_offset, R, ent, nets);
+            for (int m = threadIdx.x; m < kEnsPowers; m += NT) powers[m] = pow_int(jump.sq[0], m);
+            jump.size = kEnsPowers;
         } else {
             for (int i = threadIdx.x; i < R; i += NT) rt[i] = reactions[i];
             __syncthreads();
@@ -100,6 +150,7 @@ __global__ void __launch_bounds__(NT) k_ensemble(EnsArgs A) {
         const uint32_t key0 = s_inst.seed, key1 = s_inst.realisation;
         const int bm[4] = {s_inst.boundary_mask[0], s_inst.boundary_mask[1], s_inst.boundary_mask[2],
                            s_inst.boundary_mask[3]};
+        const bool stop_on_error = (s_inst.flags & GPGMP_FLAG_STOP_ON_ERROR) != 0;
         if (threadIdx.x == 0) {
             // HomogeneousSolver.cpp:154-166, in float as the host does it
             const float h = s_inst.physical_length / (float)W;
@@ -116,18 +167,17 @@ __global__ void __launch_bounds__(NT) k_ensemble(EnsArgs A) {
             c.nsnap = 0;
         }
         __syncthreads();
-        // stay and jump probabilities (as gpgmp_solver_create computes them)
-        const float stay = (float)(1.0 - (double)s_inst.p0);
-        const float pi = (float)((1.0 - (double)stay) / 6.0);
-        const float pmove = pi * 4.0f;
         int32_t* snaps = s_inst.snapshot_offset >= 0 ? A.snapshots + s_inst.snapshot_offset : nullptr;
         float* stimes = A.snap_time_off[id] >= 0 ? A.snap_times + A.snap_time_off[id] : nullptr;
+        // every thread copies its own cells
         auto snapshot = [&](float t) {
             const int k = c.nsnap;   // read by all threads before thread 0 advances it
             if (snaps && k < s_inst.max_snapshots) {
                 int32_t* dst = snaps + (int64_t)k * S * area;
-                for (int i = threadIdx.x; i < S * area; i += NT) dst[i] = st[i];
-                if (threadIdx.x == 0 && stimes) stimes[k] = t;
+                for (int s = 0; s < S; ++s)
+                    for (int cell = me; cell < area; cell += stride)
+                        dst[(int64_t)s * area + cell] = st[(int64_t)s * area + cell];
+                if (rank == 0 && threadIdx.x == 0 && stimes) stimes[k] = t;
             }
             __syncthreads();
             if (threadIdx.x == 0) c.nsnap = k + 1;
@@ -158,7 +208,7 @@ __global__ void __launch_bounds__(NT) k_ensemble(EnsArgs A) {
             if (R > 0) {
                 int* x = xs + threadIdx.x;
                 int err = 0;
-                for (int cell = threadIdx.x; cell < area; cell += NT) {
+                for (int cell = me; cell < area; cell += stride) {
                     Stream rs;
                     rs.init(key0, key1, sd, (uint32_t)cell, PH_SSA);
                     const auto at = [&](int s) -> int32_t& { return st[(int64_t)s * area + cell]; };
@@ -178,21 +228,22 @@ __global__ void __launch_bounds__(NT) k_ensemble(EnsArgs A) {
                 if (err) atomicOr(&A.status[id], err);
                 sd++;
             }
-            __syncthreads();
             if (c.ev == 0) {
                 for (int i = 0; i < S; ++i) {
                     if (!(i == c.minspec || s_next[i] <= c.mindt)) continue;
                     if (!(s_next[i] > 0)) continue;
                     int32_t* plane = st + (int64_t)i * area;
-                    for (int cell = threadIdx.x; cell < area; cell += NT) {
+                    int32_t* lost = lost2 + (int64_t)half * (A.lost_stride / 2);
+                    half ^= 1;
+                    for (int cell = me; cell < area; cell += stride) {
                         Stream rs;
                         rs.init(key0, key1, sd, (uint32_t)cell, PH_DIFF | ((uint32_t)i << 8));
                         int l[4];
-                        homog_lost(plane[cell], pmove, rs, cell % W, cell / W, W, W, bm, l);
+                        homog_lost(plane[cell], jump, rs, cell % W, cell / W, W, W, bm, l);
                         reinterpret_cast<int4*>(lost)[cell] = make_int4(l[0], l[1], l[2], l[3]);
                     }
-                    __syncthreads();
-                    for (int cell = threadIdx.x; cell < area; cell += NT) {
+                    sync();
+                    for (int cell = me; cell < area; cell += stride) {
                         const int x = cell % W, y = cell / W;
                         const int4 o = reinterpret_cast<const int4*>(lost)[cell];
                         int v = plane[cell] - (o.x + o.y + o.z + o.w);
@@ -202,24 +253,29 @@ __global__ void __launch_bounds__(NT) k_ensemble(EnsArgs A) {
                         if (y < W - 1) v += lost[4 * (cell + W) + 2];
                         plane[cell] = v;
                     }
-                    __syncthreads();
-                    if (threadIdx.x == 0) s_next[i] += s_dt[i];
                 }
             } else if (c.simTime >= c.outputLast + s_inst.output_interval) {
                 snapshot(c.mindt);
                 if (threadIdx.x == 0) c.outputLast += s_inst.output_interval;
             }
+            // the status as every CTA of the cluster sees it: between two barriers
+            if (stop_on_error) sync();
             __syncthreads();
             if (threadIdx.x == 0) {
+                if (c.ev == 0) {
+                    for (int i = 0; i < S; ++i)
+                        if ((i == c.minspec || s_next[i] <= c.mindt) && s_next[i] > 0) s_next[i] += s_dt[i];
+                }
                 c.simTime = c.mindt;
                 c.n += 1;
-                if ((s_inst.flags & GPGMP_FLAG_STOP_ON_ERROR) && *((volatile int32_t*)&A.status[id]) != 0) c.stop = 2;
+                if (stop_on_error && *((volatile int32_t*)&A.status[id]) != 0) c.stop = 2;
             }
+            if (stop_on_error) sync();
             __syncthreads();
             if (c.stop == 2) break;
         }
         snapshot(c.simTime);
-        if (threadIdx.x == 0) A.steps[id] = c.n;
+        if (rank == 0 && threadIdx.x == 0) A.steps[id] = c.n;
         __syncthreads();
     }
 }
@@ -242,6 +298,12 @@ __global__ void k_ensemble_init(const gpgmp_instance* inst, int n_inst, const fl
 
 }  // namespace
 
+namespace {
+struct EnsCost {
+    double work, steps;
+};
+}  // namespace
+
 struct gpgmp_ensemble {
     int n = 0;
     int max_species = 0, max_area = 0, max_reactions = 0;
@@ -261,6 +323,8 @@ struct gpgmp_ensemble {
     int32_t* d_lost = nullptr;
     unsigned int* d_queue = nullptr;
     int threads = 256, ctas_per_sm = 4, num_sms = 148, grid = 0;
+    int cluster = 1;                 // CTAs per instance
+    std::vector<EnsCost> cost;       // of the instances in decreasing order (d_order's)
     size_t smem = 0;
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
@@ -287,22 +351,62 @@ void ens_free(gpgmp_ensemble* h) {
 }
 
 // longest-processing-time order: cells x species x steps x (1 + reactions / 4)
-double est_cost(const gpgmp_instance& I, const float* diffusion) {
+EnsCost est_cost(const gpgmp_instance& I, const float* diffusion) {
     float dmax = 0.f;
     for (int s = 0; s < I.num_species; ++s) dmax = std::max(dmax, diffusion[I.species_offset + s]);
     const double h = (double)I.physical_length / I.width;
     const double dtmin = dmax > 0 ? I.p0 / 6.0 * h * h / dmax : I.max_time;
     const double steps = I.max_time / std::max(dtmin, 1e-9) + 1.0;
-    return (double)I.width * I.width * I.num_species * steps * (1.0 + I.num_reactions / 4.0);
+    return {(double)I.width * I.width * I.num_species * steps * (1.0 + I.num_reactions / 4.0), steps};
 }
 
-const void* ens_kernel(int threads) {
+const void* ens_kernel(int threads, bool cluster) {
+#define GPGMP_ENS(N) \
+    case N: return cluster ? (const void*)k_ensemble<N, true> : (const void*)k_ensemble<N, false>;
     switch (threads) {
-        case 128: return (const void*)k_ensemble<128>;
-        case 256: return (const void*)k_ensemble<256>;
-        case 512: return (const void*)k_ensemble<512>;
-        default: return (const void*)k_ensemble<1024>;
+        GPGMP_ENS(128)
+        GPGMP_ENS(256)
+        GPGMP_ENS(512)
+        default: return cluster ? (const void*)k_ensemble<1024, true> : (const void*)k_ensemble<1024, false>;
     }
+#undef GPGMP_ENS
+}
+
+void ens_launch_config(const gpgmp_ensemble* h, int cluster, int grid, cudaLaunchConfig_t* cfg,
+                       cudaLaunchAttribute* attr, cudaStream_t st) {
+    *cfg = {};
+    cfg->gridDim = dim3(grid, 1, 1);
+    cfg->blockDim = dim3(h->threads, 1, 1);
+    cfg->dynamicSmemBytes = h->smem;
+    cfg->stream = st;
+    if (cluster > 1) {
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = cluster;
+        attr[0].val.clusterDim.y = 1;
+        attr[0].val.clusterDim.z = 1;
+        cfg->attrs = attr;
+        cfg->numAttrs = 1;
+    }
+}
+
+// the estimated time of all instances on `groups` of `cluster` CTAs, each instance (in
+// decreasing cost) to the group that is free first.  What a cluster does not share out is
+// the latency of a step (one window's chain of events, a jump's draw, the barriers): a step
+// of A + B <-> C on 32 x 32 cells takes 11.6 us + 4.2 us / CTAs, as long as the cells' work
+// of 12,700 of est_cost's units; a cluster's barriers add about 1,000.
+double ens_makespan(const std::vector<EnsCost>& cost, int cluster, int groups) {
+    const double kStep = cluster > 1 ? 13700.0 : 12700.0;
+    std::priority_queue<double, std::vector<double>, std::greater<double>> free;
+    double end = 0;
+    const size_t n = std::min(cost.size(), (size_t)groups);
+    for (size_t i = 0; i < n; ++i) free.push(0.0);
+    for (const EnsCost& c : cost) {
+        const double t = free.top() + c.work / cluster + c.steps * kStep;
+        free.pop();
+        free.push(t);
+        end = std::max(end, t);
+    }
+    return end;
 }
 
 int configure(gpgmp_ensemble* h, int threads, int ctas_per_sm) {
@@ -311,20 +415,45 @@ int configure(gpgmp_ensemble* h, int threads, int ctas_per_sm) {
     h->threads = threads;
     h->smem = kEnsTables + sizeof(int) * (size_t)h->max_species * threads +
               sizeof(float) * (size_t)h->max_reactions * threads;
-    CK(cudaFuncSetAttribute(ens_kernel(threads), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)h->smem));
+    CK(cudaFuncSetAttribute(ens_kernel(threads, false), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)h->smem));
     int dev = 0, sms = 0;
     CK(cudaGetDevice(&dev));
     CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     int occ = 0;
-    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, ens_kernel(threads), threads, h->smem));
+    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, ens_kernel(threads, false), threads, h->smem));
     if (occ < 1) return set_error(GPGMP_ERR_UNSUPPORTED, "ensemble kernel does not fit an SM");
     h->num_sms = sms;
     h->ctas_per_sm = std::max(1, std::min(ctas_per_sm, occ));
     h->grid = sms * h->ctas_per_sm;
-    // lost-count scratch: one slot per CTA
+    // CTAs per instance: where that shortens the estimated run by a twentieth or more (few
+    // instances, or one that outlasts the rest: 592 random instances 74 -> 58 ms with two, 60
+    // of them 33 -> 13 ms with eight, 16 of A + B <-> C on 32 x 32 cells 1.90 -> 1.52 with four)
+    h->cluster = 1;
+    double best = ens_makespan(h->cost, 1, h->grid);
+    const void* ck = ens_kernel(threads, true);
+    CK(cudaFuncSetAttribute(ck, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)h->smem));
+    for (int cl : {2, 4, 8}) {
+        cudaLaunchConfig_t cfg;
+        cudaLaunchAttribute attr[1];
+        ens_launch_config(h, cl, cl, &cfg, attr, nullptr);
+        int most = 0;
+        if (cudaOccupancyMaxActiveClusters(&most, ck, &cfg) != cudaSuccess) {
+            cudaGetLastError();
+            break;
+        }
+        const int groups = std::min(most, sms * h->ctas_per_sm / cl);
+        if (groups < 1) break;
+        const double t = ens_makespan(h->cost, cl, groups);
+        if (t < 0.95 * best) {
+            best = t;
+            h->cluster = cl;
+            h->grid = std::min(groups, h->n) * cl;
+        }
+    }
+    // lost-count scratch: two buffers per CTA or cluster
     if (h->d_lost) cudaFree(h->d_lost);
     h->d_lost = nullptr;
-    CK(cudaMalloc(&h->d_lost, sizeof(int32_t) * 4 * (size_t)h->max_area * h->grid));
+    CK(cudaMalloc(&h->d_lost, sizeof(int32_t) * 2 * 4 * (size_t)h->max_area * (h->grid / h->cluster)));
     if (h->exec) { cudaGraphExecDestroy(h->exec); h->exec = nullptr; }
     if (h->graph) { cudaGraphDestroy(h->graph); h->graph = nullptr; }
     return GPGMP_OK;
@@ -385,9 +514,10 @@ int gpgmp_ensemble_create(const gpgmp_instance* instances, int32_t n, const floa
     }
     std::vector<int32_t> order(n);
     for (int i = 0; i < n; ++i) order[i] = i;
-    std::vector<double> cost(n);
+    std::vector<EnsCost> cost(n);
     for (int i = 0; i < n; ++i) cost[i] = est_cost(instances[i], diffusion);
-    std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return cost[a] > cost[b]; });
+    std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return cost[a].work > cost[b].work; });
+    for (int i : order) h->cost.push_back(cost[i]);
     cudaError_t e = cudaSuccess;
     auto A = [&](void** p, size_t b) { if (e == cudaSuccess) e = cudaMalloc(p, b > 0 ? b : 1); };
     A((void**)&h->d_inst, sizeof(gpgmp_instance) * n);
@@ -467,7 +597,7 @@ int gpgmp_ensemble_run(gpgmp_ensemble* h, int32_t* state, int32_t* snapshots, vo
         a.packed = h->d_packed; a.nnet = h->d_nnet;
         a.state = state; a.snapshots = snapshots; a.snap_times = h->d_snap_times;
         a.snap_time_off = h->d_snap_time_off; a.status = h->d_status; a.steps = h->d_steps;
-        a.lost = h->d_lost; a.lost_stride = 4 * (int64_t)h->max_area; a.queue = h->d_queue; a.n_inst = h->n;
+        a.lost = h->d_lost; a.lost_stride = 2 * 4 * (int64_t)h->max_area; a.cluster = h->cluster; a.queue = h->d_queue; a.n_inst = h->n;
         a.max_species = h->max_species;
         a.max_reactions = h->max_reactions;
         cudaError_t e = cudaStreamBeginCapture(cap, cudaStreamCaptureModeThreadLocal);
@@ -475,8 +605,12 @@ int gpgmp_ensemble_run(gpgmp_ensemble* h, int32_t* state, int32_t* snapshots, vo
             cudaMemsetAsync(h->d_queue, 0, sizeof(unsigned int), cap);
             cudaMemsetAsync(h->d_status, 0, sizeof(int32_t) * h->n, cap);
             void* args[] = {&a};
-            cudaLaunchKernel(ens_kernel(h->threads), dim3(h->grid), dim3(h->threads), args, h->smem, cap);
+            cudaLaunchConfig_t cfg;
+            cudaLaunchAttribute attr[1];
+            ens_launch_config(h, h->cluster, h->grid, &cfg, attr, cap);
+            const cudaError_t launched = cudaLaunchKernelExC(&cfg, ens_kernel(h->threads, h->cluster > 1), args);
             e = cudaStreamEndCapture(cap, &h->graph);
+            if (e == cudaSuccess) e = launched;
         }
         cudaStreamDestroy(cap);
         if (e != cudaSuccess) return set_error(GPGMP_ERR_CUDA, "graph capture: %s", cudaGetErrorString(e));

@@ -365,11 +365,21 @@ __device__ __forceinline__ int packed_window(const gpgmp_reaction* rt, int R, co
     return e;
 }
 
-// Four lost counts (-x, +x, -y, +y) of one cell of n particles.
-__device__ __forceinline__ void homog_lost(int n, float pmove, Stream& st, int x, int y, int W, int H,
+// Four lost counts (-x, +x, -y, +y) of one cell of n particles; jump: the draw of the moved
+// ones (BinomialSetup or BinomialTable).
+template <class JUMP>
+__device__ __forceinline__ void homog_lost(int n, const JUMP& jump, Stream& st, int x, int y, int W, int H,
                                            const int* bmask, int l[4]) {
     l[0] = l[1] = l[2] = l[3] = 0;
-    const int moved = binomial(st, n, pmove);
+    if (n <= 0 || jump.kind == 0) return;
+    int moved;
+    if (jump.single(n)) {          // one draw, the first of the block whose others serve the directions
+        st.block(st.buf);
+        st.idx = 1;
+        moved = jump.count(st.buf[0], n);
+    } else {
+        moved = binomial(st, n, jump);
+    }
     if (moved <= 64) {
         // sixteen 2-bit directions per draw, counted by their bits
         int c1 = 0, c2 = 0, c3 = 0;

@@ -177,6 +177,8 @@ __global__ void __launch_bounds__(NT) k_diffuse_tile(const int* __restrict__ in,
     const int64_t plane = ((int64_t)r * S + species) * area;
     const int bm[4] = {bm4.x, bm4.y, bm4.z, bm4.w};
     const uint32_t phase = PH_DIFF | ((uint32_t)species << 8);
+    BinomialSetup<7> jump;
+    jump.init(pmove);
     for (int i = threadIdx.x; i < RW * RH; i += NT) {
         const int lx = i % RW, ly = i / RW;
         const int gx = x0 + lx - 1, gy = y0 + ly - 1;
@@ -186,7 +188,7 @@ __global__ void __launch_bounds__(NT) k_diffuse_tile(const int* __restrict__ in,
             const int n = in[plane + c];
             Stream st;
             st.init(seed, (uint32_t)r, step_seed, (uint32_t)c, phase);
-            homog_lost(n, pmove, st, gx, gy, W, H, bm, l);
+            homog_lost(n, jump, st, gx, gy, W, H, bm, l);
             if (lx >= 1 && lx < 1 + TW && ly >= 1 && ly < 1 + TH) s_n[(ly - 1) * TW + (lx - 1)] = n;
         }
 #pragma unroll

@@ -379,16 +379,15 @@ __device__ __forceinline__ int binomial(Stream& st, int n, float p) {
     return binomial(st, n, b);
 }
 
-// Unit-rate arrivals before lam: the logarithms of a block's four draws are independent,
-// only the sums are a chain (lam = 100 for two species on 1M cells: 654 us, now 400).
-__device__ __forceinline__ int poisson(Stream& st, float lam) {
-    if (!(lam > 0.0f)) return 0;
+// Unit-rate arrivals before lam: the times are the running sums of -log_draw, each rounded,
+// and the count is how many of them stay at or below lam.
+__device__ __forceinline__ int poisson_exact(Stream& st, float lam) {
     int k = 0;
     float t = 0.0f;
     for (;;) {
         uint32_t w[4];
         st.block(w);
-        float a[4];
+        float a[4];      // the logarithms are independent, only the sums are a chain
 #pragma unroll
         for (int i = 0; i < 4; ++i) a[i] = log_draw(w[i]);
 #pragma unroll
@@ -399,6 +398,63 @@ __device__ __forceinline__ int poisson(Stream& st, float lam) {
             if (k == INT_MAX) return k;
         }
     }
+}
+
+__device__ __forceinline__ float log2_approx(float x) {
+    float r;
+    asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+
+// The same count with a bound instead of the sums: most blocks lie well below lam, and for
+// them one approximate logarithm of the four draws' product tells that all four arrivals
+// count.  `off` bounds how far the approximate time can be from the rounded running sum, in
+// 2^-24: each running sum is rounded by at most its own size (4 a block, at most the block's
+// last) and so is the approximate one (5 sum), log_draw and lg2.approx are off by at most 8
+// and 4 of the time, and a block's product and an argument near 1 add 6; all of it doubled.
+// An arrival within that of lam (one cell in a thousand at lam = 100) sends the cell to
+// poisson_exact, and from lam = 256 on, where it would be one in a hundred, all cells.  Two
+// species at lam = 100 on 1M cells: 400 us, now 257; at lam = 50 on 8.4M cells 1.68 ms, now
+// 0.96.
+__device__ __forceinline__ int poisson(Stream& st, float lam) {
+    if (!(lam > 0.0f)) return 0;
+    const Stream from = st;
+    if (lam < 256.0f) {
+        constexpr float kLn2 = 0.6931471806f, kScale = 5.9604644775390625e-08f;      // 2^-24
+        float t = 0.0f, sum = 0.0f, blocks = 0.0f;
+        int k = 0;
+        for (;;) {
+            uint32_t w[4];
+            st.block(w);
+            float v[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) v[i] = (float)((w[i] >> 8) + 1u);
+            const float p = ((v[0] * v[1]) * (v[2] * v[3])) * 1.262177448353619e-29f;      // 2^-96
+            const float t4 = fmaf(-kLn2, log2_approx(p), t);
+            sum += t4;
+            blocks += 1.0f;
+            const float off = 2.0f * kScale * fmaf(5.0f, sum, fmaf(12.0f, t4, fmaf(6.0f, blocks, 16.0f)));
+            if (t4 + off <= lam) {
+                t = t4;
+                k += 4;
+                continue;
+            }
+            bool sure = true;
+            int more = -1;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                t = fmaf(-kLn2, log2_approx(v[i] * kScale), t);
+                if (more < 0) {
+                    sure = sure && fabsf(t - lam) > off;
+                    if (t > lam) more = i;
+                }
+            }
+            if (sure && more >= 0) return k + more;
+            break;
+        }
+    }
+    st = from;
+    return poisson_exact(st, lam);
 }
 
 __device__ __forceinline__ void normal2(Stream& st, float* z0, float* z1) {

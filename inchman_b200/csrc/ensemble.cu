@@ -287,7 +287,7 @@ __global__ void k_ensemble_init(const gpgmp_instance* inst, int n_inst, const fl
     if (id >= n_inst) return;
     const gpgmp_instance I = inst[id];
     const int area = I.width * I.width;
-    for (int cell = threadIdx.x; cell < area; cell += blockDim.x) {
+    for (int cell = blockIdx.y * blockDim.x + threadIdx.x; cell < area; cell += gridDim.y * blockDim.x) {
         for (int s = 0; s < I.num_species; ++s) {
             Stream st;
             st.init(I.seed, I.realisation, 0u, (uint32_t)cell, PH_INIT | ((uint32_t)s << 8));
@@ -577,7 +577,10 @@ int gpgmp_ensemble_configure(gpgmp_ensemble* h, int32_t threads_per_cta, int32_t
 
 int gpgmp_ensemble_init_poisson(gpgmp_ensemble* h, int32_t* state, void* stream) {
     if (!h || !state) return set_error(GPGMP_ERR_INVALID, "bad argument");
-    k_ensemble_init<<<h->n, 256, 0, (cudaStream_t)stream>>>(h->d_inst, h->n, h->d_lambda, state);
+    // blocks for the largest instance's cells each (one block per instance left 16 instances on
+    // 16 SMs: 72 us instead of 27)
+    const unsigned per = (unsigned)std::min((h->max_area + 127) / 128, 128);
+    k_ensemble_init<<<dim3(h->n, per), 128, 0, (cudaStream_t)stream>>>(h->d_inst, h->n, h->d_lambda, state);
     CK(cudaGetLastError());
     return GPGMP_OK;
 }

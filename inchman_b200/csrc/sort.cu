@@ -21,6 +21,7 @@
 //    left/right indices follow from them.
 // Every look-back spin has an iteration limit; exceeding it sets the error word
 // (GPGMP_ERR_TIMEOUT for the caller) and the kernel continues without waiting.
+#include <type_traits>
 #include <algorithm>
 #include <cstdint>
 #include <mutex>
@@ -320,89 +321,163 @@ __global__ void __launch_bounds__(kStreamThreads, 1) k_scan_stream(const uint32_
 }
 
 // ---- radix sort ------------------------------------------------------------------
-// A tile is kThreads threads x kSortItems keys.  8-bit passes run 256-thread tiles, four
-// CTAs per SM (one CTA's barriers overlap the others' work); 10-bit passes 512-thread
-// tiles, two per SM (with 256 threads each would own four digits and spill registers).
-constexpr int kSortItems = 15;
+// A tile is kThreads threads x kItems keys, kItems as many as the registers hold: 16.8M pairs
+// of 32 bits took 446 us with tiles of 15 keys per thread, 440 with 18 (6 four-CTA shapes of
+// 256 to 384 threads: 445 to 490).
 template <int RB>
 struct SortShape {
-    static constexpr int kThreads = RB == 8 ? 256 : 512;
-    static constexpr int kMinBlocks = RB == 8 ? 4 : 2;
-    static constexpr int kTile = kThreads * kSortItems;   // 3840 / 7680 keys
+    static constexpr int kThreads = 512;
+    static constexpr int kMinBlocks = 2;
+    static constexpr int kItems = RB == 8 ? 18 : 15;
+    static constexpr int kTile = kThreads * kItems;
     static constexpr int kWarps = kThreads / 32;
     // keys and values of a tile in sorted order (dynamic shared memory: 30 / 60 KB)
     static constexpr int kStagingBytes = 2 * kTile * (int)sizeof(uint32_t);
-    static_assert(kThreads >= 256 && kThreads % 32 == 0, "a thread per digit (8-bit digits)");
+    static_assert(kTile < 65536, "positions in a tile fit 16 bits");
 };
-// 8-bit passes copy the values asynchronously into the values' staging area while the
-// tile ranks and stage them in two steps (through registers); 10-bit passes read them at
-// the staging step, which measured faster for them than the extra barrier of the
-// two-step form.
-template <int RB>
-constexpr bool kValuePrefetch = RB == 8;
 constexpr uint32_t kFlagA = 1u << 30, kFlagP = 2u << 30, kValMask = (1u << 30) - 1;
+constexpr int kMatchItems = 3;   // items of a lane ranked together
 constexpr int kLookWindow = 4;   // predecessor tiles read per look-back step
 constexpr int kHistWords = 3 * 1024;   // digit counts of every pass: 4 x 256 or up to 3 x 1024
 
-// Digits of RB bits: DIG values, owned kDPT at a time by the first kDigitThreads threads
-// in the digit phases (8 bits: all 256 threads, one each; 10 bits: all 512, two each).
+// Digits of RB bits: DIG values, owned two at a time by the first kDigitThreads threads in
+// the digit phases (two 16-bit counts are one word of shared memory, two look-back words
+// one 8-byte access).
 template <int RB>
 struct Radix {
     static constexpr int DIG = 1 << RB;
     static constexpr uint32_t MASK = (uint32_t)DIG - 1u;
-    static constexpr int kDigitThreads = DIG < SortShape<RB>::kThreads ? DIG : SortShape<RB>::kThreads;
-    static constexpr int kDPT = DIG / kDigitThreads;
+    static constexpr int kDigitThreads = DIG / 2;
     static constexpr int kDigitWarps = kDigitThreads / 32;
+    static_assert(kDigitThreads <= SortShape<RB>::kThreads, "a thread per two digits");
 };
 
-// One pass over the keys counts every digit position: hist[pass][DIG].  A few CTAs
-// per SM each count a long stretch of keys into shared memory (16-byte loads, two in
-// flight per thread), then add their counts to the global histogram once: with one
-// CTA per few thousand keys, the global atomics of the flush (passes x DIG per CTA)
-// cost more than the counting.
-constexpr int kHistThreads = 512;
+// One pass over the keys counts every digit position: hist[pass][DIG].  A CTA per SM
+// counts into shared memory, where every lane has counters of its own (a word of lane l in
+// bank l), so that neither equal digits nor digits of one bank make a warp's additions wait
+// for one another: with counters shared by the lanes an addition took 3.5 cycles of the
+// shared-memory pipe on random keys and 32 on equal ones.  10-bit digits have two counters
+// to a word (three passes of words of their own are 384 KB), which go to the global
+// histogram before one of 16 bits can overflow: after kHistFlush rounds of 512 keys per
+// lane.  The passes are a constant because the instructions bound this kernel next: a shift,
+// a mask and an addition per digit.
+// 16.8M keys, four digits: 33 us with shared counters, 17.6 now.
+constexpr int kHistThreads = 1024, kHistFlush = 96;
 template <int RB>
-__global__ void __launch_bounds__(kHistThreads) k_radix_histogram(const uint32_t* __restrict__ keys, int64_t n,
-                                                                  int passes, uint32_t* __restrict__ hist) {
+constexpr int kHistPair = RB == 8 ? 1 : 2;   // counters per word
+template <int RB, int PASSES>
+constexpr int kHistSmem = PASSES * Radix<RB>::DIG / kHistPair<RB> * 32 * (int)sizeof(uint32_t);
+template <int RB, int PASSES>
+__global__ void __launch_bounds__(kHistThreads, 1) k_radix_histogram(const uint32_t* __restrict__ keys, int64_t n,
+                                                                     uint32_t* __restrict__ hist) {
     using R = Radix<RB>;
-    __shared__ uint32_t s_h[kHistWords];
-    for (int i = threadIdx.x; i < passes * R::DIG; i += blockDim.x) s_h[i] = 0;
-    __syncthreads();
-    auto count = [&](uint32_t k) {
-        for (int p = 0; p < passes; ++p) atomicAdd(&s_h[p * R::DIG + ((k >> (RB * p)) & R::MASK)], 1u);
+    constexpr int PAIR = kHistPair<RB>, ROWS = R::DIG / PAIR, words = PASSES * ROWS;
+    extern __shared__ __align__(16) uint32_t s_h[];
+    const int lane = threadIdx.x & 31;
+    const auto clear = [&] {
+        for (int i = threadIdx.x; i < words * 8; i += kHistThreads)
+            reinterpret_cast<uint4*>(s_h)[i] = make_uint4(0, 0, 0, 0);
+        __syncthreads();
     };
-    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-    const int64_t t0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    const auto count = [&](uint32_t k) {
+#pragma unroll
+        for (int p = 0; p < PASSES; ++p) {
+            // byte offset: 128 * (row of the digit) + 4 * lane
+            constexpr int down = PAIR - 1 - 7;
+            const int s = RB * p + down;
+            const uint32_t row = (s >= 0 ? k >> (s & 31) : k << (-s & 31)) & (uint32_t)((ROWS - 1) << 7);
+            uint32_t* w = reinterpret_cast<uint32_t*>(reinterpret_cast<char*>(s_h) + p * ROWS * 128 + (row | lane << 2));
+            atomicAdd(w, PAIR == 2 && (k >> (RB * p) & 1u) ? 0x10000u : 1u);
+        }
+    };
+    const auto flush = [&] {
+        __syncthreads();
+        for (int w = threadIdx.x; w < words; w += kHistThreads) {
+            uint32_t lo = 0, hi = 0;
+#pragma unroll 8
+            for (int l = 0; l < 32; ++l) {
+                const uint32_t c = s_h[w * 32 + ((w + l) & 31)];
+                lo += PAIR == 2 ? c & 0xffffu : c;
+                if (PAIR == 2) hi += c >> 16;
+            }
+            if (lo) atomicAdd(&hist[PAIR * w], lo);
+            if (hi) atomicAdd(&hist[PAIR * w + 1], hi);
+        }
+        __syncthreads();
+    };
+    clear();
+    const int64_t stride = (int64_t)gridDim.x * kHistThreads;
+    const int64_t t0 = blockIdx.x * (int64_t)kHistThreads + threadIdx.x;
     // 16-byte loads where the pointer allows them; the head before the first 16-byte
     // boundary and the tail after the last whole quad take single loads
     const int head = (int)((16 - ((uintptr_t)keys & 15)) & 15) / 4;
     const int64_t h = head < n ? head : n;
     const uint4* q = reinterpret_cast<const uint4*>(keys + h);
     const int64_t nq = ((uintptr_t)keys & 3) ? 0 : (n - h) / 4;
-    int64_t i = t0;
-    for (; i + stride < nq; i += 2 * stride) {
-        const uint4 a = __ldg(q + i), b = __ldg(q + i + stride);
-        count(a.x); count(a.y); count(a.z); count(a.w);
-        count(b.x); count(b.y); count(b.z); count(b.w);
+    int since = 0;   // rounds since the last flush (the same in every thread)
+    for (int64_t base = 0; base < nq; base += 4 * stride) {
+        if (PAIR == 2 && since++ == kHistFlush) {
+            flush();
+            clear();
+            since = 1;
+        }
+        uint4 a[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+            if (base + u * stride + t0 < nq) a[u] = __ldg(q + base + u * stride + t0);
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+            if (base + u * stride + t0 < nq) {
+                count(a[u].x); count(a[u].y); count(a[u].z); count(a[u].w);
+            }
     }
-    for (; i < nq; i += stride) {
-        const uint4 a = __ldg(q + i);
-        count(a.x); count(a.y); count(a.z); count(a.w);
-    }
+    // at most 3 + 3 keys, or the whole of a list whose pointer is not a multiple of 4
     const int64_t done = nq > 0 ? h + 4 * nq : 0;
-    if (nq > 0)
-        for (int64_t j = t0; j < h; j += stride) count(keys[j]);
-    for (int64_t j = done + t0; j < n; j += stride) count(keys[j]);
-    __syncthreads();
-    for (int i2 = threadIdx.x; i2 < passes * R::DIG; i2 += blockDim.x) {
-        const uint32_t c = s_h[i2];
-        if (c) atomicAdd(&hist[i2], c);
+    if (nq > 0 && t0 < h) count(keys[t0]);
+    for (int64_t base = done; base < n; base += stride) {
+        if (PAIR == 2 && since++ == kHistFlush) {
+            flush();
+            clear();
+            since = 1;
+        }
+        if (base + t0 < n) count(keys[base + t0]);
     }
+    flush();
 }
+
+// the lanes of `mask` whose digit agrees with d in bits LO..HI-1, by a ballot per bit
+template <int LO, int HI>
+__device__ __forceinline__ unsigned match_bits(uint32_t d, unsigned mask) {
+#pragma unroll
+    for (int b = LO; b < HI; ++b) {
+        const bool bit = (d >> b) & 1u;
+        const unsigned bal = __ballot_sync(0xffffffffu, bit);
+        mask &= bit ? bal : ~bal;
+    }
+    return mask;
+}
+// N positions in a tile, two to a register (indexes are constants after unrolling)
+template <int N>
+struct Positions {
+    uint32_t p[(N + 1) / 2];
+    __device__ __forceinline__ void set(int i, uint32_t v) {
+        p[i / 2] = __byte_perm(p[i / 2], v, i & 1 ? 0x5410 : 0x3254);
+    }
+    __device__ __forceinline__ uint32_t get(int i) const { return i & 1 ? p[i / 2] >> 16 : p[i / 2] & 0xffffu; }
+};
 
 // One onesweep pass.  Warp w of a tile owns keys [w*32*IT, (w+1)*32*IT) of the tile
 // in a warp-striped layout (item j of lane l is key j*32 + l), so processing items in
 // order and lanes in order is index order: the ranks are stable.
+// Bound by shared-memory accesses (63-70 % of their pipe; the arithmetic at 26 %): each
+// scattered one costs 3.3 wavefronts per warp (32 random digits on 32 banks).  So the
+// tile's digit counts come out of the ranking instead of a pass of atomics of their own,
+// one atomic of a group's leader reads and advances the warp's count, and the values
+// travel through registers, loaded before the look-back and staged after it.  Equal digits
+// are found by words of lane bits; ballots take 10 wavefronts fewer and 50 instructions
+// more per 32 keys: 548 us for 16.8M pairs of 32 bits against 460.  Three items are ranked
+// together, so that the chain of an item (bits, read, count, shuffle) has company.
+// A pass over 16.8M pairs: 116 us before, 95 now.
 template <int RB>
 __global__ void __launch_bounds__(SortShape<RB>::kThreads, SortShape<RB>::kMinBlocks) k_onesweep(const uint32_t* __restrict__ kin,
                                                            const uint32_t* __restrict__ vin,
@@ -412,297 +487,224 @@ __global__ void __launch_bounds__(SortShape<RB>::kThreads, SortShape<RB>::kMinBl
                                                            int* err, uint32_t* __restrict__ cell_count,
                                                            uint32_t ncells) {
     using R = Radix<RB>;
-    constexpr int kSortThreads = SortShape<RB>::kThreads;
-    constexpr int kSortTile = SortShape<RB>::kTile;
+    constexpr int kThreads = SortShape<RB>::kThreads, kItems = SortShape<RB>::kItems;
+    constexpr int kTile = SortShape<RB>::kTile;
     constexpr int kWarps = SortShape<RB>::kWarps;
     constexpr int DIG = R::DIG;
-    constexpr int DPT = R::kDPT;
-    // per warp and digit: the warp's count, then the tile-local position of the warp's
-    // first key of that digit (at most 7680, so 16 bits)
-    __shared__ uint16_t s_warp_hist[kWarps][DIG];
-    __shared__ uint32_t s_count[DIG];        // the tile's count of each digit
+    // per warp and digit, two digits to a word: the warp's count, then the tile-local
+    // position of the warp's first key of that digit
+    __shared__ uint32_t s_warp_hist[kWarps][DIG / 2];
     __shared__ uint32_t s_delta[DIG];        // global start minus tile-local start of each digit
     __shared__ uint32_t s_w[R::kDigitWarps];
     __shared__ uint32_t s_hw[R::kDigitWarps];
-    extern __shared__ uint32_t s_staging[];  // keys, values in tile-sorted order [, values as loaded]
+    extern __shared__ uint32_t s_staging[];  // keys, values in tile-sorted order
     uint32_t* s_keys = s_staging;
-    uint32_t* s_vals = s_staging + kSortTile;
-    uint32_t* s_vraw = s_vals;   // values as loaded, until the staging step
+    uint32_t* s_vals = s_staging + kTile;
     __shared__ uint32_t s_tile;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     if (threadIdx.x == 0) s_tile = atomicAdd(tile_counter, 1u);
-    for (int i = threadIdx.x; i < kWarps * DIG / 2; i += kSortThreads)
-        reinterpret_cast<uint32_t*>(&s_warp_hist[0][0])[i] = 0;
-    for (int i = threadIdx.x; i < DIG; i += kSortThreads) s_count[i] = 0;
+    for (int i = threadIdx.x; i < kWarps * DIG / 2; i += kThreads) (&s_warp_hist[0][0])[i] = 0;
     // ranking: per warp and value of a digit's low 8 bits, the lanes holding it (in the
     // keys' staging area, which is free until the staging step)
-    static_assert(kWarps * 256 <= kSortTile, "match words fit in the keys' staging area");
-    uint32_t* s_match = s_staging;
-    for (int i = threadIdx.x; i < kWarps * 256; i += kSortThreads) s_match[i] = 0;
+    static_assert(kItems % kMatchItems == 0 && kMatchItems * kWarps * 256 <= 2 * kTile, "match words fit in the staging area");
+    uint32_t* s_match = s_staging + warp * kMatchItems * 256;
+    for (int i = threadIdx.x; i < kMatchItems * kWarps * 256; i += kThreads) s_staging[i] = 0;
     __syncthreads();
     const uint32_t tile = s_tile;
-    const int64_t tbase = (int64_t)tile * kSortTile;
-    const int64_t wbase = tbase + (int64_t)warp * 32 * kSortItems;
-    // item j of this lane is in range iff j * 32 < rem
-    const int64_t rem64 = n - (wbase + lane);
-    const int rem = rem64 < kSortTile ? (int)rem64 : kSortTile;
-    // values are not held in registers (fewer registers, more warps per SM): 8-bit passes
-    // copy them into the values' area with cp.async while the tile ranks, 10-bit passes
-    // read them at the staging step
-    uint32_t key[kSortItems], rank[kSortItems];
+    const int64_t tbase = (int64_t)tile * kTile;
+    const int64_t wbase = tbase + (int64_t)warp * 32 * kItems;
+    // a tile with every key in range needs no tests of the items
+    const auto run = [&](auto all) {
+        constexpr bool FULL = decltype(all)::value;
+        // item j of this lane is in range iff j * 32 < rem
+        const int64_t rem64 = n - (wbase + lane);
+        const int rem = FULL ? kTile : rem64 < kTile ? (int)rem64 : kTile;
+        uint32_t key[kItems];
+        Positions<kItems> pos;
 #pragma unroll
-    for (int j = 0; j < kSortItems; ++j) {
-        const int64_t idx = wbase + j * 32 + lane;
-        const bool ok = j * 32 < rem;
-        key[j] = ok ? kin[idx] : 0xffffffffu;
-        if constexpr (kValuePrefetch<RB>) {
-            if (ok) {
-                const uint32_t dst =
-                    (uint32_t)__cvta_generic_to_shared(s_vraw + warp * 32 * kSortItems + j * 32 + lane);
-                asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(dst), "l"(vin + idx) : "memory");
+        for (int j = 0; j < kItems; ++j) key[j] = j * 32 < rem ? kin[wbase + j * 32 + lane] : 0xffffffffu;
+        // warp-level ranking (stable): the lowest lane of each group of equal digits adds the
+        // group to the warp's count of the digit, and the count before it comes back to the
+        // whole group by one shuffle
+        const unsigned lt = (1u << lane) - 1u;
+        uint32_t* hist = s_warp_hist[warp];
+#pragma unroll
+        for (int j0 = 0; j0 < kItems; j0 += kMatchItems) {
+            uint32_t d[kMatchItems], prior[kMatchItems];
+            unsigned peers[kMatchItems];
+            bool ok[kMatchItems];
+#pragma unroll
+            for (int u = 0; u < kMatchItems; ++u) {
+                ok[u] = (j0 + u) * 32 < rem;
+                d[u] = (key[j0 + u] >> shift) & R::MASK;
+                if (ok[u]) atomicOr(&s_match[u * 256 + (d[u] & 255u)], 1u << lane);
+            }
+            __syncwarp();
+#pragma unroll
+            for (int u = 0; u < kMatchItems; ++u)
+                peers[u] = ok[u] ? s_match[u * 256 + (d[u] & 255u)] : 0u;
+            __syncwarp();
+#pragma unroll
+            for (int u = 0; u < kMatchItems; ++u) {
+                // cleared for the next items
+                if (ok[u] && lane == __ffs(peers[u]) - 1) s_match[u * 256 + (d[u] & 255u)] = 0u;
+                peers[u] = match_bits<8, RB>(d[u], peers[u]);
+                prior[u] = 0;
+                if (ok[u] && lane == __ffs(peers[u]) - 1)
+                    prior[u] = atomicAdd(&hist[d[u] >> 1], (uint32_t)__popc(peers[u]) << ((d[u] & 1u) * 16)) >>
+                               ((d[u] & 1u) * 16);
+                __syncwarp();
+            }
+#pragma unroll
+            for (int u = 0; u < kMatchItems; ++u) {
+                const int leader = ok[u] ? __ffs(peers[u]) - 1 : lane;
+                pos.set(j0 + u, (__shfl_sync(0xffffffffu, prior[u], leader) & 0xffffu) + __popc(peers[u] & lt));
             }
         }
-    }
-    if constexpr (kValuePrefetch<RB>) asm volatile("cp.async.commit_group;\n" ::: "memory");
-    // the tile's digit counts first (order-free shared-memory atomics), published
-    // before the ranking so that the look-back of later tiles can start early
-#pragma unroll
-    for (int j = 0; j < kSortItems; ++j)
-        if (j * 32 < rem) atomicAdd(&s_count[(key[j] >> shift) & R::MASK], 1u);
-    __syncthreads();
-    // digit thread t owns digits t*DPT .. t*DPT + DPT - 1
-    const bool digit_thread = threadIdx.x < R::kDigitThreads;
-    const int d0 = threadIdx.x * DPT;
-    uint32_t tile_count[DPT];
-    uint32_t* lk = look + (size_t)tile * DIG;
-    // exclusive scan of the tile's counts over the digits (tile-local starts): the digit
-    // warps' totals here, the scan itself after the ranking (the counts are re-read from
-    // shared memory then, so nothing of this stays live across the ranking)
-    const auto warp_scan = [&](uint32_t& mine) {
-        mine = 0;
-#pragma unroll
-        for (int q = 0; q < DPT; ++q) {
-            tile_count[q] = digit_thread ? s_count[d0 + q] : 0u;
-            mine += tile_count[q];
-        }
-        uint32_t incl = mine;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t t = __shfl_up_sync(0xffffffffu, incl, o);
-            if (lane >= o) incl += t;
-        }
-        return incl;
-    };
-    if (digit_thread) {
-        uint32_t mine;
-        const uint32_t incl = warp_scan(mine);
-        if (lane == 31) s_w[warp] = incl;
-#pragma unroll
-        for (int q = 0; q < DPT; ++q)
-            if (tile > 0) st_relaxed_u32(&lk[d0 + q], kFlagA | tile_count[q]);
-    }
-    // tile 0 alone scans the pass's digit counts into the digits' global starts and
-    // publishes start + its own count as its inclusive prefix, so every later tile's
-    // look-back sum already holds its digit's global start
-    if (tile == 0) {
-        uint32_t hc[DPT], hmine = 0;
-#pragma unroll
-        for (int q = 0; q < DPT; ++q) {
-            hc[q] = digit_thread ? bins[d0 + q] : 0u;
-            hmine += hc[q];
-        }
-        uint32_t hincl = hmine;
-        if (digit_thread) {
+        __syncthreads();
+        // digit thread t owns digits 2t and 2t + 1: the tile's counts of them, published so that
+        // the look-back of later tiles can pass over this one
+        const bool digit_thread = threadIdx.x < R::kDigitThreads;
+        const int w0 = threadIdx.x, d0 = 2 * threadIdx.x;
+        uint64_t* lk = reinterpret_cast<uint64_t*>(look) + (size_t)tile * (DIG / 2) + w0;
+        const auto pair = [](uint32_t flag, uint32_t a, uint32_t b) {
+            return (uint64_t)(flag | (b & kValMask)) << 32 | (flag | (a & kValMask));
+        };
+        // exclusive scan over the digit threads: within the warp here, the warps' totals in tot
+        const auto scan = [&](uint32_t mine, uint32_t* tot) {
+            uint32_t incl = mine;
 #pragma unroll
             for (int o = 1; o < 32; o <<= 1) {
-                const uint32_t t = __shfl_up_sync(0xffffffffu, hincl, o);
-                if (lane >= o) hincl += t;
+                const uint32_t t = __shfl_up_sync(0xffffffffu, incl, o);
+                if (lane >= o) incl += t;
             }
-            if (lane == 31) s_hw[warp] = hincl;
+            if (lane == 31) tot[warp] = incl;
+            return incl - mine;
+        };
+        uint32_t count0 = 0, count1 = 0, first = 0, excl0 = 0, excl1 = 0;
+        if (digit_thread) {
+            uint32_t c = 0;
+#pragma unroll
+            for (int w = 0; w < kWarps; ++w) c += s_warp_hist[w][w0];
+            count0 = c & 0xffffu;
+            count1 = c >> 16;
+            if (tile > 0) st_relaxed_u64(lk, pair(kFlagA, count0, count1));
+            first = scan(count0 + count1, s_w);
+            // tile 0 alone scans the pass's digit counts into the digits' global starts and
+            // publishes start + its own count as its inclusive prefix, so every later tile's
+            // look-back sum already holds its digit's global start
+            if (tile == 0) {
+                const uint32_t b0 = bins[d0], b1 = bins[d0 + 1];
+                excl0 = scan(b0 + b1, s_hw);
+                excl1 = excl0 + b0;
+            }
         }
         __syncthreads();
         if (digit_thread) {
-            uint32_t hoff = hincl - hmine;
-            for (int w = 0; w < warp; ++w) hoff += s_hw[w];
-#pragma unroll
-            for (int q = 0; q < DPT; ++q) {
-                st_relaxed_u32(&lk[d0 + q], kFlagP | ((hoff + tile_count[q]) & kValMask));
-                s_delta[d0 + q] = hoff;   // this tile's exclusive prefix
-                hoff += hc[q];
-            }
-        }
-    }
-    // warp-level ranking (stable): the lanes holding the same digit, as the lanes that
-    // set their bit in the word of the digit's low 8 bits (shared-memory atomicOr) and,
-    // for 10-bit digits, agree on the top bits by ballot
-    const unsigned lt = (1u << lane) - 1u;
-#pragma unroll
-    for (int j = 0; j < kSortItems; ++j) {
-        const bool ok = j * 32 < rem;
-        const uint32_t dj = (key[j] >> shift) & R::MASK;
-        uint32_t* m = s_match + warp * 256 + (dj & 255u);
-        if (ok) atomicOr(m, 1u << lane);
-        __syncwarp();
-        const unsigned low = ok ? *m : 0u;
-        __syncwarp();
-        unsigned peers = low;
-#pragma unroll
-        for (int b = 8; b < RB; ++b) {
-            const unsigned bal = __ballot_sync(0xffffffffu, (dj >> b) & 1u);
-            peers &= ((dj >> b) & 1u) ? bal : ~bal;
-        }
-        // the lowest lane holding a low-8-bit value clears its word for the next item
-        if (ok && lane == __ffs(low) - 1) *m = 0u;
-        // the lowest lane of each group adds the group to the warp's digit count; the
-        // count before it comes back to the whole group by one full-warp shuffle
-        const int leader = peers ? __ffs(peers) - 1 : lane;
-        uint32_t prior = 0;
-        if (ok && lane == leader) {
-            prior = s_warp_hist[warp][dj];
-            s_warp_hist[warp][dj] = (uint16_t)(prior + __popc(peers));
-        }
-        prior = __shfl_sync(0xffffffffu, prior, leader);
-        rank[j] = prior + __popc(peers & lt);
-        __syncwarp();
-    }
-    __syncthreads();
-    // per digit: tile-local start, then the start of each warp's keys of that digit (in
-    // place of the warp's count)
-    uint32_t toff[DPT], excl[DPT];
-    if (digit_thread) {
-        uint32_t mine;
-        uint32_t o = warp_scan(mine) - mine;
-        for (int w = 0; w < warp; ++w) o += s_w[w];
-#pragma unroll
-        for (int q = 0; q < DPT; ++q) {
-            toff[q] = o;
-            uint32_t run = o;
+            for (int w = 0; w < warp; ++w) first += s_w[w];
+            // the start of each warp's keys of the two digits, in place of the warp's counts
+            uint32_t run = first | (first + count0) << 16;
 #pragma unroll
             for (int w = 0; w < kWarps; ++w) {
-                const uint32_t c = s_warp_hist[w][d0 + q];
-                s_warp_hist[w][d0 + q] = (uint16_t)run;
+                const uint32_t c = s_warp_hist[w][w0];
+                s_warp_hist[w][w0] = run;
                 run += c;
             }
-            o += tile_count[q];
-        }
-    }
-    // look back for the prefix of each owned digit: kLookWindow tiles at a time (the
-    // loads of all owned digits in flight together), summing the counts up to and
-    // including the nearest inclusive prefix (tile 0's holds the digit's global start)
-#pragma unroll
-    for (int q = 0; q < DPT; ++q) excl[q] = (digit_thread && tile == 0) ? s_delta[d0 + q] : 0u;
-    if (digit_thread && tile > 0) {
-        bool done[DPT];
-#pragma unroll
-        for (int q = 0; q < DPT; ++q) done[q] = false;
-        int64_t t = (int64_t)tile - 1;
-        uint32_t spins = 0;
-        while (true) {
-            bool all_done = true;
-#pragma unroll
-            for (int q = 0; q < DPT; ++q) all_done = all_done && done[q];
-            if (all_done) break;
-            uint32_t w[DPT][kLookWindow];
-#pragma unroll
-            for (int q = 0; q < DPT; ++q)
-#pragma unroll
-                for (int j = 0; j < kLookWindow; ++j)
-                    w[q][j] = (!done[q] && t - j >= 0) ? ld_relaxed_u32(&look[(size_t)(t - j) * DIG + d0 + q]) : kFlagP;
-            bool ready = true;
-#pragma unroll
-            for (int q = 0; q < DPT; ++q)
-#pragma unroll
-                for (int j = 0; j < kLookWindow; ++j) ready = ready && (w[q][j] & ~kValMask) != 0;
-            if (!ready) {
-                if (++spins > kSpinLimit) {
-                    atomicExch(err, 1);
-                    break;
+            if (tile == 0) {
+                for (int w = 0; w < warp; ++w) {
+                    excl0 += s_hw[w];
+                    excl1 += s_hw[w];
                 }
-                continue;
-            }
-#pragma unroll
-            for (int q = 0; q < DPT; ++q) {
-#pragma unroll
-                for (int j = 0; j < kLookWindow; ++j) {
-                    if (!done[q]) {
-                        excl[q] += w[q][j] & kValMask;
-                        done[q] = (w[q][j] & ~kValMask) == kFlagP;
-                    }
-                }
-            }
-            t -= kLookWindow;
-        }
-#pragma unroll
-        for (int q = 0; q < DPT; ++q) st_relaxed_u32(&lk[d0 + q], kFlagP | ((excl[q] + tile_count[q]) & kValMask));
-    }
-    if (digit_thread) {
-#pragma unroll
-        for (int q = 0; q < DPT; ++q) s_delta[d0 + q] = excl[q] - toff[q];
-    }
-    // each thread reads back only the values it copied itself, so its own wait suffices
-    if constexpr (kValuePrefetch<RB>) asm volatile("cp.async.wait_all;\n" ::: "memory");
-    __syncthreads();
-    if constexpr (kValuePrefetch<RB>) {
-        // stage keys in tile-sorted order, taking each thread's values out of the values'
-        // area (into the keys' registers) and their positions (into the ranks' registers)
-#pragma unroll
-        for (int j = 0; j < kSortItems; ++j) {
-            if (j * 32 < rem) {
-                const uint32_t dd = (key[j] >> shift) & R::MASK;
-                const uint32_t lp = s_warp_hist[warp][dd] + rank[j];
-                s_keys[lp] = key[j];
-                rank[j] = lp;
-                key[j] = s_vraw[warp * 32 * kSortItems + j * 32 + lane];
             }
         }
         __syncthreads();
-        // then the values
+        // stage the keys in tile-sorted order; the values are on their way during the look-back
 #pragma unroll
-        for (int j = 0; j < kSortItems; ++j)
-            if (j * 32 < rem) s_vals[rank[j]] = key[j];
-    } else {
-        // stage keys and values in tile-sorted order
-#pragma unroll
-        for (int j = 0; j < kSortItems; ++j) {
+        for (int j = 0; j < kItems; ++j) {
             if (j * 32 < rem) {
-                const uint32_t dd = (key[j] >> shift) & R::MASK;
-                const uint32_t lp = s_warp_hist[warp][dd] + rank[j];
-                s_keys[lp] = key[j];
-                s_vals[lp] = vin[wbase + j * 32 + lane];
+                const uint32_t d = (key[j] >> shift) & R::MASK;
+                const uint32_t q = pos.get(j) + ((hist[d >> 1] >> ((d & 1u) * 16)) & 0xffffu);
+                pos.set(j, q);
+                s_keys[q] = key[j];
+                key[j] = vin[wbase + j * 32 + lane];
             }
         }
-    }
-    __syncthreads();
-    const int valid = (int)(n - tbase < kSortTile ? n - tbase : kSortTile);
-    if (!cell_count) {
-        for (int i = threadIdx.x; i < valid; i += kSortThreads) {
-            const uint32_t k = s_keys[i];
-            const uint32_t g = s_delta[(k >> shift) & R::MASK] + (uint32_t)i;
-            kout[g] = k;
-            vout[g] = s_vals[i];
+        // look back for the prefix of the two digits: kLookWindow tiles at a time, summing the
+        // counts up to and including the nearest inclusive prefix (a tile publishes both digits'
+        // words in one store, so both reach it together)
+        if (digit_thread) {
+            if (tile > 0) {
+                int64_t t = (int64_t)tile - 1;
+                uint32_t spins = 0;
+                bool done = false;
+                while (!done) {
+                    uint64_t w[kLookWindow];
+                    bool ready = true;
+#pragma unroll
+                    for (int j = 0; j < kLookWindow; ++j) {
+                        w[j] = t - j >= 0 ? ld_volatile_u64(lk - (size_t)(tile - (t - j)) * (DIG / 2)) : pair(kFlagP, 0, 0);
+                        ready = ready && ((uint32_t)w[j] & ~kValMask) != 0;
+                    }
+                    if (!ready) {
+                        if (++spins > kSpinLimit) {
+                            atomicExch(err, 1);
+                            break;
+                        }
+                        continue;
+                    }
+#pragma unroll
+                    for (int j = 0; j < kLookWindow; ++j) {
+                        if (!done) {
+                            excl0 += (uint32_t)w[j] & kValMask;
+                            excl1 += (uint32_t)(w[j] >> 32) & kValMask;
+                            done = ((uint32_t)w[j] & ~kValMask) == kFlagP;
+                        }
+                    }
+                    t -= kLookWindow;
+                }
+            }
+            st_relaxed_u64(lk, pair(kFlagP, excl0 + count0, excl1 + count1));
+            s_delta[d0] = excl0 - first;
+            s_delta[d0 + 1] = excl1 - (first + count0);
         }
-        return;
-    }
-    // last pass with cell counts: the staged keys are the tile's keys in full order, so
-    // a warp's 32 consecutive keys form a few runs of equal cells; the last lane of each
-    // run adds the run's length (whole warps step together for the shuffles)
-    for (int b = threadIdx.x - lane; b < valid; b += kSortThreads) {
-        const int i = b + lane;
-        const bool ok = i < valid;
-        const uint32_t k = ok ? s_keys[i] : 0xffffffffu;
-        if (ok) {
-            const uint32_t g = s_delta[(k >> shift) & R::MASK] + (uint32_t)i;
-            kout[g] = k;
-            vout[g] = s_vals[i];
+#pragma unroll
+        for (int j = 0; j < kItems; ++j)
+            if (j * 32 < rem) s_vals[pos.get(j)] = key[j];
+        __syncthreads();
+        const int valid = FULL ? kTile : (int)(n - tbase);
+        if (!cell_count) {
+#pragma unroll (FULL ? 5 : 1)
+            for (int i = threadIdx.x; i < valid; i += kThreads) {
+                const uint32_t k = s_keys[i];
+                const uint32_t g = s_delta[(k >> shift) & R::MASK] + (uint32_t)i;
+                kout[g] = k;
+                vout[g] = s_vals[i];
+            }
+            return;
         }
-        const uint32_t prev = __shfl_up_sync(0xffffffffu, k, 1);
-        const uint32_t next = __shfl_down_sync(0xffffffffu, k, 1);
-        const unsigned starts = __ballot_sync(0xffffffffu, lane == 0 || k != prev);
-        if (ok && k < ncells && (lane == 31 || k != next)) {
-            const int first = 31 - __clz(starts & (0xffffffffu >> (31 - lane)));
-            atomicAdd(&cell_count[k], (uint32_t)(lane - first + 1));
+        // last pass with cell counts: the staged keys are the tile's keys in full order, so
+        // a warp's 32 consecutive keys form a few runs of equal cells; the last lane of each
+        // run adds the run's length (whole warps step together for the shuffles)
+        for (int b = threadIdx.x - lane; b < valid; b += kThreads) {
+            const int i = b + lane;
+            const bool ok = i < valid;
+            const uint32_t k = ok ? s_keys[i] : 0xffffffffu;
+            if (ok) {
+                const uint32_t g = s_delta[(k >> shift) & R::MASK] + (uint32_t)i;
+                kout[g] = k;
+                vout[g] = s_vals[i];
+            }
+            const uint32_t prev = __shfl_up_sync(0xffffffffu, k, 1);
+            const uint32_t next = __shfl_down_sync(0xffffffffu, k, 1);
+            const unsigned starts = __ballot_sync(0xffffffffu, lane == 0 || k != prev);
+            if (ok && k < ncells && (lane == 31 || k != next)) {
+                const int first = 31 - __clz(starts & (0xffffffffu >> (31 - lane)));
+                atomicAdd(&cell_count[k], (uint32_t)(lane - first + 1));
+            }
         }
-    }
+    };
+    if (n - tbase >= kTile) run(std::true_type());
+    else run(std::false_type());
 }
 
 // ---- small lists ----------------------------------------------------------------
@@ -1040,13 +1042,21 @@ cudaError_t radix_sort_pairs_u32(const uint32_t* kin, const uint32_t* vin, uint3
     cudaError_t e = radix_sort_begin(n, key_bits, scratch, st);
     if (e != cudaSuccess) return e;
     uint32_t* hist = radix_sort_hist(n, key_bits, scratch);
-    // about 16 keys per thread, at most two CTAs per SM
-    int64_t hb = (n + (int64_t)kHistThreads * 16 - 1) / ((int64_t)kHistThreads * 16);
-    if (hb < 1) hb = 1;
-    if (hb > 148 * 2) hb = 148 * 2;
-    if (L.digit_bits == 10) k_radix_histogram<10><<<(unsigned)hb, kHistThreads, 0, st>>>(kin, n, L.passes, hist);
-    else k_radix_histogram<8><<<(unsigned)hb, kHistThreads, 0, st>>>(kin, n, L.passes, hist);
-    e = cudaGetLastError();
+    const unsigned hb = (unsigned)std::min<int64_t>((n + 16 * kHistThreads - 1) / (16 * kHistThreads), 148);
+    const auto histogram = [&](auto kernel, int smem) -> cudaError_t {
+        cudaError_t a = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        if (a != cudaSuccess) return a;
+        kernel<<<hb, kHistThreads, smem, st>>>(kin, n, hist);
+        return cudaGetLastError();
+    };
+    if (L.digit_bits == 10)
+        e = L.passes == 2 ? histogram(k_radix_histogram<10, 2>, kHistSmem<10, 2>)
+                          : histogram(k_radix_histogram<10, 3>, kHistSmem<10, 3>);
+    else
+        e = L.passes == 1   ? histogram(k_radix_histogram<8, 1>, kHistSmem<8, 1>)
+            : L.passes == 2 ? histogram(k_radix_histogram<8, 2>, kHistSmem<8, 2>)
+            : L.passes == 3 ? histogram(k_radix_histogram<8, 3>, kHistSmem<8, 3>)
+                            : histogram(k_radix_histogram<8, 4>, kHistSmem<8, 4>);
     if (e != cudaSuccess) return e;
     return radix_sort_finish(kin, vin, kout, vout, n, key_bits, scratch, st, cell_count, ncells);
 }

@@ -192,14 +192,11 @@ __device__ __forceinline__ void gp_sincos2pi(float u, float* sn, float* cs) {
     pc = fmaf(z, pc, 1.0f / 24.0f);
     pc = fmaf(z, pc, -0.5f);
     float cy = fmaf(z, pc, 1.0f);
-    int q = ((int)qf) & 3;
-    float s_, c_;
-    if (q == 0) { s_ = sy; c_ = cy; }
-    else if (q == 1) { s_ = cy; c_ = -sy; }
-    else if (q == 2) { s_ = -sy; c_ = -cy; }
-    else { s_ = -cy; c_ = sy; }
-    *sn = s_;
-    *cs = c_;
+    // quadrant: odd ones swap sine and cosine, 2 and 3 negate the sine, 1 and 2 the cosine
+    const uint32_t q = (uint32_t)(int)qf;
+    const float s_ = q & 1u ? cy : sy, c_ = q & 1u ? sy : cy;
+    *sn = __uint_as_float(__float_as_uint(s_) ^ ((q & 2u) << 30));
+    *cs = __uint_as_float(__float_as_uint(c_) ^ (((q + 1u) & 2u) << 30));
 }
 
 
@@ -457,12 +454,11 @@ __device__ __forceinline__ int poisson(Stream& st, float lam) {
     return poisson_exact(st, lam);
 }
 
-__device__ __forceinline__ void normal2(Stream& st, float* z0, float* z1) {
-    float u1 = u01_open0(st.next());
-    float u2 = u01(st.next());
-    float rad = sqrtf(-2.0f * gp_logf(u1));
+// two normals from two draws (Box-Muller)
+__device__ __forceinline__ void normal2(uint32_t w0, uint32_t w1, float* z0, float* z1) {
+    float rad = sqrtf(-2.0f * log_draw(w0));
     float s, c;
-    gp_sincos2pi(u2, &s, &c);
+    gp_sincos2pi(u01(w1), &s, &c);
     *z0 = rad * c;
     *z1 = rad * s;
 }

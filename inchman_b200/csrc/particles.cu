@@ -6,7 +6,8 @@
 // re-sorts after every move (IndividualSolver::computeDiffusionConstants ->
 // sortSpecies, IndividualSolver.cpp:1100-1153, :673-712) and handles births and
 // deaths by scans and compaction (maintainPopulation, IndividualSolver.cpp:458-671).
-// This path keeps continuous positions (float2) and a species byte per particle;
+// This path keeps continuous positions (one float2 each, so that a gather is one access) and a
+// species byte per particle;
 // a step is
 //   move:    x += vx dt + sqrt(2 D dt) z (Box-Muller normals from the particle's
 //            Philox stream), reflecting walls, key = floor(y) G + floor(x);
@@ -16,9 +17,11 @@
 //            pair is removed with probability p (one 32-bit draw per pair against
 //            floor(p 2^32));
 //   compact: survivors in sorted order.
-// React and compact are one kernel over the cells that also scans the counts into
-// the cell starts.
+// In lists that fill their grid, react and compact go by the sorted list (k_pairs, k_compact);
+// in sparse ones they are one kernel over the cells, which also scans the counts into the
+// cell starts (k_react_compact).
 // Compiled with -fmad=false: positions must round as the CPU replay does.
+#include <algorithm>
 #include <cmath>
 #include <cstdint>
 #include <cuda_runtime.h>
@@ -41,58 +44,63 @@ __device__ __forceinline__ float reflect_into(float x, float L) {
 }
 
 // The move also counts the radix digits of the new keys for every sort pass (the
-// histogram the sort would otherwise read the keys again for).
-__global__ void k_move(float* __restrict__ px, float* __restrict__ py, int64_t n, int G, float sig, float ax, float ay,
-                       uint32_t seed, uint32_t step, uint32_t* __restrict__ keys, uint32_t* __restrict__ vals,
-                       uint32_t* __restrict__ hist, int passes, int rb) {
-    __shared__ uint32_t s_h[3 * 1024];   // [passes][1 << rb]: 4 x 256 or up to 3 x 1024
-    const int dig = 1 << rb;
-    const uint32_t dmask = (uint32_t)dig - 1u;
-    for (int i = threadIdx.x; i < passes * dig; i += blockDim.x) s_h[i] = 0;
+// histogram the sort would otherwise read the keys again for).  Bound by its instructions
+// (a Philox block, a logarithm, sine and cosine, a square root): one block of draws without
+// the stream's buffer, the passes unrolled, the next position loaded a round ahead, and no
+// index written (the sort's first pass makes it).  4.2M particles on 1024 x 1024: 52 us
+// before, 37 now.
+template <int RB, int PASSES>
+__global__ void __launch_bounds__(256, 6) k_move(float2* __restrict__ pos, int n, int G,
+                                                 float sig, float ax, float ay, uint32_t seed, uint32_t step,
+                                                 uint32_t* __restrict__ keys, uint32_t* __restrict__ hist) {
+    constexpr int DIG = 1 << RB;
+    __shared__ uint32_t s_h[PASSES * DIG];
+    for (int i = threadIdx.x; i < PASSES * DIG; i += blockDim.x) s_h[i] = 0;
     __syncthreads();
     const float L = (float)G;
     const int lane = threadIdx.x & 31;
-    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+    const int stride = (int)(gridDim.x * blockDim.x);
+    int i = (int)(blockIdx.x * blockDim.x + threadIdx.x);
+    float2 at = make_float2(0.0f, 0.0f);
+    if (i < n) at = pos[i];
     // whole warps step together (the digit counts below are warp-collective)
-    for (int64_t base = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) - lane; base < n; base += stride) {
-        const int64_t i = base + lane;
+    for (; i - lane < n; i += stride) {
         const bool valid = i < n;
-        const unsigned vmask = __ballot_sync(0xffffffffu, valid);
-        uint32_t k = 0;
+        const float2 from = at;
+        if (i + stride < n) at = pos[i + stride];      // n < 2^30, the grid has fewer threads than that
+        uint32_t w[4];
+        philox4x32_10(0u, step, (uint32_t)i, PH_PART, seed, 0u, w);
+        float z0, z1;
+        normal2(w[0], w[1], &z0, &z1);
+        float xn = from.x + ax;
+        xn = xn + sig * z0;
+        float yn = from.y + ay;
+        yn = yn + sig * z1;
+        xn = reflect_into(xn, L);
+        yn = reflect_into(yn, L);
+        const uint32_t k = (uint32_t)(int)yn * (uint32_t)G + (uint32_t)(int)xn;
         if (valid) {
-            Stream st;
-            st.init(seed, 0u, step, (uint32_t)i, PH_PART);
-            float z0, z1;
-            normal2(st, &z0, &z1);
-            float x = px[i] + ax;
-            x = x + sig * z0;
-            float y = py[i] + ay;
-            y = y + sig * z1;
-            x = reflect_into(x, L);
-            y = reflect_into(y, L);
-            px[i] = x;
-            py[i] = y;
-            k = (uint32_t)(int)y * (uint32_t)G + (uint32_t)(int)x;
+            pos[i] = make_float2(xn, yn);
             keys[i] = k;
-            vals[i] = (uint32_t)i;
         }
         // The particles come in the last step's cell order, so a warp's upper digits
         // are mostly all the same: one add for the warp then, one per lane otherwise.
-        const int lead = __ffs(vmask) - 1;
-        for (int p = 0; p < passes; ++p) {
-            const uint32_t d = (k >> (rb * p)) & dmask;
-            const uint32_t d0 = __shfl_sync(0xffffffffu, d, lead);
+        const unsigned vmask = __ballot_sync(0xffffffffu, valid);
+#pragma unroll
+        for (int p = 0; p < PASSES; ++p) {
+            const uint32_t d = (k >> (RB * p)) & (DIG - 1u);
+            const uint32_t d0 = __shfl_sync(0xffffffffu, d, 0);      // lane 0 is in range
             if (__all_sync(0xffffffffu, !valid || d == d0)) {
-                if (lane == lead) atomicAdd(&s_h[p * dig + d0], (uint32_t)__popc(vmask));
+                if (lane == 0) atomicAdd(&s_h[p * DIG + d0], (uint32_t)__popc(vmask));
             } else if (valid) {
-                atomicAdd(&s_h[p * dig + d], 1u);
+                atomicAdd(&s_h[p * DIG + d], 1u);
             }
         }
     }
     __syncthreads();
-    for (int i = threadIdx.x; i < passes * dig; i += blockDim.x) {
-        const uint32_t c = s_h[i];
-        if (c) atomicAdd(&hist[i], c);
+    for (int i2 = threadIdx.x; i2 < PASSES * DIG; i2 += blockDim.x) {
+        const uint32_t c = s_h[i2];
+        if (c) atomicAdd(&hist[i2], c);
     }
 }
 
@@ -140,11 +148,11 @@ __device__ __forceinline__ uint32_t block_excl_sum(uint32_t v, uint32_t* s_warp,
     return (warp == 0 ? 0u : s_warp[warp - 1]) + incl - v;
 }
 
-// Pairs one cell's A's and B's in order; dead pairs are marked in sp (kRcDead) or,
-// with alive != nullptr, cleared in alive.  Returns the number of pairs removed.
-template <class SP>
+// Pairs one cell's A's and B's in order; dead(place) is called for both of a pair that goes.
+// Returns the number of pairs removed.
+template <class SP, class DEAD>
 __device__ __forceinline__ uint32_t pair_cell(uint32_t b, uint32_t f, const SP& species, uint32_t seed, uint32_t step,
-                                              uint32_t cell, uint32_t thresh, uint8_t* mark, uint32_t* alive) {
+                                              uint32_t cell, uint32_t thresh, const DEAD& dead) {
     Stream st;
     st.init(seed, 1u, step, cell, PH_PAIR);
     uint32_t ia = b, ib = b, removed = 0;
@@ -153,13 +161,8 @@ __device__ __forceinline__ uint32_t pair_cell(uint32_t b, uint32_t f, const SP& 
         while (ib < f && species(ib) != 1) ib++;
         if (ia >= f || ib >= f) break;
         if (st.next() < thresh) {
-            if (mark) {
-                mark[ia] = kRcDead;
-                mark[ib] = kRcDead;
-            } else {
-                alive[ia] = 0;
-                alive[ib] = 0;
-            }
+            dead(ia);
+            dead(ib);
             removed++;
         }
         ia++;
@@ -175,9 +178,8 @@ __device__ __forceinline__ uint32_t pair_cell(uint32_t b, uint32_t f, const SP& 
 // are resident in one wave)
 __global__ void __launch_bounds__(kRcThreads, 8) k_react_compact(
     const uint32_t* __restrict__ count, uint32_t* __restrict__ start, int64_t ncells,
-    const uint32_t* __restrict__ svals, const float* __restrict__ x, const float* __restrict__ y,
-    const uint8_t* __restrict__ sp, uint32_t seed, uint32_t step, uint32_t thresh, uint32_t* __restrict__ alive,
-    float* __restrict__ x2, float* __restrict__ y2, uint8_t* __restrict__ sp2, uint64_t* __restrict__ scratch,
+    const uint32_t* __restrict__ svals, const float2* __restrict__ pos, const uint8_t* __restrict__ sp,
+    uint32_t seed, uint32_t step, uint32_t thresh, uint32_t* __restrict__ alive, float2* __restrict__ pos2, uint8_t* __restrict__ sp2, uint64_t* __restrict__ scratch,
     uint32_t ntiles, uint32_t cap) {
     extern __shared__ uint8_t s_sp[];          // [cap] species, kRcDead = removed
     __shared__ uint32_t s_tile, s_prefix;
@@ -245,9 +247,9 @@ __global__ void __launch_bounds__(kRcThreads, 8) k_react_compact(
 #pragma unroll
         for (int j = 0; j < kRcCells; ++j) {
             if (cnt[j] >= 2) {
-                Stream st;
-                st.init(seed, 1u, step, (uint32_t)(c0 + j), PH_PAIR);
                 if (cnt[j] <= 32) {
+                    Stream st;
+                    st.init(seed, 1u, step, (uint32_t)(c0 + j), PH_PAIR);
                     // species masks of the cell; the k-th set bits of the two masks pair
                     uint32_t am = 0, bm = 0;
                     for (uint32_t q = 0; q < cnt[j]; ++q) {
@@ -266,20 +268,8 @@ __global__ void __launch_bounds__(kRcThreads, 8) k_react_compact(
                         }
                     }
                 } else {
-                    uint32_t ia = o[j], ib = o[j];
-                    const uint32_t f = o[j + 1];
-                    for (;;) {
-                        while (ia < f && s_sp[ia] != 0) ia++;
-                        while (ib < f && s_sp[ib] != 1) ib++;
-                        if (ia >= f || ib >= f) break;
-                        if (st.next() < thresh) {
-                            s_sp[ia] = kRcDead;
-                            s_sp[ib] = kRcDead;
-                            removed++;
-                        }
-                        ia++;
-                        ib++;
-                    }
+                    removed += pair_cell(o[j], o[j + 1], [&](uint32_t q) { return s_sp[q]; }, seed, step,
+                                         (uint32_t)(c0 + j), thresh, [&](uint32_t q) { s_sp[q] = kRcDead; });
                 }
             }
         }
@@ -290,7 +280,7 @@ __global__ void __launch_bounds__(kRcThreads, 8) k_react_compact(
         for (int j = 0; j < kRcCells; ++j) {
             if (cnt[j] >= 2) {
                 removed += pair_cell(S + o[j], S + o[j + 1], global_sp, seed, step, (uint32_t)(c0 + j), thresh,
-                                     nullptr, alive);
+                                     [&](uint32_t q) { alive[q] = 0u; });
             }
         }
     }
@@ -317,8 +307,7 @@ __global__ void __launch_bounds__(kRcThreads, 8) k_react_compact(
             if (live) {
                 const uint32_t dd = d + __popc(m & ((1u << lane) - 1u));
                 const uint32_t src = svals[S + p];
-                x2[dd] = x[src];
-                y2[dd] = y[src];
+                pos2[dd] = pos[src];
                 sp2[dd] = s_sp[p];
             }
             d += __popc(m);
@@ -328,20 +317,339 @@ __global__ void __launch_bounds__(kRcThreads, 8) k_react_compact(
         for (uint32_t q = S + o[0]; q < S + o[kRcCells]; ++q) {
             if (removed && !alive[q]) continue;
             const uint32_t src = svals[q];
-            x2[d] = x[src];
-            y2[d] = y[src];
+            pos2[d] = pos[src];
             sp2[d] = sp[src];
             d++;
         }
     }
 }
 
-inline unsigned grid_of(int64_t n, int threads) {
-    int64_t b = (n + threads - 1) / threads;
-    if (b < 1) b = 1;
-    if (b > 148 * 32) b = 148 * 32;
-    return (unsigned)b;
+// The same from the sorted keys, for lists that fill their grid (particles_step_one), as two
+// kernels that wait for no other tile: k_pairs marks the removed places of the sorted list,
+// a bit each, and counts them per tile and per group of tiles; k_compact adds up the counts
+// before its tile and writes the survivors.  A tile is kRrTile places and owns the cells that
+// begin there.  Cells' starts and counts come from the places where the key changes, so the
+// sort need not count the cells; the cell after a gap of empty ones writes theirs.  A tile's
+// last cell may reach up to 256 places into the next tile; one that goes on after that is
+// paired in global memory.
+// Bound by the loads' latency and the instructions around them, so k_pairs takes eight places
+// per thread with 16-byte loads and keeps heads and species as bits (a place per lane and a
+// ballot per row: 33 us, now 26).  4.2M particles on 1024 x 1024, both kernels: 57 us, with
+// which k_react_compact and the counting in the sort are level (60); 16.8M on 1024 x 1024 a
+// step of 543 us against 674, 1M 90 against 101, 4.2M on 2000 x 2000 227 against 276.  As one
+// kernel with a look-back between pairs and survivors it took 84 to 94 us: 2048 tiles in
+// four waves, each waiting for its slowest.
+constexpr int kRrThreads = 256, kRrWarps = kRrThreads / 32, kRrRows = 8;
+constexpr int kRrTile = kRrThreads * kRrRows, kRrGroup = 1024;      // places of a tile, tiles of a group
+constexpr int kRrGroups = (1 << 30) / (kRrTile * kRrGroup);
+constexpr int kRrBigGap = 512, kRrGaps = 16;
+// removed places of a list of `tiles` tiles: counts per group and tile, then the bits
+struct Removed {
+    uint32_t *groups, *tile, *bits;
+    __host__ __device__ Removed(uint32_t* p, uint32_t tiles)
+        : groups(p), tile(p + kRrGroups), bits(p + kRrGroups + tiles) {}
+    static size_t words(uint32_t tiles) { return kRrGroups + (size_t)tiles * (1 + kRrTile / 32); }
+    __device__ __forceinline__ void add(uint32_t t, uint32_t count) const {
+        atomicAdd(&tile[t], count);
+        atomicAdd(&groups[t / kRrGroup], count);
+    }
+};
+// Every warp sums up the bits of words 0 .. W - 1 by itself: the total, and at(r), the bits
+// before this warp's word of row r.
+struct WordSums {
+    uint32_t v[3], all;
+    template <class WORD>
+    __device__ __forceinline__ WordSums(int words, const WORD& word) {
+        const int lane = threadIdx.x & 31;
+        uint32_t c[3], mine = 0;
+#pragma unroll
+        for (int u = 0; u < 3; ++u) {
+            c[u] = 3 * lane + u < words ? __popc(word(3 * lane + u)) : 0u;
+            mine += c[u];
+        }
+        uint32_t incl = mine;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t t = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += t;
+        }
+        v[0] = incl - mine;
+        v[1] = v[0] + c[0];
+        v[2] = v[1] + c[1];
+        all = __shfl_sync(0xffffffffu, incl, 31);
+    }
+    __device__ __forceinline__ uint32_t at(int r) const {
+        const int w = r * kRrWarps + (threadIdx.x >> 5), u = w % 3;
+        return __shfl_sync(0xffffffffu, u == 0 ? v[0] : u == 1 ? v[1] : v[2], w / 3);
+    }
+};
+
+__global__ void __launch_bounds__(kRrThreads, 6) k_pairs(
+    const uint32_t* __restrict__ skeys, const uint32_t* __restrict__ svals, uint32_t n, uint32_t ncells,
+    const uint8_t* __restrict__ sp, uint32_t seed, uint32_t step, uint32_t thresh, uint32_t* __restrict__ start,
+    uint32_t* __restrict__ count, Removed removed) {
+    constexpr int kSpan = kRrTile + kRrThreads;     // places a tile looks at
+    constexpr int kWords = kSpan / 32;              // a bit per place: a thread's eight are a byte
+    __shared__ __align__(16) uint32_t s_key[kRrTile];
+    __shared__ uint16_t s_head[kRrTile + 1];        // the tile's cells: their first places, then the end
+    __shared__ uint32_t s_dead[kWords];             // removed places
+    __shared__ uint32_t s_a[kWords + 1], s_b[kWords + 1];      // places of species 0 and 1
+    __shared__ uint32_t s_cnt[kRrWarps];
+    __shared__ uint32_t s_end, s_ngaps;
+    __shared__ uint32_t s_gap[kRrGaps][3];          // long gaps: first cell, cell after, start
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const uint32_t tile = blockIdx.x, i0 = tile * kRrTile;
+    const uint32_t m = min(n - i0, (uint32_t)kSpan);          // places there are
+    const uint32_t own = min(m, (uint32_t)kRrTile);
+    // eight places from p on: keys and species bits (places past the list: key 2^32 - 1)
+    uint32_t key[8], abits, bbits;
+    const auto load = [&](uint32_t p) {
+        uint32_t src[8];
+        if (p + 8 <= m) {
+            const uint4* k = reinterpret_cast<const uint4*>(skeys + i0 + p);
+            const uint4* v = reinterpret_cast<const uint4*>(svals + i0 + p);
+            const uint4 k0 = k[0], k1 = k[1], v0 = v[0], v1 = v[1];
+            key[0] = k0.x; key[1] = k0.y; key[2] = k0.z; key[3] = k0.w;
+            key[4] = k1.x; key[5] = k1.y; key[6] = k1.z; key[7] = k1.w;
+            src[0] = v0.x; src[1] = v0.y; src[2] = v0.z; src[3] = v0.w;
+            src[4] = v1.x; src[5] = v1.y; src[6] = v1.z; src[7] = v1.w;
+        } else {
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                key[j] = p + j < m ? skeys[i0 + p + j] : 0xffffffffu;
+                src[j] = p + j < m ? svals[i0 + p + j] : 0u;
+            }
+        }
+        uint8_t t[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) t[j] = sp[src[j]];
+        abits = bbits = 0;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            abits |= (uint32_t)(t[j] == 0) << j;
+            bbits |= (uint32_t)(t[j] == 1) << j;
+        }
+    };
+    // which of the eight begin a cell; before: the key of the place before them
+    const auto begins = [&](uint32_t before) {
+        uint32_t h = 0;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) h |= (uint32_t)(key[j] != (j ? key[j - 1] : before)) << j;
+        return h;
+    };
+    uint8_t* a8 = reinterpret_cast<uint8_t*>(s_a);
+    uint8_t* b8 = reinterpret_cast<uint8_t*>(s_b);
+    const uint32_t p0 = 8 * tid;
+    if (tid < kWords) s_dead[tid] = 0;
+    if (tid == 0) {
+        s_ngaps = 0;
+        s_a[kWords] = s_b[kWords] = 0;
+    }
+    if (warp == 0) {
+        // the places after the tile's own: where its last cell ends, if in sight
+        load(kRrTile + p0);
+        uint32_t before = __shfl_up_sync(0xffffffffu, key[7], 1);
+        if (lane == 0) before = m > kRrTile ? skeys[i0 + kRrTile - 1] : 0xffffffffu;
+        const uint32_t h = begins(before);
+        const unsigned any = __ballot_sync(0xffffffffu, h != 0);
+        const uint32_t mine = kRrTile + p0 + __ffs(h) - 1;
+        const uint32_t e = __shfl_sync(0xffffffffu, mine, any ? __ffs(any) - 1 : 0);
+        if (lane == 0) s_end = any ? e : (uint32_t)kSpan;
+        a8[kRrTile / 8 + tid] = (uint8_t)abits;
+        b8[kRrTile / 8 + tid] = (uint8_t)bbits;
+    }
+    load(p0);
+    uint32_t heads;
+    {
+        uint32_t before = __shfl_up_sync(0xffffffffu, key[7], 1);
+        if (lane == 0) before = i0 + p0 && p0 < m ? skeys[i0 + p0 - 1] : 0xffffffffu;
+        heads = begins(before);
+        // the list's end is not a cell's beginning
+        if (p0 + 8 > m) heads &= p0 < m ? (1u << (m - p0)) - 1u : 0u;
+    }
+    a8[tid] = (uint8_t)abits;
+    b8[tid] = (uint8_t)bbits;
+    reinterpret_cast<uint4*>(s_key)[2 * tid] = make_uint4(key[0], key[1], key[2], key[3]);
+    reinterpret_cast<uint4*>(s_key)[2 * tid + 1] = make_uint4(key[4], key[5], key[6], key[7]);
+    uint32_t incl = __popc(heads);
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t t = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += t;
+    }
+    if (lane == 31) s_cnt[warp] = incl;
+    __syncthreads();
+    uint32_t at = incl - __popc(heads), nheads = 0;
+#pragma unroll
+    for (int w = 0; w < kRrWarps; ++w) {
+        at += w < warp ? s_cnt[w] : 0u;
+        nheads += s_cnt[w];
+    }
+#pragma unroll
+    for (int j = 0; j < 8; ++j)
+        if (heads >> j & 1u) s_head[at++] = (uint16_t)(p0 + j);
+    // the last cell ends at a beginning in sight, at the list's end, or out of sight
+    const uint32_t head_end = s_end;
+    const bool big = nheads > 0 && head_end == kSpan && n - i0 > kSpan;
+    if (tid == 0) s_head[nheads] = (uint16_t)(m <= kRrTile ? m : min(head_end, m));
+    __syncthreads();
+    const uint32_t cells = nheads - (big ? 1u : 0u);           // cells to pair here
+    // the cells a .. b - 1 are empty and would start at place q
+    const auto fill = [&](uint32_t a, uint32_t b, uint32_t q, uint32_t from, uint32_t by) {
+        for (uint32_t c = a + from; c < b; c += by) {
+            start[c] = q;
+            count[c] = 0u;
+        }
+    };
+    const auto dead = [&](uint32_t q) { atomicOr(&s_dead[q >> 5], 1u << (q & 31u)); };
+    for (uint32_t c0 = warp * 32; c0 < nheads; c0 += kRrThreads) {
+        const uint32_t c = c0 + lane;
+        uint32_t cell = 0, gap0 = 0, p = 0;
+        if (c < nheads) {
+            p = s_head[c];
+            cell = s_key[p];
+            gap0 = p ? s_key[p - 1] + 1u : i0 ? skeys[i0 - 1] + 1u : 0u;
+            start[cell] = i0 + p;
+        }
+        if (c < cells) {
+            const uint32_t f = s_head[c + 1], cnt = f - p;
+            count[cell] = cnt;
+            if (cnt <= 32) {
+                // species masks of the cell; the k-th set bits of the two masks pair
+                const uint32_t w = p >> 5, mask = 0xffffffffu >> (32 - cnt);
+                uint32_t am = __funnelshift_r(s_a[w], s_a[w + 1], p) & mask;
+                uint32_t bm = __funnelshift_r(s_b[w], s_b[w + 1], p) & mask;
+                if (am && bm) {
+                    Stream st;
+                    st.init(seed, 1u, step, cell, PH_PAIR);
+                    do {
+                        uint32_t d[4];
+                        st.block(d);
+#pragma unroll
+                        for (int u = 0; u < 4; ++u) {
+                            if (am && bm && d[u] < thresh) {
+                                dead(p + __ffs(am) - 1);
+                                dead(p + __ffs(bm) - 1);
+                            }
+                            am &= am - 1u;
+                            bm &= bm - 1u;
+                        }
+                    } while (am && bm);
+                }
+            } else {
+                pair_cell(p, f, [&](uint32_t q) {
+                    const uint32_t bit = q & 31u;
+                    return s_a[q >> 5] >> bit & 1u ? 0 : s_b[q >> 5] >> bit & 1u ? 1 : 2;
+                }, seed, step, cell, thresh, dead);
+            }
+        }
+        // empty cells before this one: a few by the thread, more by the warp, many by the
+        // block below
+        const uint32_t gap = c < nheads ? cell - gap0 : 0u;
+        bool wide = gap > 4;
+        if (gap >= kRrBigGap) {
+            const uint32_t slot = atomicAdd(&s_ngaps, 1u);
+            if (slot < kRrGaps) {
+                s_gap[slot][0] = gap0;
+                s_gap[slot][1] = cell;
+                s_gap[slot][2] = i0 + p;
+                wide = false;
+            }
+        } else if (!wide) {
+            fill(gap0, cell, i0 + p, 0, 1);
+        }
+        for (unsigned todo = __ballot_sync(0xffffffffu, wide); todo; todo &= todo - 1u) {
+            const int l = __ffs(todo) - 1;
+            fill(__shfl_sync(0xffffffffu, gap0, l), __shfl_sync(0xffffffffu, cell, l),
+                 i0 + __shfl_sync(0xffffffffu, p, l), lane, 32);
+        }
+    }
+    __syncthreads();
+    // the tile's bits are words 0 .. 63 (warps 0 and 1), the next tile's the rest (warp 2)
+    if (warp < 3) {
+        const uint32_t w = tid < kWords ? s_dead[tid] : 0u;
+        if (w) atomicOr(&removed.bits[(size_t)tile * (kRrTile / 32) + tid], w);
+        const uint32_t sum = __reduce_add_sync(0xffffffffu, (uint32_t)__popc(w));
+        if (sum && lane == 0) removed.add(tile + (warp == 2 ? 1u : 0u), sum);
+    }
+    const uint32_t gaps = min(s_ngaps, (uint32_t)kRrGaps);
+    for (uint32_t g = 0; g < gaps; ++g) fill(s_gap[g][0], s_gap[g][1], s_gap[g][2], tid, kRrThreads);
+    if (tile == gridDim.x - 1) fill(s_key[own - 1] + 1u, ncells, n, tid, kRrThreads);
+    if (big && tid == 0) {
+        const uint32_t p = i0 + s_head[cells], cell = s_key[s_head[cells]];
+        uint32_t lo = i0 + kSpan, hi = n;      // every place before lo that is not before p is the cell's
+        while (lo < hi) {
+            const uint32_t mid = lo + (hi - lo) / 2;
+            if (skeys[mid] == cell) lo = mid + 1;
+            else hi = mid;
+        }
+        count[cell] = lo - p;
+        pair_cell(p, lo, [&](uint32_t q) { return sp[svals[q]]; }, seed, step, cell, thresh, [&](uint32_t q) {
+            atomicOr(&removed.bits[q >> 5], 1u << (q & 31u));
+            removed.add(q / kRrTile, 1u);
+        });
+    }
 }
+
+__global__ void __launch_bounds__(kRrThreads, 6) k_compact(
+    const uint32_t* __restrict__ svals, uint32_t n, const float2* __restrict__ pos, const uint8_t* __restrict__ sp,
+    Removed removed, float2* __restrict__ pos2, uint8_t* __restrict__ sp2, uint32_t* __restrict__ total) {
+    __shared__ uint32_t s_sum[kRrWarps];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const uint32_t tile = blockIdx.x, i0 = tile * kRrTile, m = min(n - i0, (uint32_t)kRrTile);
+    uint32_t src[kRrRows], word[kRrRows];
+#pragma unroll
+    for (int r = 0; r < kRrRows; ++r) {
+        const uint32_t p = r * kRrThreads + tid;
+        src[r] = p < m ? svals[i0 + p] : 0u;
+        word[r] = removed.bits[(size_t)tile * (kRrTile / 32) + r * kRrWarps + warp];
+    }
+    // removed places before the tile
+    const uint32_t group = tile / kRrGroup;
+    uint32_t sum = 0;
+    for (uint32_t g = tid; g < group; g += kRrThreads) sum += removed.groups[g];
+    for (uint32_t t = group * kRrGroup + tid; t < tile; t += kRrThreads) sum += removed.tile[t];
+    sum = __reduce_add_sync(0xffffffffu, sum);
+    if (lane == 0) s_sum[warp] = sum;
+    const WordSums gone(kRrTile / 32, [&](int w) { return removed.bits[(size_t)tile * (kRrTile / 32) + w]; });
+    float2 at[kRrRows];
+    uint8_t sv[kRrRows];
+#pragma unroll
+    for (int r = 0; r < kRrRows; ++r) {
+        if ((uint32_t)(r * kRrThreads + tid) < m) {
+            at[r] = pos[src[r]];
+            sv[r] = sp[src[r]];
+        }
+    }
+    __syncthreads();
+    uint32_t base = i0;
+#pragma unroll
+    for (int w = 0; w < kRrWarps; ++w) base -= s_sum[w];
+    if (tile == gridDim.x - 1 && tid == 0) *total = base + m - gone.all;
+#pragma unroll
+    for (int r = 0; r < kRrRows; ++r) {
+        const uint32_t p = r * kRrThreads + tid;
+        const uint32_t d = base + p - gone.at(r) - __popc(word[r] & ((1u << lane) - 1u));
+        if (p < m && !(word[r] >> lane & 1u)) {
+            pos2[d] = at[r];
+            sp2[d] = sv[r];
+        }
+    }
+}
+
+// positions between the caller's two arrays and the steps' one
+__global__ void k_join(const float* __restrict__ x, const float* __restrict__ y, float2* __restrict__ pos, int64_t n) {
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
+        pos[i] = make_float2(x[i], y[i]);
+}
+__global__ void k_split(const float2* __restrict__ pos, float* __restrict__ x, float* __restrict__ y, int64_t n) {
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+        const float2 p = pos[i];
+        x[i] = p.x;
+        y[i] = p.y;
+    }
+}
+inline unsigned grid_of(int64_t n) { return (unsigned)std::min<int64_t>((n + 255) / 256, 148 * 8); }
 
 }  // namespace
 
@@ -353,11 +661,12 @@ struct gpgmp_particles {
     int32_t step = 0;
     int key_bits = 32;
     cudaStream_t stream = nullptr;
-    float *x = nullptr, *y = nullptr, *x2 = nullptr, *y2 = nullptr;
+    float2 *pos = nullptr, *pos2 = nullptr;      // pos2: the next step's, and free between steps
     uint8_t *sp = nullptr, *sp2 = nullptr;
-    uint32_t *keys = nullptr, *vals = nullptr, *skeys = nullptr, *svals = nullptr;
+    uint32_t *keys = nullptr, *skeys = nullptr, *svals = nullptr;
     uint32_t *start = nullptr, *count = nullptr, *alive = nullptr;
     void* sort_scratch = nullptr;
+    uint32_t* removed = nullptr;     // k_pairs: counts and bits of the removed places
     uint64_t* rc_scratch = nullptr;  // react + compact: tile counter, error word, total, scan status words
     uint32_t rc_tiles = 0;
     uint32_t* host_tail = nullptr;   // pinned: the number of particles after a step
@@ -374,8 +683,8 @@ extern "C" {
 int gpgmp_particles_destroy(gpgmp_particles* h) {
     if (!h) return GPGMP_OK;
     cudaStreamSynchronize(h->stream);
-    void* ptrs[] = {h->x, h->y, h->x2, h->y2, h->sp, h->sp2, h->keys, h->vals, h->skeys, h->svals, h->start,
-                    h->count, h->alive, h->sort_scratch, h->rc_scratch};
+    void* ptrs[] = {h->pos, h->pos2, h->sp, h->sp2, h->keys, h->skeys, h->svals, h->start,
+                    h->count, h->alive, h->sort_scratch, h->removed, h->rc_scratch};
     for (void* p : ptrs)
         if (p) cudaFree(p);
     if (h->host_tail) cudaFreeHost(h->host_tail);
@@ -402,15 +711,15 @@ int gpgmp_particles_create(int64_t capacity, int32_t grid, float D, float vx, fl
     const size_t n4 = sizeof(uint32_t) * (size_t)capacity;
     cudaError_t e = cudaSuccess;
     auto A = [&](void** p, size_t b) { if (e == cudaSuccess) e = cudaMalloc(p, b); };
-    A((void**)&h->x, sizeof(float) * capacity); A((void**)&h->y, sizeof(float) * capacity);
-    A((void**)&h->x2, sizeof(float) * capacity); A((void**)&h->y2, sizeof(float) * capacity);
+    A((void**)&h->pos, sizeof(float2) * capacity); A((void**)&h->pos2, sizeof(float2) * capacity);
     A((void**)&h->sp, capacity); A((void**)&h->sp2, capacity);
-    A((void**)&h->keys, n4); A((void**)&h->vals, n4); A((void**)&h->skeys, n4); A((void**)&h->svals, n4);
+    A((void**)&h->keys, n4); A((void**)&h->skeys, n4); A((void**)&h->svals, n4);
     A((void**)&h->alive, n4);
     A((void**)&h->start, sizeof(uint32_t) * (size_t)ncells); A((void**)&h->count, sizeof(uint32_t) * (size_t)ncells);
     A(&h->sort_scratch, sort_layout(capacity, bits).bytes);
     h->rc_tiles = (uint32_t)((ncells + kRcTile - 1) / kRcTile);
     A((void**)&h->rc_scratch, sizeof(uint64_t) * (4 + 2 * (size_t)h->rc_tiles));
+    A((void**)&h->removed, sizeof(uint32_t) * Removed::words((uint32_t)((capacity + kRrTile - 1) / kRrTile)));
     if (e == cudaSuccess) e = cudaMallocHost((void**)&h->host_tail, 2 * sizeof(uint32_t));
     if (e != cudaSuccess) {
         int c = set_error(e == cudaErrorMemoryAllocation ? GPGMP_ERR_NOMEM : GPGMP_ERR_CUDA, "allocation: %s",
@@ -431,8 +740,13 @@ int gpgmp_particles_set_stream(gpgmp_particles* h, void* stream) {
 int gpgmp_particles_set(gpgmp_particles* h, const float* x, const float* y, const uint8_t* species, int64_t n,
                         int32_t step) {
     if (!h || n < 0 || n > h->cap || (n > 0 && (!x || !y || !species))) return set_error(GPGMP_ERR_INVALID, "bad argument");
-    CK(cudaMemcpyAsync(h->x, x, sizeof(float) * n, cudaMemcpyHostToDevice, h->stream));
-    CK(cudaMemcpyAsync(h->y, y, sizeof(float) * n, cudaMemcpyHostToDevice, h->stream));
+    float *dx = reinterpret_cast<float*>(h->pos2), *dy = dx + h->cap;
+    CK(cudaMemcpyAsync(dx, x, sizeof(float) * n, cudaMemcpyHostToDevice, h->stream));
+    CK(cudaMemcpyAsync(dy, y, sizeof(float) * n, cudaMemcpyHostToDevice, h->stream));
+    if (n > 0) {
+        k_join<<<grid_of(n), 256, 0, h->stream>>>(dx, dy, h->pos, n);
+        CK(cudaGetLastError());
+    }
     CK(cudaMemcpyAsync(h->sp, species, n, cudaMemcpyHostToDevice, h->stream));
     CK(cudaStreamSynchronize(h->stream));
     h->n = n;
@@ -442,8 +756,13 @@ int gpgmp_particles_set(gpgmp_particles* h, const float* x, const float* y, cons
 
 int gpgmp_particles_get(gpgmp_particles* h, float* x, float* y, uint8_t* species, int64_t* n) {
     if (!h || !n) return set_error(GPGMP_ERR_INVALID, "bad argument");
-    if (x) CK(cudaMemcpyAsync(x, h->x, sizeof(float) * h->n, cudaMemcpyDeviceToHost, h->stream));
-    if (y) CK(cudaMemcpyAsync(y, h->y, sizeof(float) * h->n, cudaMemcpyDeviceToHost, h->stream));
+    float *dx = reinterpret_cast<float*>(h->pos2), *dy = dx + h->cap;
+    if ((x || y) && h->n > 0) {
+        k_split<<<grid_of(h->n), 256, 0, h->stream>>>(h->pos, dx, dy, h->n);
+        CK(cudaGetLastError());
+    }
+    if (x) CK(cudaMemcpyAsync(x, dx, sizeof(float) * h->n, cudaMemcpyDeviceToHost, h->stream));
+    if (y) CK(cudaMemcpyAsync(y, dy, sizeof(float) * h->n, cudaMemcpyDeviceToHost, h->stream));
     if (species) CK(cudaMemcpyAsync(species, h->sp, h->n, cudaMemcpyDeviceToHost, h->stream));
     CK(cudaStreamSynchronize(h->stream));
     *n = h->n;
@@ -458,36 +777,61 @@ static int particles_step_one(gpgmp_particles* h) {
     const float sig = sqrtf(2.0f * h->D * h->dt);
     const float ax = h->vx * h->dt, ay = h->vy * h->dt;
     const uint32_t step = (uint32_t)h->step;
-    CK(cudaMemsetAsync(h->count, 0, sizeof(uint32_t) * (size_t)ncells, st));
+    // k_pairs goes by the particles, k_react_compact by the cells.  At 0.57 particles per cell
+    // a step takes 86 us the one way and 98 the other (1024 x 1024 cells); the line is lower,
+    // where the longest run of empty cells, which one block of k_pairs writes, could cost
+    // more than the cells' kernel (half a cell per particle: 1M cells, at most 20 us).
+    const bool rows = 2 * n >= ncells;
+    if (!rows) CK(cudaMemsetAsync(h->count, 0, sizeof(uint32_t) * (size_t)ncells, st));
     if (n > 0) {
         CK(radix_sort_begin(n, h->key_bits, h->sort_scratch, st));
         const SortLayout L = sort_layout(n, h->key_bits);
-        k_move<<<grid_of(n, 256 * 8), 256, 0, st>>>(h->x, h->y, n, h->grid, sig, ax, ay, h->seed, step, h->keys,
-                                                     h->vals, radix_sort_hist(n, h->key_bits, h->sort_scratch),
-                                                     L.passes, L.digit_bits);
+        const unsigned blocks = (unsigned)std::min<int64_t>((n + 255) / 256, 148 * 6);
+        const auto move = [&](auto kernel) {
+            kernel<<<blocks, 256, 0, st>>>(h->pos, (int)n, h->grid, sig, ax, ay, h->seed, step, h->keys,
+                                           radix_sort_hist(n, h->key_bits, h->sort_scratch));
+        };
+        if (L.digit_bits == 10) {
+            if (L.passes == 2) move(k_move<10, 2>);
+            else move(k_move<10, 3>);
+        } else {
+            if (L.passes == 1) move(k_move<8, 1>);
+            else if (L.passes == 2) move(k_move<8, 2>);
+            else move(k_move<8, 3>);      // at most 30 bits: four passes of 8 are three of 10
+        }
         CK(cudaGetLastError());
-        // the last pass also counts the particles per cell
-        CK(radix_sort_finish(h->keys, h->vals, h->skeys, h->svals, n, h->key_bits, h->sort_scratch, st, h->count,
-                             ncells));
+        // where k_react_compact follows, the last pass also counts the particles per cell
+        CK(radix_sort_finish(h->keys, nullptr, h->skeys, h->svals, n, h->key_bits, h->sort_scratch, st,
+                             rows ? nullptr : h->count, ncells));
     }
-    CK(cudaMemsetAsync(h->rc_scratch, 0, sizeof(uint64_t) * (4 + 2 * (size_t)h->rc_tiles), st));
-    // staging for twice the mean number of particles per tile (+ 1024), up to 47 KB
-    // (with the static shared memory, within the 48 KB a launch gets without opting in)
-    uint64_t want = (uint64_t)(2.0 * (double)n * kRcTile / (double)ncells) + 1024;
-    if (want > 47 * 1024) want = 47 * 1024;
-    const uint32_t cap = (uint32_t)want;
-    k_react_compact<<<h->rc_tiles, kRcThreads, cap, st>>>(
-        h->count, h->start, ncells, h->svals, h->x, h->y, h->sp, h->seed, step, h->thresh, h->alive, h->x2, h->y2,
-        h->sp2, h->rc_scratch, h->rc_tiles, cap);
-    CK(cudaGetLastError());
+    if (rows) {
+        const uint32_t tiles = (uint32_t)((n + kRrTile - 1) / kRrTile);
+        const Removed removed(h->removed, tiles);
+        CK(cudaMemsetAsync(h->removed, 0, sizeof(uint32_t) * Removed::words(tiles), st));
+        k_pairs<<<tiles, kRrThreads, 0, st>>>(h->skeys, h->svals, (uint32_t)n, (uint32_t)ncells, h->sp, h->seed, step,
+                                              h->thresh, h->start, h->count, removed);
+        CK(cudaGetLastError());
+        k_compact<<<tiles, kRrThreads, 0, st>>>(h->svals, (uint32_t)n, h->pos, h->sp, removed, h->pos2, h->sp2,
+                                                reinterpret_cast<uint32_t*>(h->rc_scratch) + 4);
+        CK(cudaGetLastError());
+    } else {
+        CK(cudaMemsetAsync(h->rc_scratch, 0, sizeof(uint64_t) * (4 + 2 * (size_t)h->rc_tiles), st));
+        // staging for twice the mean number of particles per tile (+ 1024), up to 47 KB
+        // (with the static shared memory, within the 48 KB a launch gets without opting in)
+        uint64_t want = (uint64_t)(2.0 * (double)n * kRcTile / (double)ncells) + 1024;
+        if (want > 47 * 1024) want = 47 * 1024;
+        const uint32_t cap = (uint32_t)want;
+        k_react_compact<<<h->rc_tiles, kRcThreads, cap, st>>>(
+            h->count, h->start, ncells, h->svals, h->pos, h->sp, h->seed, step, h->thresh, h->alive, h->pos2, h->sp2,
+            h->rc_scratch, h->rc_tiles, cap);
+        CK(cudaGetLastError());
+    }
     CK(cudaMemcpyAsync(&h->host_tail[0], reinterpret_cast<uint32_t*>(h->rc_scratch) + 4, sizeof(uint32_t),
                        cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
     h->n = (int64_t)h->host_tail[0];
     {
-        float* t;
-        t = h->x; h->x = h->x2; h->x2 = t;
-        t = h->y; h->y = h->y2; h->y2 = t;
+        float2* t = h->pos; h->pos = h->pos2; h->pos2 = t;
         uint8_t* ts = h->sp; h->sp = h->sp2; h->sp2 = ts;
     }
     h->step++;

@@ -626,7 +626,7 @@ __global__ void __launch_bounds__(SortShape<RB>::kThreads, SortShape<RB>::kMinBl
                 const uint32_t q = pos.get(j) + ((hist[d >> 1] >> ((d & 1u) * 16)) & 0xffffu);
                 pos.set(j, q);
                 s_keys[q] = key[j];
-                key[j] = vin[wbase + j * 32 + lane];
+                key[j] = vin ? vin[wbase + j * 32 + lane] : (uint32_t)(wbase + j * 32 + lane);
             }
         }
         // look back for the prefix of the two digits: kLookWindow tiles at a time, summing the

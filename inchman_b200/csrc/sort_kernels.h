@@ -28,7 +28,8 @@ cudaError_t radix_sort_pairs_u32(const uint32_t* kin, const uint32_t* vin, uint3
 // The same in two halves around a caller's kernel that adds the digit counts of every
 // pass ([passes][1 << digit_bits], radix_sort_hist) while it writes the keys: begin clears the
 // scratch, finish sorts.  With cell_count (zeroed by the caller), the last pass also
-// adds the number of keys equal to each c < ncells into cell_count[c].
+// adds the number of keys equal to each c < ncells into cell_count[c].  vin == nullptr in
+// finish: the values are the keys' indexes.
 cudaError_t radix_sort_begin(int64_t n, int key_bits, void* scratch, cudaStream_t st);
 uint32_t* radix_sort_hist(int64_t n, int key_bits, void* scratch);
 cudaError_t radix_sort_finish(const uint32_t* kin, const uint32_t* vin, uint32_t* kout, uint32_t* vout, int64_t n,

@@ -485,7 +485,7 @@ __global__ void __launch_bounds__(SortShape<RB>::kThreads, SortShape<RB>::kMinBl
                                                            int64_t n, int shift, const uint32_t* __restrict__ bins,
                                                            uint32_t* __restrict__ look, unsigned int* tile_counter,
                                                            int* err, uint32_t* __restrict__ cell_count,
-                                                           uint32_t ncells) {
+                                                           uint32_t ncells, const uint32_t* __restrict__ count) {
     using R = Radix<RB>;
     constexpr int kThreads = SortShape<RB>::kThreads, kItems = SortShape<RB>::kItems;
     constexpr int kTile = SortShape<RB>::kTile;
@@ -512,6 +512,10 @@ __global__ void __launch_bounds__(SortShape<RB>::kThreads, SortShape<RB>::kMinBl
     __syncthreads();
     const uint32_t tile = s_tile;
     const int64_t tbase = (int64_t)tile * kTile;
+    if (count) {      // the list may be shorter than the launch; no tile waits for a later one
+        n = *count;
+        if (tbase >= n) return;
+    }
     const int64_t wbase = tbase + (int64_t)warp * 32 * kItems;
     // a tile with every key in range needs no tests of the items
     const auto run = [&](auto all) {
@@ -981,7 +985,8 @@ uint32_t* radix_sort_hist(int64_t n, int key_bits, void* scratch) {
 }
 
 cudaError_t radix_sort_finish(const uint32_t* kin, const uint32_t* vin, uint32_t* kout, uint32_t* vout, int64_t n,
-                              int key_bits, void* scratch, cudaStream_t st, uint32_t* cell_count, int64_t ncells) {
+                              int key_bits, void* scratch, cudaStream_t st, uint32_t* cell_count, int64_t ncells,
+                              const uint32_t* count) {
     if (n <= 0) return cudaSuccess;
     const SortLayout L = sort_layout(n, key_bits);
     const int rb = L.digit_bits, dig = 1 << rb;
@@ -1003,11 +1008,11 @@ cudaError_t radix_sort_finish(const uint32_t* kin, const uint32_t* vin, uint32_t
         if (rb == 10)
             k_onesweep<10><<<(unsigned)L.tiles, SortShape<10>::kThreads, SortShape<10>::kStagingBytes, st>>>(
                 sk, sv, dk, dv, n, rb * p, hist + dig * p, lp, counters + p, (int*)(counters + 4), cc,
-                (uint32_t)ncells);
+                (uint32_t)ncells, count);
         else
             k_onesweep<8><<<(unsigned)L.tiles, SortShape<8>::kThreads, SortShape<8>::kStagingBytes, st>>>(
                 sk, sv, dk, dv, n, rb * p, hist + dig * p, lp, counters + p, (int*)(counters + 4), cc,
-                (uint32_t)ncells);
+                (uint32_t)ncells, count);
         cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) return e;
         sk = dk;

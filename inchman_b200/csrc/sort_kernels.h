@@ -29,12 +29,14 @@ cudaError_t radix_sort_pairs_u32(const uint32_t* kin, const uint32_t* vin, uint3
 // pass ([passes][1 << digit_bits], radix_sort_hist) while it writes the keys: begin clears the
 // scratch, finish sorts.  With cell_count (zeroed by the caller), the last pass also
 // adds the number of keys equal to each c < ncells into cell_count[c].  vin == nullptr in
-// finish: the values are the keys' indexes.
+// finish: the values are the keys' indexes; count: where the device holds the number of
+// pairs, n being at least that.
 cudaError_t radix_sort_begin(int64_t n, int key_bits, void* scratch, cudaStream_t st);
 uint32_t* radix_sort_hist(int64_t n, int key_bits, void* scratch);
 cudaError_t radix_sort_finish(const uint32_t* kin, const uint32_t* vin, uint32_t* kout, uint32_t* vout, int64_t n,
                               int key_bits, void* scratch, cudaStream_t st, uint32_t* cell_count = nullptr,
-                              int64_t ncells = 0);
+                              int64_t ncells = 0,
+                              const uint32_t* count = nullptr);
 
 // count[c] = number of keys equal to c (keys at or past ncells are not counted)
 cudaError_t cell_counts_u32(const uint32_t* sorted_keys, int64_t n, int64_t ncells, uint32_t* count, cudaStream_t st);

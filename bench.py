@@ -233,7 +233,7 @@ def bench_gray_scott(args, rank, world):
     value = cell_steps * args.steps * world / t_total      # replica_value with the reduced time
     t_launch = sum(per) / len(per)
     # ---- batched: the nine solves of the central finite-difference check (base and
-    # +-h in F, k, Du, Dv), one 16-CTA cluster each in one launch, against the same
+    # +-h in F, k, Du, Dv), a cluster each in one launch, against the same
     # nine solved one after another
     h = 1e-3
     members = [[cfg.F, cfg.k, cfg.Du, cfg.Dv, 0.0, 0.0]]
@@ -398,9 +398,12 @@ def forward_kernel(n):
         c, g = gs.MULTI_CLUSTER[v]
         return {"variant": v, "name": f"k_gs_forward_mc<{n},{c},{g},{(n // c + 2 * g) // 16}>", "clusters": c,
                 "ghost_rows": g, "sms": 16 * c, "rows_per_step": n + 2 * g * c}
-    if v > 10:
+    if 10 < v < 40:
         return {"variant": v, "name": f"k_gs_forward_rr<{n},{v - 10}>", "clusters": 1, "ghost_rows": 0, "sms": 16,
                 "rows_per_step": n}
+    if v == 50:
+        return {"variant": v, "name": "k_gs_forward_tile", "clusters": 1, "ghost_rows": 0,
+                "sms": min(148, ((n + 15) // 16) ** 2), "rows_per_step": n}
     return {"variant": v, "name": "shared-memory column walk", "clusters": 1, "ghost_rows": 0, "sms": 16,
             "rows_per_step": n}
 

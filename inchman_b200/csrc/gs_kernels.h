@@ -10,7 +10,8 @@ struct GSParams {
     double F, k, Du, Dv, vx, vy, dt;
     int cluster;   // CTAs per cluster, 0 = 16 where the lattice fits, else the smallest that fits
     int variant;   // 0 automatic, 1 one cell per iteration, 2 shared-memory column walk,
-                   // 3 register-resident (float32), 10 + w register-resident with w warps per CTA
+                   // 3 register-resident, 10 + w the same with w warps per CTA (float32), 40 + i
+                   // several clusters (float32), 50 tiles over the whole chip
 };
 
 // per-lattice parameters of a batched forward solve
@@ -18,13 +19,13 @@ struct GSBatchMember {
     double F, k, Du, Dv, vx, vy;
 };
 // batch independent float32 n x n lattices (u0/v0/u/v: [batch][n][n]) with their own
-// parameters (p.n, p.steps, p.dt shared), one 16-CTA cluster each, in one launch of
-// the register-resident kernel
+// parameters (p.n, p.steps, p.dt shared) in one launch: a cluster of 1 to 16 CTAs each, by
+// the lattice's side and how many there are
 cudaError_t gs_forward_batch_f32(const GSParams& p, int batch, const GSBatchMember* members, const float* u0,
                                  const float* v0, float* u, float* v, cudaStream_t st);
 
 // how many lattices of side n a batched launch runs at the same time on this device
-// (16-CTA clusters that fit at once)
+// (the most over the cluster shapes)
 cudaError_t gs_batch_capacity(int n, int* clusters);
 // the float32 family variant 0 resolves to for an n x n lattice on the current device
 cudaError_t gs_auto_variant(int n, bool drift, int* variant);

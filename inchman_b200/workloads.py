@@ -209,15 +209,15 @@ def particles(args, rank, world):
     t = a.elapsed_time(b) / 1e3
     x1, _, _ = p.get()
     ps = (n0 + len(x1)) / 2 * args.steps
-    # kernels per step for the 20-bit cell keys: move, two 10-bit onesweep passes (the
-    # last counts the cells), react + compact
-    launches = 4 * args.steps
+    # kernels per step for the 20-bit cell keys: move, two 10-bit onesweep passes, pairs,
+    # compact
+    launches = 5 * args.steps
     # Roofline of the whole step (the kernels run inside one library call): the bytes
-    # that must move at least once per particle -- move 24 (read x, y; write x, y, key,
-    # index), two sort passes 2 x 16 (the cell counts come with the last), react +
-    # compact 4 index + 1 species + 8 position read, 9 written -- plus 12 B per cell
-    # (count written and read, start written)
-    alg = 78.0 * ps / args.steps + 12.0 * G * G
+    # that must move at least once per particle -- move 20 (read x, y; write x, y, key),
+    # two sort passes 12 + 16 (the first makes the index), pairs 4 key + 4 index + 1
+    # species, compact 4 index + 1 species + 8 position read, 9 written -- plus 8 B per
+    # cell (start, count written)
+    alg = 79.0 * ps / args.steps + 8.0 * G * G
     ach = alg / (t / args.steps) / 1e9
     peak, peak_kind = _peaks()
     extra = {"particles_left": len(x1), "dtype": "f32+u32", "gpu_launches": launches,

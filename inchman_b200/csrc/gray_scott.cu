@@ -772,7 +772,7 @@ const void* tile_kernel(int n, bool drift) {
 int tile_count(int n) { return (n + kTileCore - 1) / kTileCore; }
 
 // whether all CTAs of an n x n lattice can be resident at once (cached per device and kernel)
-cudaError_t tile_fits(const void* fn, int n, bool* fits) {
+cudaError_t tile_fits(const void* fn, int n, bool* fits, int times = 1) {
     static std::map<std::pair<int, const void*>, int> cache;
     static std::mutex mu;
     int dev = 0;
@@ -787,7 +787,7 @@ cudaError_t tile_fits(const void* fn, int n, bool* fits) {
         if (e != cudaSuccess) return e;
         most = std::max(1, per_sm * sms);
     }
-    *fits = tile_count(n) * tile_count(n) <= most;
+    *fits = times * tile_count(n) * tile_count(n) <= most;
     return cudaSuccess;
 }
 
@@ -1050,6 +1050,15 @@ cudaError_t gs_adjoint_segment(const GSParams& p, const T* states, int len, cons
     // the packed float32 adjoint also holds two state buffers in shared memory
     const size_t smem = smem_bytes<T>(p.n, cl) * (sizeof(T) == 4 ? 2 : 1);
     if (blk.x != 0 && ak && p.variant != 1) return launch_cluster<T>(ak, p.n, cl, smem, st, args, blk);
+    if ((p.variant == 0 || p.variant == kTileVariant) && p.cluster <= 0 && !gs_own_side(p.n)) {
+        // where its tiles and as many of the segment's recomputation, which runs beside it, fit
+        // on the chip at once: neither then waits for room that the other holds
+        const void* fn = (const void*)k_gs_adjoint_tile<T>;
+        bool fits = false;
+        cudaError_t e = tile_fits(fn, p.n, &fits, 2);
+        if (e != cudaSuccess) return e;
+        if (fits) return tile_run<T>(fn, p.n, len, args, 9, st);
+    }
     return launch_cluster<T>((const void*)k_gs_adjoint<T>, p.n, cl, smem_bytes<T>(p.n, cl), st, args);
 }
 

@@ -388,3 +388,147 @@ __global__ void __launch_bounds__(32 * kTileWarps, sizeof(T) == 4 ? 5 : 2)
         c.store(vo, r, xv[r]);
     }
 }
+
+// Adjoint of a segment on the same tiles, for the sides without a kernel of their own: the
+// adjoint fields take the place of u and v in registers, edges and swaps, and the stored
+// states of a step (the lane's four rows, the row above and the row below) come from L2 a
+// step ahead.  Every cell of the window is updated, the parameter sums count the tile's own.
+// The updates and the sums' terms are k_gs_adjoint's, expression for expression; the sums
+// are in double, so their order over the tiles changes nothing that the result shows.
+// A gradient of 2,000 steps, with k_gs_adjoint -> now: float32 75^2 16.6 -> 5.5 ms, 96^2 5.9 ->
+// 4.8, 192^2 10.0 -> 5.2; float64 24^2 5.15 -> 4.9, 96^2 6.3 -> 5.1, 160^2 9.2 -> 5.6.
+template <typename T>
+__global__ void __launch_bounds__(32 * kTileWarps, sizeof(T) == 4 ? 3 : 2)
+    k_gs_adjoint_tile(GSArgs<T> k, const T* __restrict__ states, int len, const T* __restrict__ lu_in,
+                      const T* __restrict__ lv_in, T* __restrict__ lu_out, T* __restrict__ lv_out,
+                      double* __restrict__ grad, int* __restrict__ err, uint64_t* __restrict__ xbuf, int px, int py) {
+    using P = typename TilePair<T>::type;
+    __shared__ __align__(16) unsigned char s_edges[2 * 2 * 8 * 2 * 16 * sizeof(P)];
+    __shared__ int s_failed;
+    __shared__ double s_red[6][kTileWarps];
+    TileCtx<T> c;
+    c.init(k.n, px, py, s_edges, &s_failed);
+    const size_t nn = (size_t)k.n * k.n;
+    const int above = c.gy[0] == 0 ? k.n - 1 : c.gy[0] - 1, below = c.gy[3] == k.n - 1 ? 0 : c.gy[3] + 1;
+    const auto row = [&](const T* p, int y) {
+        const T* q = p + (size_t)y * k.n;
+        if (c.pair) return *reinterpret_cast<const P*>(q + c.gx[0]);
+        P v;
+        v.x = q[c.gx[0]];
+        v.y = q[c.gx[1]];
+        return v;
+    };
+    P nu[6], nv[6];                // the next step's states: rows above, the four, below
+    const auto fetch = [&](int j) {
+        if (j < 0) return;
+        const T* us = states + (size_t)(2 * j) * nn;
+        const T* vs = us + nn;
+        nu[0] = row(us, above);
+        nv[0] = row(vs, above);
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+            nu[r + 1] = c.load(us, r);
+            nv[r + 1] = c.load(vs, r);
+        }
+        nu[5] = row(us, below);
+        nv[5] = row(vs, below);
+    };
+    double gF = 0, gk = 0, gDu = 0, gDv = 0, gvx = 0, gvy = 0;
+    const T two = T(2), half = T(0.5), four = T(4);
+    const T Fk = k.F + k.k;
+    const auto cell = [&](bool own, T uU, T uc, T uD, T uL, T uR, T vU, T vc, T vD, T vL, T vR, T aU, T ac, T aD, T aL,
+                          T aR, T bU, T bc, T bD, T bL, T bR, T* an, T* bn) {
+        const T lap_a = aL + aR + aU + aD - four * ac;
+        const T lap_b = bL + bR + bU + bD - four * bc;
+        const T dxa = (aR - aL) * half, dya = (aD - aU) * half;
+        const T dxb = (bR - bL) * half, dyb = (bD - bU) * half;
+        const T v2 = vc * vc, uv = uc * vc;
+        *an = ac + k.dt * (k.Du * lap_a + k.vx * dxa + k.vy * dya + ac * (-v2 - k.F) + bc * v2);
+        *bn = bc + k.dt * (k.Dv * lap_b + k.vx * dxb + k.vy * dyb + ac * (-two * uv) + bc * (two * uv - Fk));
+        if (own) {
+            const double lu = (double)(uL + uR + uU + uD - four * uc);
+            const double lv = (double)(vL + vR + vU + vD - four * vc);
+            gF += (double)ac * (1.0 - (double)uc) - (double)bc * (double)vc;
+            gk += -(double)bc * (double)vc;
+            gDu += (double)ac * lu;
+            gDv += (double)bc * lv;
+            gvx += -(double)ac * (double)((uR - uL) * half) - (double)bc * (double)((vR - vL) * half);
+            gvy += -(double)ac * (double)((uD - uU) * half) - (double)bc * (double)((vD - vU) * half);
+        }
+    };
+    const auto step = [&](int par, int j, const P (&xa)[4], const P (&xb)[4], P (&ya)[4], P (&yb)[4]) {
+        P su[6], sv[6];
+#pragma unroll
+        for (int r = 0; r < 6; ++r) {
+            su[r] = nu[r];
+            sv[r] = nv[r];
+        }
+        fetch(j - 1);
+        const int up = (c.group + 7) & 7, dn = (c.group + 1) & 7;     // the outermost rows are stale anyway
+        const P ta = *c.edge(par, 0, up, 1), tb = *c.edge(par, 1, up, 1);
+        const P ba = *c.edge(par, 0, dn, 0), bb = *c.edge(par, 1, dn, 0);
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+            const auto left = [](T v) { return __shfl_up_sync(0xffffffffu, v, 1, 16); };
+            const auto right = [](T v) { return __shfl_down_sync(0xffffffffu, v, 1, 16); };
+            const P aU = r == 0 ? ta : xa[r == 0 ? 0 : r - 1], aD = r == 3 ? ba : xa[r == 3 ? 3 : r + 1];
+            const P bU = r == 0 ? tb : xb[r == 0 ? 0 : r - 1], bD = r == 3 ? bb : xb[r == 3 ? 3 : r + 1];
+            const P u = su[r + 1], v = sv[r + 1];
+            const T al = left(xa[r].y), ar = right(xa[r].x), bl = left(xb[r].y), br = right(xb[r].x);
+            const T ul = left(u.y), ur = right(u.x), vl = left(v.y), vr = right(v.x);
+            cell(c.cy[r] && c.cx[0], su[r].x, u.x, su[r + 2].x, ul, u.y, sv[r].x, v.x, sv[r + 2].x, vl, v.y, aU.x, xa[r].x,
+                 aD.x, al, xa[r].y, bU.x, xb[r].x, bD.x, bl, xb[r].y, &ya[r].x, &yb[r].x);
+            cell(c.cy[r] && c.cx[1], su[r].y, u.y, su[r + 2].y, u.x, ur, sv[r].y, v.y, sv[r + 2].y, v.x, vr, aU.y, xa[r].y,
+                 aD.y, xa[r].x, ar, bU.y, xb[r].y, bD.y, xb[r].x, br, &ya[r].y, &yb[r].y);
+        }
+    };
+    P xa[4], xb[4], ya[4], yb[4];
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+        xa[r] = c.load(lu_in, r);
+        xb[r] = c.load(lv_in, r);
+    }
+    fetch(len - 1);
+    c.put_edges(0, xa, xb);
+    int s = 0;
+    for (; s + 2 <= len; s += 2) {
+        step(0, len - 1 - s, xa, xb, ya, yb);
+        c.put_edges(1, ya, yb);
+        step(1, len - 2 - s, ya, yb, xa, xb);
+        if ((s + 2) % kTileGhost == 0 && s + 2 < len) c.swap(xbuf, (s + 2) / kTileGhost, xa, xb);
+        c.put_edges(0, xa, xb);
+    }
+    if (s < len) {
+        step(0, len - 1 - s, xa, xb, ya, yb);
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+            xa[r] = ya[r];
+            xb[r] = yb[r];
+        }
+    }
+    double g[6] = {gF, gk, gDu, gDv, gvx, gvy};
+    const double dtd = (double)k.dt;
+#pragma unroll
+    for (int q = 0; q < 6; ++q) {
+        double v = g[q] * dtd;
+        for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+        if (c.lane == 0) s_red[q][threadIdx.x >> 5] = v;
+    }
+    __syncthreads();
+    if (s_failed) {
+        if (threadIdx.x == 0) atomicOr(err, 1);
+        const T nan = (T)__int_as_float(0x7fc00000);
+#pragma unroll
+        for (int r = 0; r < 4; ++r) xa[r].x = xa[r].y = xb[r].x = xb[r].y = nan;
+    }
+    if (threadIdx.x < 6) {
+        double v = 0;
+        for (int w = 0; w < kTileWarps; ++w) v += s_red[threadIdx.x][w];
+        atomicAdd(&grad[threadIdx.x], v);
+    }
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+        c.store(lu_out, r, xa[r]);
+        c.store(lv_out, r, xb[r]);
+    }
+}

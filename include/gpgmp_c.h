@@ -218,6 +218,7 @@ int gpgmp_timesteps(gpgmp_solver* h, float* dt_x, float* dt_y);
 /* Launch shapes of the stochastic kernels (the reference fixes its work-group shape,
  * Globals.h:24-28, Solver.cpp:30-33): the diffusion kernels' tile of tile_w x tile_h
  * cells (256 threads) and the SSA kernel's block of ssa_threads threads, one cell each.
+ * (The drift-diffusion sweeps have one shape.)
  * Every draw is keyed by its cell, so the results do not depend on the shape.
  *  gpgmp_solver_launch_choices: the shapes there are (arrays of at least 8 entries,
  *                               any may be NULL);
@@ -290,8 +291,10 @@ typedef struct gpgmp_gs_params {
                                    adjoint runs the multi-cluster adjoint under 40 + i (the same
                                    lambda bits); under 0, where the forward is multi-cluster, it
                                    recomputes the segments on two clusters (40) and runs the
-                                   four-cluster adjoint beside it.  The batched forward treats
-                                   40 + i as 0. */
+                                   four-cluster adjoint beside it.  On sides other than 64, 128,
+                                   256, 512 it runs on tiles under 0 and 50 (cluster = 0) where
+                                   they fit twice (the same lambda bits in float32).  The batched
+                                   forward treats 40 + i as 0. */
 } gpgmp_gs_params;
 
 /* bytes of the checkpoint buffer and of the adjoint's work buffer */

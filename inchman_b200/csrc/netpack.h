@@ -9,8 +9,8 @@ namespace gpgmp {
 
 // False where a reaction does not fit the packed form: more than two reactant molecules, a
 // species named twice among the reactants (its hazard is then A * A, and counts may turn
-// negative), a stoichiometry outside 0..256 (the changes are kept as the upper half of a
-// float, exact up to 256) or more than four changed species, a negative or non-finite rate
+// negative), a stoichiometry outside 0..kPackedChange (the changes are kept as the upper half
+// of a float, exact up to 256) or more than four changed species, a negative or non-finite rate
 // (the running sums must not fall).  *nnet: the most species that one reaction changes.
 inline bool pack_network(const gpgmp_reaction* r, int R, int S, PackedReaction* out, int* nnet) {
     *nnet = 1;
@@ -35,13 +35,13 @@ inline bool pack_network(const gpgmp_reaction* r, int R, int S, PackedReaction* 
             change[sp] -= st;
         }
         for (int j = 0; j < a.num_products; ++j) {
-            if (a.product_stoich[j] < 0 || a.product_stoich[j] > 256) return false;
+            if (a.product_stoich[j] < 0 || a.product_stoich[j] > kPackedChange) return false;
             change[a.product_species[j]] += a.product_stoich[j];
         }
         int n = 0;
         for (int s = 0; s < S; ++s) {
             if (change[s] == 0) continue;
-            if (n == 4 || change[s] > 256) return false;
+            if (n == 4 || change[s] > kPackedChange) return false;
             const float f = (float)change[s];
             uint32_t bits;
             std::memcpy(&bits, &f, 4);

@@ -175,7 +175,7 @@ __device__ __forceinline__ int ssa_cell_inc(const gpgmp_reaction* rt, const uint
 // ---- packed networks -------------------------------------------------------------
 // A network whose reactions have at most two reactant molecules and change at most four
 // species (pack_network, netpack.h) runs its windows on float copies of the counts, which
-// are exact below 2^24.  Every hazard then is the same three operations, rate * x[s1] *
+// are exact up to 2^24.  Every hazard then is the same three operations, rate * x[s1] *
 // (x[s2] - sub): an absent reactant is slot 0, which holds 1 (the
 // products by 1 and the difference of 0 are exact; species s is slot s + 1), and 2A has s2 = s1, sub = 1, so the
 // values and their running sums are those of ssa_cell bit for bit.  No table of the
@@ -183,14 +183,16 @@ __device__ __forceinline__ int ssa_cell_inc(const gpgmp_reaction* rt, const uint
 // selection instead of formed twice: A + B <-> C on 1M cells, a window of 1.7 events per
 // cell, 47 us instead of 78; predator and prey on 8.4M cells, 112 us instead of 171; 592
 // random networks of 8 to 32 reactions, 75 ms instead of 238.
-// A cell whose counts are negative or reach 2^24 goes on in ssa_slow, which keeps the
-// counts as integers in the same slots.
+// A cell whose counts are negative or reach kPackedMax goes on in ssa_slow, which keeps the
+// counts as integers in the same slots.  The limit is the largest change of a packed
+// reaction below 2^24, so that the sum that passes it is still exact.
 struct PackedReaction {
     float rate, sub;
     int32_t s1, s2;      // slots of the reactants
     uint32_t net[4];     // slot << 16 | upper half of the float change; unused: 0
 };
-constexpr float kPackedMax = 16777216.0f;
+constexpr int kPackedChange = 256;      // pack_network's largest change of a count
+constexpr int kPackedMax = (1 << 24) - kPackedChange;
 
 // Where a window stands: time, events, the last draws and how many of them are used.
 struct SsaPos {
@@ -209,7 +211,7 @@ __device__ __forceinline__ float ssa_wait(uint32_t draw, float h0) {
     return h0 > 8.6736174e-19f && h0 < 1.1529215e18f ? div_mid(l, h0) : l / h0;
 }
 
-// applies one event's changes; true while every changed count stays below 2^24
+// applies one event's changes; true while every changed count stays below kPackedMax
 template <int STRIDE>
 __device__ __forceinline__ bool packed_apply(const uint4& n, int nnet, float* x) {
     const uint32_t e[4] = {n.x, n.y, n.z, n.w};
@@ -223,7 +225,7 @@ __device__ __forceinline__ bool packed_apply(const uint4& n, int nnet, float* x)
             top = fmaxf(top, v);
         }
     }
-    return top < kPackedMax;
+    return top < (float)kPackedMax;
 }
 
 // One window of a network of NR reactions given by value (kernel parameters): the running
@@ -317,13 +319,13 @@ __device__ __forceinline__ void packed_tables(const PackedReaction* __restrict__
 }
 
 // The counts of one cell from memory (at(s): species s) into the float slots; false where
-// a count is outside the floats' exact range (the slots then hold the integers' bits).
+// a count is negative or at least kPackedMax (the slots then hold the integers' bits).
 template <int STRIDE, class AT>
 __device__ __forceinline__ bool packed_load(const AT& at, int S, float* x) {
     bool fits = true;
     for (int s = 0; s < S; ++s) {
         const int v = at(s);
-        fits = fits && (uint32_t)v < (1u << 24);
+        fits = fits && (uint32_t)v < (uint32_t)kPackedMax;
         x[(s + 1) * STRIDE] = (float)v;
     }
     if (!fits)

@@ -22,6 +22,7 @@
 #include <cooperative_groups.h>
 #include <cstdint>
 #include <cstdio>
+#include <initializer_list>
 #include <map>
 #include <mutex>
 #include <type_traits>
@@ -791,10 +792,20 @@ cudaError_t tile_fits(const void* fn, int n, bool* fits, int times = 1) {
     return cudaSuccess;
 }
 
+// whether every array (null ones aside) begins on a multiple of `bytes`: the caller's may be
+// views that begin anywhere in a buffer
+bool aligned(std::initializer_list<const void*> arrays, size_t bytes) {
+    uintptr_t all = 0;
+    for (const void* p : arrays) all |= (uintptr_t)p;
+    return all % bytes == 0;
+}
+
 // one tiled launch: the exchange buffer from the stream-ordered pool (private to the launch),
-// cleared on the stream, then the kernel with `args` and the buffer and tile counts
+// cleared on the stream, then the kernel with `args` and the buffer, tile counts and whether
+// the columns go in pairs (even sides, arrays aligned to a pair)
 template <typename T>
-cudaError_t tile_run(const void* fn, int n, int steps, void** args, int nargs, cudaStream_t st) {
+cudaError_t tile_run(const void* fn, int n, int steps, std::initializer_list<const void*> arrays, void** args, int nargs,
+                     cudaStream_t st) {
     const size_t bytes = steps > kTileGhost ? (size_t)n * n * 2 * 2 * sizeof(uint64_t) * (sizeof(T) / 4) : 0;
     uint64_t* xb = nullptr;
     cudaError_t e = cudaSuccess;
@@ -804,12 +815,13 @@ cudaError_t tile_run(const void* fn, int n, int steps, void** args, int nargs, c
         e = cudaMemsetAsync(xb, 0, bytes, st);
     }
     if (e == cudaSuccess) {
-        int tiles = tile_count(n);
+        int tiles = tile_count(n), pairs = n % 2 == 0 && aligned(arrays, 2 * sizeof(T));
         void* all[16];
         for (int q = 0; q < nargs; ++q) all[q] = args[q];
         all[nargs] = &xb;
         all[nargs + 1] = &tiles;
         all[nargs + 2] = &tiles;
+        all[nargs + 3] = &pairs;
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3(tiles * tiles, 1, 1);
         cfg.blockDim = dim3(32 * kTileWarps, 1, 1);
@@ -960,7 +972,7 @@ cudaError_t gs_forward(const GSParams& p, const T* u0, const T* v0, T* u, T* v, 
         bool fits = false;
         cudaError_t e = tile_fits(fn, p.n, &fits);
         if (e != cudaSuccess) return e;
-        if (fits) return tile_run<T>(fn, p.n, p.steps, args, 7, st);
+        if (fits) return tile_run<T>(fn, p.n, p.steps, {u0, v0, u, v, trace}, args, 7, st);
         if (p.variant != 0) return cudaErrorInvalidConfiguration;
     }
     if constexpr (std::is_same<T, float>::value) {
@@ -991,7 +1003,8 @@ cudaError_t gs_forward(const GSParams& p, const T* u0, const T* v0, T* u, T* v, 
         if (p.variant != 0) return cudaErrorInvalidValue;
     }
     if constexpr (std::is_same<T, double>::value) {
-        if (cl == kRRCluster && p.variant == 0) {
+        // (pairs of doubles; an array that begins between them takes the column walk below)
+        if (cl == kRRCluster && p.variant == 0 && aligned({u0, v0, u, v, trace}, 16)) {
             size_t smem = 0;
             int wpc = 0;
             const void* rk = rr_kernel_f64(p.n, false, p.vx != 0.0 || p.vy != 0.0, &wpc, &smem);
@@ -1038,7 +1051,7 @@ cudaError_t gs_adjoint_segment(const GSParams& p, const T* states, int len, cons
         if (variant != 0) return cudaErrorInvalidValue;
     }
     if constexpr (std::is_same<T, double>::value) {
-        if (cl == kRRCluster && p.variant == 0) {
+        if (cl == kRRCluster && p.variant == 0 && aligned({states, lu_in, lv_in, lu_out, lv_out}, 16)) {
             size_t smem = 0;
             int wpc = 0;
             const void* rk = rr_kernel_f64(p.n, true, p.vx != 0.0 || p.vy != 0.0, &wpc, &smem);
@@ -1057,7 +1070,7 @@ cudaError_t gs_adjoint_segment(const GSParams& p, const T* states, int len, cons
         bool fits = false;
         cudaError_t e = tile_fits(fn, p.n, &fits, 2);
         if (e != cudaSuccess) return e;
-        if (fits) return tile_run<T>(fn, p.n, len, args, 9, st);
+        if (fits) return tile_run<T>(fn, p.n, len, {states, lu_in, lv_in, lu_out, lv_out}, args, 9, st);
     }
     return launch_cluster<T>((const void*)k_gs_adjoint<T>, p.n, cl, smem_bytes<T>(p.n, cl), st, args);
 }

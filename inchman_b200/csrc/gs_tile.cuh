@@ -13,7 +13,8 @@
 //
 // A lane owns two adjacent columns of four rows (16 lanes a row, two row groups a warp):
 // vertical neighbours inside the group are its own registers, the rows above and below come
-// from shared memory, horizontal neighbours by shuffles inside the 16 lanes.
+// from shared memory, horizontal neighbours by shuffles inside the 16 lanes.  On even sides
+// the two columns are one access where the caller's arrays are aligned for it.
 //
 // Swap: at every state 8 m each CTA writes its tile's values, packed with m into 64-bit words
 // (a double as two words with half its bits each), to the exchange buffer and polls its
@@ -115,13 +116,13 @@ struct TileCtx {
     int gx[2], gy[4];            // lattice columns and rows of the lane's cells (periodic)
     bool cx[2], cy[4];           // whether they belong to the tile
     bool ex[2], ey[4];           // whether they are within 8 cells of it
-    bool pair;                   // the two columns are an aligned pair in memory
+    bool pair;                   // the two columns are an aligned pair in every array (the host's `pairs`)
     P* edges;                    // [parity][field][group][top / bottom][16 lanes]
     volatile int* failed;
     __device__ __forceinline__ P* edge(int par, int f, int g, int bottom) const {
         return edges + ((((par * 2 + f) * 8 + g) * 2 + bottom) * 16) + (lane & 15);
     }
-    __device__ __forceinline__ void init(int side, int px, int py, unsigned char* smem, volatile int* fail) {
+    __device__ __forceinline__ void init(int side, int px, int py, int pairs, unsigned char* smem, volatile int* fail) {
         n = side;
         lane = threadIdx.x & 31;
         group = (int)(threadIdx.x >> 5) * 2 + (lane >> 4);
@@ -142,7 +143,7 @@ struct TileCtx {
             cy[r] = e >= kTileGhost && e < kTileGhost + ch;
             ey[r] = e < ch + 2 * kTileGhost;
         }
-        pair = n % 2 == 0;
+        pair = pairs != 0;
         edges = reinterpret_cast<P*>(smem);
         failed = fail;
         if (threadIdx.x == 0) *failed = 0;
@@ -324,12 +325,12 @@ template <typename T, int DRIFT, int FORM>
 __global__ void __launch_bounds__(32 * kTileWarps, sizeof(T) == 4 ? 5 : 2)
     k_gs_forward_tile(GSArgs<T> a, const T* __restrict__ u0, const T* __restrict__ v0, T* __restrict__ uo,
                       T* __restrict__ vo, T* __restrict__ trace, int trace_every, uint64_t* __restrict__ xbuf, int px,
-                      int py) {
+                      int py, int pairs) {
     using P = typename TilePair<T>::type;
     __shared__ __align__(16) unsigned char s_edges[2 * 2 * 8 * 2 * 16 * sizeof(P)];
     __shared__ int s_failed;
     TileCtx<T> c;
-    c.init(a.n, px, py, s_edges, &s_failed);
+    c.init(a.n, px, py, pairs, s_edges, &s_failed);
     const TileCoef<T, FORM> k(a);
     const size_t nn = (size_t)a.n * a.n;
     P xu[4], xv[4], yu[4], yv[4];
@@ -401,13 +402,14 @@ template <typename T>
 __global__ void __launch_bounds__(32 * kTileWarps, sizeof(T) == 4 ? 3 : 2)
     k_gs_adjoint_tile(GSArgs<T> k, const T* __restrict__ states, int len, const T* __restrict__ lu_in,
                       const T* __restrict__ lv_in, T* __restrict__ lu_out, T* __restrict__ lv_out,
-                      double* __restrict__ grad, int* __restrict__ err, uint64_t* __restrict__ xbuf, int px, int py) {
+                      double* __restrict__ grad, int* __restrict__ err, uint64_t* __restrict__ xbuf, int px, int py,
+                      int pairs) {
     using P = typename TilePair<T>::type;
     __shared__ __align__(16) unsigned char s_edges[2 * 2 * 8 * 2 * 16 * sizeof(P)];
     __shared__ int s_failed;
     __shared__ double s_red[6][kTileWarps];
     TileCtx<T> c;
-    c.init(k.n, px, py, s_edges, &s_failed);
+    c.init(k.n, px, py, pairs, s_edges, &s_failed);
     const size_t nn = (size_t)k.n * k.n;
     const int above = c.gy[0] == 0 ? k.n - 1 : c.gy[0] - 1, below = c.gy[3] == k.n - 1 ? 0 : c.gy[3] + 1;
     const auto row = [&](const T* p, int y) {

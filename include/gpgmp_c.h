@@ -265,7 +265,11 @@ int gpgmp_set_individual_properties(gpgmp_solver* h, int32_t species, const floa
  * Deterministic.cl:71-136).  The reference has no adjoint; gpgmp_gs_adjoint_* is the
  * hand-written discrete adjoint of the same steps.
  * Device pointers; u and v are n*n row-major arrays.  Checkpoint buffers hold
- * ceil(steps / checkpoint_every) states, each u then v. */
+ * ceil(steps / checkpoint_every) states, each u then v.  Arrays may begin at any element (a
+ * view into a larger buffer; where the elements of a pair are not aligned together the solve
+ * loads them one by one), except for float32 on sides 64, 128, 256 and 512 outside families 1
+ * and 50: there u0, v0, u, v, checkpoints, grad_u0, grad_v0 and work begin on 16 bytes, as
+ * allocations do. */
 typedef struct gpgmp_gs_params {
     int32_t n;                  /* lattice side; a multiple of the cluster size */
     int32_t steps;

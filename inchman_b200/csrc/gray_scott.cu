@@ -800,6 +800,26 @@ bool aligned(std::initializer_list<const void*> arrays, size_t bytes) {
     return all % bytes == 0;
 }
 
+// Whether a tiled solve may read (u0, v0) and write (u, v, trace).  A tile stores its result
+// without waiting for the tiles that load the cells around it, unless they have swapped in
+// between (steps > kTileGhost: a swap's words come from CTAs that have loaded); so a
+// solve in place needs a swap, and any other overlap a cluster kernel, which loads the whole
+// lattice before it stores.
+template <typename T>
+bool tile_apart(int n, int steps, const T* u0, const T* v0, const T* u, const T* v, const T* trace, int every) {
+    const uintptr_t plane = (uintptr_t)n * n * sizeof(T);
+    const auto apart = [&](const T* in, const T* out, uintptr_t bytes) {
+        const uintptr_t a = (uintptr_t)in, b = (uintptr_t)out;
+        return a + plane <= b || b + bytes <= a;
+    };
+    for (const T* in : {u0, v0}) {
+        for (const T* out : {u, v})
+            if (!apart(in, out, plane) && !(in == out && steps > kTileGhost)) return false;
+        if (trace && !apart(in, trace, 2 * plane * (uintptr_t)((steps + every - 1) / every))) return false;
+    }
+    return true;
+}
+
 // one tiled launch: the exchange buffer from the stream-ordered pool (private to the launch),
 // cleared on the stream, then the kernel with `args` and the buffer, tile counts and whether
 // the columns go in pairs (even sides, arrays aligned to a pair)
@@ -967,7 +987,8 @@ cudaError_t gs_forward(const GSParams& p, const T* u0, const T* v0, T* u, T* v, 
     GSArgs<T> a{p.n, p.steps, (T)p.F, (T)p.k, (T)p.Du, (T)p.Dv, (T)p.vx, (T)p.vy, (T)p.dt};
     int every = trace_every > 0 ? trace_every : 1;
     void* args[] = {&a, (void*)&u0, (void*)&v0, &u, &v, &trace, &every};
-    if (p.variant == kTileVariant || (p.variant == 0 && p.cluster <= 0 && tile_side(p.n, (int)sizeof(T)))) {
+    if ((p.variant == kTileVariant || (p.variant == 0 && p.cluster <= 0 && tile_side(p.n, (int)sizeof(T)))) &&
+        tile_apart(p.n, p.steps, u0, v0, u, v, trace, every)) {
         const void* fn = tile_kernel<T>(p.n, p.vx != 0.0 || p.vy != 0.0);
         bool fits = false;
         cudaError_t e = tile_fits(fn, p.n, &fits);

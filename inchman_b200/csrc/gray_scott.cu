@@ -640,6 +640,26 @@ void rb_launch_config(const RBConfig& m, int batch, cudaLaunchConfig_t* cfg, cud
     cfg->numAttrs = 1;
 }
 
+// Whether a solve on CTAs or clusters that swap cells every `ghost` steps may read (u0, v0) and
+// write (u, v, trace).  Such a part stores its result without waiting for the parts that
+// load the cells around it, unless they have swapped in between (steps > ghost: a swap's
+// words come from CTAs that have loaded); so a solve in place needs a swap, and any other
+// overlap a kernel on one cluster, which loads the whole lattice before it stores.
+template <typename T>
+bool swaps_apart(int n, int steps, int ghost, const T* u0, const T* v0, const T* u, const T* v, const T* trace, int every) {
+    const uintptr_t plane = (uintptr_t)n * n * sizeof(T);
+    const auto apart = [&](const T* in, const T* out, uintptr_t bytes) {
+        const uintptr_t a = (uintptr_t)in, b = (uintptr_t)out;
+        return a + plane <= b || b + bytes <= a;
+    };
+    for (const T* in : {u0, v0}) {
+        for (const T* out : {u, v})
+            if (!apart(in, out, plane) && !(in == out && steps > ghost)) return false;
+        if (trace && !apart(in, trace, 2 * plane * (uintptr_t)((steps + every - 1) / every))) return false;
+    }
+    return true;
+}
+
 // Multi-cluster forward kernels (gs_mc.cuh): variant 40 + index.  Each spreads one
 // lattice over `clusters` 16-CTA clusters with `ghost` ghost rows per band side.
 struct MCConfig {
@@ -798,26 +818,6 @@ bool aligned(std::initializer_list<const void*> arrays, size_t bytes) {
     uintptr_t all = 0;
     for (const void* p : arrays) all |= (uintptr_t)p;
     return all % bytes == 0;
-}
-
-// Whether a tiled solve may read (u0, v0) and write (u, v, trace).  A tile stores its result
-// without waiting for the tiles that load the cells around it, unless they have swapped in
-// between (steps > kTileGhost: a swap's words come from CTAs that have loaded); so a
-// solve in place needs a swap, and any other overlap a cluster kernel, which loads the whole
-// lattice before it stores.
-template <typename T>
-bool tile_apart(int n, int steps, const T* u0, const T* v0, const T* u, const T* v, const T* trace, int every) {
-    const uintptr_t plane = (uintptr_t)n * n * sizeof(T);
-    const auto apart = [&](const T* in, const T* out, uintptr_t bytes) {
-        const uintptr_t a = (uintptr_t)in, b = (uintptr_t)out;
-        return a + plane <= b || b + bytes <= a;
-    };
-    for (const T* in : {u0, v0}) {
-        for (const T* out : {u, v})
-            if (!apart(in, out, plane) && !(in == out && steps > kTileGhost)) return false;
-        if (trace && !apart(in, trace, 2 * plane * (uintptr_t)((steps + every - 1) / every))) return false;
-    }
-    return true;
 }
 
 // one tiled launch: the exchange buffer from the stream-ordered pool (private to the launch),
@@ -988,7 +988,7 @@ cudaError_t gs_forward(const GSParams& p, const T* u0, const T* v0, T* u, T* v, 
     int every = trace_every > 0 ? trace_every : 1;
     void* args[] = {&a, (void*)&u0, (void*)&v0, &u, &v, &trace, &every};
     if ((p.variant == kTileVariant || (p.variant == 0 && p.cluster <= 0 && tile_side(p.n, (int)sizeof(T)))) &&
-        tile_apart(p.n, p.steps, u0, v0, u, v, trace, every)) {
+        swaps_apart(p.n, p.steps, kTileGhost, u0, v0, u, v, trace, every)) {
         const void* fn = tile_kernel<T>(p.n, p.vx != 0.0 || p.vy != 0.0);
         bool fits = false;
         cudaError_t e = tile_fits(fn, p.n, &fits);
@@ -996,8 +996,10 @@ cudaError_t gs_forward(const GSParams& p, const T* u0, const T* v0, T* u, T* v, 
         if (fits) return tile_run<T>(fn, p.n, p.steps, {u0, v0, u, v, trace}, args, 7, st);
         if (p.variant != 0) return cudaErrorInvalidConfiguration;
     }
+    bool one_cluster = false;      // a multi-cluster choice whose arrays overlap
     if constexpr (std::is_same<T, float>::value) {
         const bool drift = p.vx != 0.0 || p.vy != 0.0;
+        const auto apart = [&](int i) { return swaps_apart(p.n, p.steps, mc_table(i).ghost, u0, v0, u, v, trace, every); };
         if (p.variant >= kMCVariant && p.variant < kMCVariant + kMCConfigs) {
             const int i = p.variant - kMCVariant;
             bool fits = false;
@@ -1005,23 +1007,25 @@ cudaError_t gs_forward(const GSParams& p, const T* u0, const T* v0, T* u, T* v, 
             cudaError_t e = mc_fits(i, drift, &fits);
             if (e != cudaSuccess) return e;
             if (!fits) return cudaErrorInvalidConfiguration;
-            return mc_forward(i, a, drift, u0, v0, u, v, trace, every, st);
+            if (apart(i)) return mc_forward(i, a, drift, u0, v0, u, v, trace, every, st);
+            one_cluster = true;
         }
         if (p.variant == 0 && cl == kRRCluster && p.n == mc_table(kMCDefault).n) {
             bool fits = false;
             cudaError_t e = mc_fits(kMCDefault, drift, &fits);
             if (e != cudaSuccess) return e;
-            if (fits) return mc_forward(kMCDefault, a, drift, u0, v0, u, v, trace, every, st);
+            if (fits && apart(kMCDefault)) return mc_forward(kMCDefault, a, drift, u0, v0, u, v, trace, every, st);
         }
     }
-    if (sizeof(T) == 4 && cl == kRRCluster && (p.variant == 0 || p.variant == 3 || (p.variant > 10 && p.variant < kMCVariant))) {
+    const int variant = one_cluster ? 0 : p.variant;
+    if (sizeof(T) == 4 && cl == kRRCluster && (variant == 0 || variant == 3 || (variant > 10 && variant < kMCVariant))) {
         size_t smem = 0;
-        int wpc = p.variant > 10 ? p.variant - 10 : 0;
+        int wpc = variant > 10 ? variant - 10 : 0;
         const void* rk = rr_kernel(p.n, &wpc, p.vx != 0.0 || p.vy != 0.0, &smem);
         const GSArgs<float>* no_batch = nullptr;
         void* rargs[] = {&a, (void*)&u0, (void*)&v0, &u, &v, &trace, &every, &no_batch};
         if (rk) return launch_cluster<T>(rk, p.n, cl, smem, st, rargs, dim3(32 * wpc, 1, 1));
-        if (p.variant != 0) return cudaErrorInvalidValue;
+        if (variant != 0) return cudaErrorInvalidValue;
     }
     if constexpr (std::is_same<T, double>::value) {
         // (pairs of doubles; an array that begins between them takes the column walk below)

@@ -288,9 +288,10 @@ typedef struct gpgmp_gs_params {
                                    i = 0 (2, 8), 1 (4, 8), 2 (4, 16), 3 (8, 8), 4 (8, 16),
                                    5 (4, 32), 6 (2, 32), a CUDA error where the device cannot hold
                                    all its clusters at once; 50 tiled, any n, a CUDA error where
-                                   the device cannot hold all its tiles at once (a solve whose
-                                   outputs overlap its inputs in part, or in place with at
-                                   most 8 steps, runs on one cluster under 0 and 50).  Every float32
+                                   the device cannot hold all its tiles at once.  (Under 0,
+                                   40 + i and 50 a solve whose outputs overlap its inputs in
+                                   part, or in place with no more steps than ghost cells,
+                                   runs on one cluster.)  Every float32
                                    family gives the same bits (on sides other than 64, 128, 256,
                                    512 those of 1).  float64: 0 register-resident at n 64 and 128
                                    on a 16-CTA cluster, else 50 as above; 1; 2; 50.  The

@@ -53,3 +53,22 @@ def test_outputs_on_inputs(gpgmp, dtype, n, steps):
     _forward(dtype, p, ck[0, 0], ck[0, 1], u, v, ck)
     check(u, v)
     assert torch.equal(ck[0, 0], a) and torch.equal(ck[0, 1], b)
+
+
+@pytest.mark.parametrize("variant,steps", [(0, 1), (0, 8), (0, 9), (0, 40), (42, 16), (42, 17), (40, 3)])
+def test_several_clusters(gpgmp, variant, steps):
+    """The multi-cluster families at n = 256 (8 or 16 ghost rows)."""
+    import torch
+    from inchman_b200 import gray_scott as gs
+    cfg = gs.GrayScottConfig(n=256, steps=steps)
+    a, b = (torch.from_numpy(x).cuda() for x in cfg.initial_state(np.float32))
+    p = cfg.params(variant=variant)
+    want = gs.forward(a, b, p)
+    u, v = a.clone(), b.clone()
+    _forward(np.float32, p, u, v, u, v)
+    assert gs.status() == 0 and torch.equal(u, want[0]) and torch.equal(v, want[1])
+    buf = torch.cat([a.flatten(), b.flatten(), a.flatten()])
+    u0, v0, u = buf[:65536], buf[65536:131072], buf[65536 + 4096:131072 + 4096]
+    v = torch.empty_like(b)
+    _forward(np.float32, p, u0, v0, u, v)
+    assert gs.status() == 0 and torch.equal(u.view(256, 256), want[0]) and torch.equal(v, want[1])

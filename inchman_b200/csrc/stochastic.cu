@@ -5,6 +5,7 @@
 // Compiled with -fmad=false: the sampling code must round exactly as its CPU
 // replay does.
 #include <cstdio>
+#include <utility>
 #include "kernels.h"
 #include "stoch_device.cuh"
 
@@ -217,13 +218,14 @@ __global__ void __launch_bounds__(NT) k_diffuse_tile(const int* __restrict__ in,
 // and one barrier serves all the realisations.  Issue slots bound it (the random block and
 // the two searches), not its 8 bytes per cell:
 // 8.4M cells 140 us (67 MB; 198 us with one realisation and one set-up per cell and tile,
-// whose quarter-tile of halo rows was sampled again).
+// whose quarter-tile of halo rows was sampled again).  tall: the grid's first dimension, which
+// alone may exceed 65535, counts the rows of tiles instead of the columns.
 constexpr int kSweepReal = 8;
 template <int DIR>
 __global__ void __launch_bounds__(NT, 4) k_sweep(const int* __restrict__ in, int* __restrict__ out, int W, int H, int S,
                                               int R, int species, uint32_t seed, uint32_t step_seed, int wall_lo,
                                               int wall_hi, const float* __restrict__ Df, const float* __restrict__ rf,
-                                              float dt, float dx, int fpe) {
+                                              float dt, float dx, int fpe, int tall) {
     constexpr int TW = DIR == 0 ? 32 : 8, TH = DIR == 0 ? 8 : 32;
     constexpr int LINE = 34;                       // cells along the sweep with both halo cells
     constexpr int STEP = DIR == 0 ? 1 : TW;        // to the next cell along the sweep
@@ -233,7 +235,7 @@ __global__ void __launch_bounds__(NT, 4) k_sweep(const int* __restrict__ in, int
     const int64_t area = (int64_t)W * H;
     const int r0 = blockIdx.z * kSweepReal;
     const int nr = min(kSweepReal, R - r0);
-    const int x0 = blockIdx.x * TW, y0 = blockIdx.y * TH;
+    const int x0 = (tall ? blockIdx.y : blockIdx.x) * TW, y0 = (tall ? blockIdx.x : blockIdx.y) * TH;
     const uint32_t phase = PH_DIFF | ((uint32_t)species << 8) | (uint32_t)(DIR + 1);
     const int64_t plane0 = ((int64_t)r0 * S + species) * area, plane_step = (int64_t)S * area;
     const auto set_up = [&](SweepCell& cell, int gx, int gy) {
@@ -745,8 +747,10 @@ cudaError_t launch_sweep_t(const GridDesc& g, const int32_t* in, int32_t* out, i
                            cudaStream_t st) {
     constexpr int TW = DIR == 0 ? 32 : 8, TH = DIR == 0 ? 8 : 32;
     dim3 grid((g.W + TW - 1) / TW, (g.H + TH - 1) / TH, (g.R + kSweepReal - 1) / kSweepReal);
+    const int tall = grid.y > 65535;      // then fewer than 2048 cells are a row: a grid has at most 2^30
+    if (tall) std::swap(grid.x, grid.y);
     k_sweep<DIR><<<grid, NT, 0, st>>>(in, out, g.W, g.H, g.S, g.R, species, seed, step_seed, g.bmask[2 * DIR],
-                                      g.bmask[2 * DIR + 1], d_D, d_r, dt, dx, fpe);
+                                      g.bmask[2 * DIR + 1], d_D, d_r, dt, dx, fpe, tall);
     return cudaGetLastError();
 }
 }  // namespace

@@ -77,9 +77,10 @@ struct EnsArgs {
     int64_t* snap_time_off;  // per instance: first float of its snapshot times, or -1
     int32_t* status;
     int64_t* steps;
-    int32_t* lost;           // [CTA or cluster][2][max_area * 4]
+    int32_t* lost;           // [CTA or cluster][halves][lost_half]
     int cluster;             // CTAs per instance
-    int64_t lost_stride;
+    int halves;              // lost buffers, 1 or 2
+    int64_t lost_half;       // max_area * 4
     unsigned int* queue;
     int n_inst;
     int max_species;
@@ -88,7 +89,7 @@ struct EnsArgs {
 // CL: the instance's cells are shared by a cluster of CTAs (A.cluster of them); every CTA
 // steps the same clocks.  A thread keeps its cells for the whole run, so only the lost
 // counts of a species cross between threads: one barrier per jump, with the two halves of
-// the lost buffer in turn.
+// the lost buffer in turn (a second barrier where there is one half, ens_halves).
 template <int NT, bool CL>
 __global__ void __launch_bounds__(NT) k_ensemble(EnsArgs A) {
     extern __shared__ __align__(16) unsigned char smem[];
@@ -116,7 +117,7 @@ __global__ void __launch_bounds__(NT) k_ensemble(EnsArgs A) {
         else
             __syncthreads();
     };
-    int32_t* lost2 = A.lost + (int64_t)(blockIdx.x / csize) * A.lost_stride;
+    int32_t* lost2 = A.lost + (int64_t)(blockIdx.x / csize) * A.halves * A.lost_half;
     int half = 0;
     for (;;) {
         if (rank == 0 && threadIdx.x == 0) s_item = (int)atomicAdd(A.queue, 1u);
@@ -233,8 +234,8 @@ __global__ void __launch_bounds__(NT) k_ensemble(EnsArgs A) {
                     if (!(i == c.minspec || s_next[i] <= c.mindt)) continue;
                     if (!(s_next[i] > 0)) continue;
                     int32_t* plane = st + (int64_t)i * area;
-                    int32_t* lost = lost2 + (int64_t)half * (A.lost_stride / 2);
-                    half ^= 1;
+                    int32_t* lost = lost2 + (int64_t)half * A.lost_half;
+                    half ^= A.halves - 1;
                     for (int cell = me; cell < area; cell += stride) {
                         Stream rs;
                         rs.init(key0, key1, sd, (uint32_t)cell, PH_DIFF | ((uint32_t)i << 8));
@@ -253,6 +254,7 @@ __global__ void __launch_bounds__(NT) k_ensemble(EnsArgs A) {
                         if (y < W - 1) v += lost[4 * (cell + W) + 2];
                         plane[cell] = v;
                     }
+                    if (A.halves == 1) sync();
                 }
             } else if (c.simTime >= c.outputLast + s_inst.output_interval) {
                 snapshot(c.mindt);
@@ -409,6 +411,14 @@ double ens_makespan(const std::vector<EnsCost>& cost, int cluster, int groups) {
     return end;
 }
 
+// CTAs that are launched: no more than there are instances
+int ens_grid(const gpgmp_ensemble* h) { return std::min(h->grid, h->n * h->cluster); }
+// Lost buffers per CTA or cluster: two save a jump one of its two barriers, which counts where
+// a thread has few cells.  One CTA on more than 128 x 128 cells has dozens for each, and a
+// second buffer for every CTA of the chip would double the scratch (592 CTAs of 512 x 512
+// cells: 2.5 GB with one); clusters are too few for that.
+int ens_halves(const gpgmp_ensemble* h) { return h->cluster > 1 || h->max_area <= 128 * 128 ? 2 : 1; }
+
 int configure(gpgmp_ensemble* h, int threads, int ctas_per_sm) {
     if (threads != 128 && threads != 256 && threads != 512 && threads != 1024)
         return set_error(GPGMP_ERR_INVALID, "threads per CTA must be 128, 256, 512 or 1024");
@@ -450,10 +460,10 @@ int configure(gpgmp_ensemble* h, int threads, int ctas_per_sm) {
             h->grid = std::min(groups, h->n) * cl;
         }
     }
-    // lost-count scratch: two buffers per CTA or cluster
+    // lost-count scratch
     if (h->d_lost) cudaFree(h->d_lost);
     h->d_lost = nullptr;
-    CK(cudaMalloc(&h->d_lost, sizeof(int32_t) * 2 * 4 * (size_t)h->max_area * (h->grid / h->cluster)));
+    CK(cudaMalloc(&h->d_lost, sizeof(int32_t) * 4 * (size_t)h->max_area * ens_halves(h) * (ens_grid(h) / h->cluster)));
     if (h->exec) { cudaGraphExecDestroy(h->exec); h->exec = nullptr; }
     if (h->graph) { cudaGraphDestroy(h->graph); h->graph = nullptr; }
     return GPGMP_OK;
@@ -600,7 +610,8 @@ int gpgmp_ensemble_run(gpgmp_ensemble* h, int32_t* state, int32_t* snapshots, vo
         a.packed = h->d_packed; a.nnet = h->d_nnet;
         a.state = state; a.snapshots = snapshots; a.snap_times = h->d_snap_times;
         a.snap_time_off = h->d_snap_time_off; a.status = h->d_status; a.steps = h->d_steps;
-        a.lost = h->d_lost; a.lost_stride = 2 * 4 * (int64_t)h->max_area; a.cluster = h->cluster; a.queue = h->d_queue; a.n_inst = h->n;
+        a.lost = h->d_lost; a.lost_half = 4 * (int64_t)h->max_area; a.halves = ens_halves(h);
+        a.cluster = h->cluster; a.queue = h->d_queue; a.n_inst = h->n;
         a.max_species = h->max_species;
         a.max_reactions = h->max_reactions;
         cudaError_t e = cudaStreamBeginCapture(cap, cudaStreamCaptureModeThreadLocal);
@@ -610,7 +621,7 @@ int gpgmp_ensemble_run(gpgmp_ensemble* h, int32_t* state, int32_t* snapshots, vo
             void* args[] = {&a};
             cudaLaunchConfig_t cfg;
             cudaLaunchAttribute attr[1];
-            ens_launch_config(h, h->cluster, h->grid, &cfg, attr, cap);
+            ens_launch_config(h, h->cluster, ens_grid(h), &cfg, attr, cap);
             const cudaError_t launched = cudaLaunchKernelExC(&cfg, ens_kernel(h->threads, h->cluster > 1), args);
             e = cudaStreamEndCapture(cap, &h->graph);
             if (e == cudaSuccess) e = launched;

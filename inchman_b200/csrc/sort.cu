@@ -175,15 +175,18 @@ __global__ void __launch_bounds__(kScanThreads, 2) k_scan_exclusive(const uint32
     t.store(out, wbase, n, vec, lane, s_base[warp], s_row[warp]);
 }
 
-// Large scans: one CTA per SM, all of them resident (cooperative launch), in rounds of one
-// tile per CTA.  A CTA publishes its tile's sum and reads every CTA's of the round: the sums
-// before its own give its prefix, all of them the carry into the next round, so there is no
-// chain of look-backs.  A sum takes 2 to 4 us to reach the other SMs while memory is busy,
-// longer than a tile's share of the bandwidth (3 us), so a CTA keeps three tiles in shared
-// memory: one loading (bulk copy), one whose sum is published, one whose round is complete
-// and which is written.  2^27 values: 214 us, 5.0 TB/s (306 us with every tile staged in
-// shared memory by its own CTA and chained look-backs; 459 us in rounds without the third
-// tile; HBM's floor is 166).
+// Large scans: one CTA per SM, each with a ring of tiles that it takes by number as it goes.  A
+// CTA publishes its tile's sum and adds up the sums of all tiles since its last one, so there
+// is no chain of look-backs.  A sum takes 2 to 4 us to reach the other SMs while memory is
+// busy, longer than a tile's share of the bandwidth (3 us), so a CTA keeps three tiles in
+// shared memory: one loading (bulk copy), one whose sum is published, one whose prefix is
+// complete and which is written.  A tile waits only for tiles of lower numbers, which running
+// CTAs have taken, and a CTA publishes a tile's sum before it waits for that tile's prefix: the
+// CTAs need not run at once, so a scan beside another kernel's makes do with the SMs it
+// finds.  2^27 values: 187 us, 5.7 TB/s (306 us with every tile staged in shared memory by
+// its own CTA and chained look-backs; 214 us with the CTAs in rounds of fixed tiles, which had
+// to run all at once; HBM's floor is
+// 166).
 constexpr int kStreamThreads = 1024, kStreamWarps = kStreamThreads / 32, kStreamStages = 3;
 constexpr int kStreamRows = kScanTile / (128 * kStreamWarps);
 constexpr int kStreamSmem = kStreamStages * kScanTile * (int)sizeof(uint32_t);
@@ -194,14 +197,15 @@ __global__ void __launch_bounds__(kStreamThreads, 1) k_scan_stream(const uint32_
                                                                    uint64_t* __restrict__ scratch, uint32_t tiles) {
     extern __shared__ __align__(128) uint32_t s_ring[];      // [stage][kScanTile]
     __shared__ __align__(8) uint64_t s_full[kStreamStages];
+    __shared__ uint32_t s_tile[kStreamStages];               // the tiles of the ring, past the last: >= tiles
     __shared__ uint32_t s_warp[kStreamWarps], s_base[kStreamWarps];
     __shared__ __align__(16) uint32_t s_row[kStreamWarps][128];
     int* err = reinterpret_cast<int*>(scratch) + 2;
     uint64_t* status = scratch + 2;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const uint32_t G = gridDim.x, rank = blockIdx.x;
-    const uint32_t mine = rank < tiles ? (tiles - rank + G - 1) / G : 0;      // tiles rank, rank + G, ...
-    const auto first = [&](uint32_t i) { return ((int64_t)i * G + rank) * kScanTile; };
+    unsigned int* counter = reinterpret_cast<unsigned int*>(scratch);
+    const auto tile_of = [&](uint32_t i) { return s_tile[i % kStreamStages]; };
+    const auto first = [&](uint32_t i) { return (int64_t)tile_of(i) * kScanTile; };
     const auto whole = [&](uint32_t i) { return first(i) + kScanTile <= n; };  // all but the last tile of all
     const auto issue = [&](uint32_t i) {
         const uint32_t bar = scan_smem(&s_full[i % kStreamStages]);
@@ -252,46 +256,57 @@ __global__ void __launch_bounds__(kStreamThreads, 1) k_scan_stream(const uint32_
         x = __reduce_add_sync(0xffffffffu, x);
         if (lane == 0) s_warp[warp] = x;
     };
+    // thread 0 takes tile numbers a tile ahead of their loads (next), so that no load waits for one
+    uint32_t next = 0;
+    const auto take = [&](uint32_t i) {
+        s_tile[i % kStreamStages] = next;
+        if (next < tiles) {
+            if (whole(i)) issue(i);
+            next = atomicAdd(counter, 1u);
+        }
+    };
     if (threadIdx.x == 0) {
+        next = atomicAdd(counter, 1u);
         for (int b = 0; b < kStreamStages; ++b)
             asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(scan_smem(&s_full[b])) : "memory");
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
-        for (uint32_t i = 0; i < kStreamStages && i < mine; ++i)
-            if (whole(i)) issue(i);
+        for (uint32_t i = 0; i < kStreamStages; ++i) take(i);
     }
     __syncthreads();
-    uint32_t carry = 0, ex = 0;       // warp 0: the sum of all earlier rounds; the tile's sums before each warp
-    if (mine > 0) {
+    uint32_t carry = 0, from = 0, ex = 0;       // warp 0: the sum of tiles 0 .. from - 1; the tile's sums before each warp
+    if (tile_of(0) < tiles) {
         sums(0);
         __syncthreads();
         if (warp == 0) {
             uint32_t aggregate;
             ex = scan_warps<kStreamWarps>(s_warp[lane], lane, &aggregate);
-            if (lane == 0) st_relaxed_u64(&status[rank], kScanFlagA | aggregate);
+            if (lane == 0) st_relaxed_u64(&status[tile_of(0)], kScanFlagA | aggregate);
         }
         __syncthreads();
     }
-    for (uint32_t i = 0; i < mine; ++i) {
-        if (i + 1 < mine) sums(i + 1);
+    for (uint32_t i = 0; tile_of(i) < tiles; ++i) {      // the same in every thread of the block
+        const bool more = tile_of(i + 1) < tiles;
+        if (more) sums(i + 1);
         __syncthreads();
         if (warp == 0) {
             uint32_t ex_next = 0;
-            if (i + 1 < mine) {
+            if (more) {
                 uint32_t aggregate;
                 ex_next = scan_warps<kStreamWarps>(s_warp[lane], lane, &aggregate);
-                if (lane == 0) st_relaxed_u64(&status[(i + 1) * G + rank], kScanFlagA | aggregate);
+                if (lane == 0) st_relaxed_u64(&status[tile_of(i + 1)], kScanFlagA | aggregate);
             }
-            const uint32_t r0 = i * G;
-            uint32_t before = 0, all = 0, spins = 0;
-            for (uint32_t q0 = 0; q0 < G; q0 += 32 * 5) {
-                uint64_t w[5];
+            const uint32_t tile = tile_of(i);
+            uint32_t before = 0, spins = 0;
+            constexpr int kWords = 6;             // 192 tiles, a round of the SMs and some more, in one go
+            for (uint32_t q0 = from; q0 < tile; q0 += 32 * kWords) {
+                uint64_t w[kWords];
                 bool ready;
                 do {
                     ready = true;
 #pragma unroll
-                    for (int u = 0; u < 5; ++u) {
+                    for (int u = 0; u < kWords; ++u) {
                         const uint32_t q = q0 + 32 * u + lane;
-                        w[u] = q < G && r0 + q < tiles ? ld_volatile_u64(&status[r0 + q]) : kScanFlagA;
+                        w[u] = q < tile ? ld_volatile_u64(&status[q]) : kScanFlagA;
                         ready = ready && (w[u] >> 32) != 0;
                     }
                     if (!ready && ++spins > kSpinLimit) {
@@ -300,15 +315,11 @@ __global__ void __launch_bounds__(kStreamThreads, 1) k_scan_stream(const uint32_
                     }
                 } while (!__all_sync(0xffffffffu, ready));
 #pragma unroll
-                for (int u = 0; u < 5; ++u) {
-                    all += (uint32_t)w[u];
-                    if (q0 + 32 * u + lane < rank) before += (uint32_t)w[u];
-                }
+                for (int u = 0; u < kWords; ++u) before += (uint32_t)w[u];
             }
-            before = __reduce_add_sync(0xffffffffu, before);
-            all = __reduce_add_sync(0xffffffffu, all);
-            s_base[lane] = carry + before + ex;
-            carry += all;
+            carry += __reduce_add_sync(0xffffffffu, before);
+            from = tile;
+            s_base[lane] = carry + ex;
             ex = ex_next;
         }
         __syncthreads();
@@ -316,7 +327,7 @@ __global__ void __launch_bounds__(kStreamThreads, 1) k_scan_stream(const uint32_
         t.sum(lane);
         t.store(out, first(i) + warp * t.kValues, n, 1, lane, s_base[warp], s_row[warp]);
         __syncthreads();
-        if (threadIdx.x == 0 && i + kStreamStages < mine && whole(i + kStreamStages)) issue(i + kStreamStages);
+        if (threadIdx.x == 0) take(i + kStreamStages);
     }
 }
 
@@ -884,31 +895,9 @@ size_t scan_scratch_bytes(int64_t n) {
 }
 
 // Scans of more than one tile per SM stream (us, look-back -> stream: 2^22 values 14.7 ->
-// 13.7, 2^24 47 -> 35, 2^27 325 -> 214; below, both wait for the launch), where the pointers
-// are 16-byte aligned as the bulk copies want them.  *sms: the device's SMs if each holds the
-// kernel's one CTA, else 0; cached per device.
+// 13.7, 2^24 47 -> 35, 2^27 325 -> 187; below, both wait for the launch), where the pointers
+// are 16-byte aligned as the bulk copies want them.
 constexpr int64_t kStreamMinTiles = 64;
-static cudaError_t stream_sms(int* sms) {
-    static std::mutex mu;
-    static int cache[64];        // 0: not asked yet, -1: the kernel does not fit
-    int dev = 0;
-    cudaError_t e = cudaGetDevice(&dev);
-    if (e != cudaSuccess) return e;
-    *sms = 0;
-    if (dev < 0 || dev >= 64) return cudaSuccess;
-    std::lock_guard<std::mutex> lock(mu);
-    if (cache[dev] == 0) {
-        int per_sm = 0, n = 0;
-        e = cudaFuncSetAttribute(k_scan_stream, cudaFuncAttributeMaxDynamicSharedMemorySize, kStreamSmem);
-        if (e == cudaSuccess)
-            e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_scan_stream, kStreamThreads, kStreamSmem);
-        if (e == cudaSuccess) e = cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
-        if (e != cudaSuccess) return e;
-        cache[dev] = per_sm >= 1 ? n : -1;
-    }
-    *sms = cache[dev] > 0 ? cache[dev] : 0;
-    return cudaSuccess;
-}
 
 cudaError_t scan_exclusive_u32(const uint32_t* in, uint32_t* out, int64_t n, void* scratch, cudaStream_t st) {
     if (n <= 0) return cudaSuccess;
@@ -918,23 +907,16 @@ cudaError_t scan_exclusive_u32(const uint32_t* in, uint32_t* out, int64_t n, voi
         if (e != cudaSuccess) return e;
     }
     const int vec = (((uintptr_t)in | (uintptr_t)out) & 15u) == 0 ? 1 : 0;
-    int sms = 0;
     if (vec && tiles > kStreamMinTiles) {
-        cudaError_t e = stream_sms(&sms);
+        int dev = 0, sms = 0;
+        cudaError_t e = cudaGetDevice(&dev);
+        if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(k_scan_stream, cudaFuncAttributeMaxDynamicSharedMemorySize, kStreamSmem);
         if (e != cudaSuccess) return e;
-    }
-    if (tiles > sms && sms > 0) {
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3(sms, 1, 1);
-        cfg.blockDim = dim3(kStreamThreads, 1, 1);
-        cfg.dynamicSmemBytes = kStreamSmem;
-        cfg.stream = st;
-        cudaLaunchAttribute attr[1];
-        attr[0].id = cudaLaunchAttributeCooperative;
-        attr[0].val.cooperative = 1;
-        cfg.attrs = attr;
-        cfg.numAttrs = 1;
-        return cudaLaunchKernelEx(&cfg, k_scan_stream, in, out, n, (uint64_t*)scratch, (uint32_t)tiles);
+        if (tiles > sms) {
+            k_scan_stream<<<sms, kStreamThreads, kStreamSmem, st>>>(in, out, n, (uint64_t*)scratch, (uint32_t)tiles);
+            return cudaGetLastError();
+        }
     }
     k_scan_exclusive<<<(unsigned)tiles, kScanThreads, 0, st>>>(in, out, n, (uint64_t*)scratch, vec, (uint32_t)tiles);
     return cudaGetLastError();

@@ -118,9 +118,10 @@ __device__ __forceinline__ float gp_logf(float x) {
 }
 
 // a / b to the nearest, for a and b well inside the normal range (2^-60 < |b| < 2^60 and
-// |a / b| > 2^-100 or a = 0): Newton's step on the approximate reciprocal, then Markstein's
-// correction (1990, as div_small below).  Three instructions and a branch less than the
-// operator, which also serves the rest of the range.
+// |a / b| > 2^-100 or a = 0): Newton's step on the approximate reciprocal gives the nearest
+// reciprocal (compared for every significand of b; the instruction's error bound alone leaves
+// a dozen in doubt), then Markstein's correction (1990, as div_small below) the nearest
+// quotient.
 __device__ __forceinline__ float div_mid(float a, float b) {
 #ifdef __CUDA_ARCH__
     float y;

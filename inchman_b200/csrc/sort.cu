@@ -185,8 +185,7 @@ __global__ void __launch_bounds__(kScanThreads, 2) k_scan_exclusive(const uint32
 // CTAs need not run at once, so a scan beside another kernel's makes do with the SMs it
 // finds.  2^27 values: 187 us, 5.7 TB/s (306 us with every tile staged in shared memory by
 // its own CTA and chained look-backs; 214 us with the CTAs in rounds of fixed tiles, which had
-// to run all at once; HBM's floor is
-// 166).
+// to run all at once; HBM's floor is 166).
 constexpr int kStreamThreads = 1024, kStreamWarps = kStreamThreads / 32, kStreamStages = 3;
 constexpr int kStreamRows = kScanTile / (128 * kStreamWarps);
 constexpr int kStreamSmem = kStreamStages * kScanTile * (int)sizeof(uint32_t);

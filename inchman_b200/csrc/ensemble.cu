@@ -79,7 +79,7 @@ struct EnsArgs {
     int64_t* steps;
     int32_t* lost;           // [CTA or cluster][halves][lost_half]
     int cluster;             // CTAs per instance
-    int halves;              // lost buffers, 1 or 2
+    int halves;              // lost buffers, 1 or 2 (2 for clusters)
     int64_t lost_half;       // max_area * 4
     unsigned int* queue;
     int n_inst;
@@ -117,7 +117,8 @@ __global__ void __launch_bounds__(NT) k_ensemble(EnsArgs A) {
         else
             __syncthreads();
     };
-    int32_t* lost2 = A.lost + (int64_t)(blockIdx.x / csize) * A.halves * A.lost_half;
+    const int halves = CL ? 2 : A.halves;
+    int32_t* lost2 = A.lost + (int64_t)(blockIdx.x / csize) * halves * A.lost_half;
     int half = 0;
     for (;;) {
         if (rank == 0 && threadIdx.x == 0) s_item = (int)atomicAdd(A.queue, 1u);
@@ -235,7 +236,7 @@ __global__ void __launch_bounds__(NT) k_ensemble(EnsArgs A) {
                     if (!(s_next[i] > 0)) continue;
                     int32_t* plane = st + (int64_t)i * area;
                     int32_t* lost = lost2 + (int64_t)half * A.lost_half;
-                    half ^= A.halves - 1;
+                    half ^= halves - 1;
                     for (int cell = me; cell < area; cell += stride) {
                         Stream rs;
                         rs.init(key0, key1, sd, (uint32_t)cell, PH_DIFF | ((uint32_t)i << 8));
@@ -254,7 +255,7 @@ __global__ void __launch_bounds__(NT) k_ensemble(EnsArgs A) {
                         if (y < W - 1) v += lost[4 * (cell + W) + 2];
                         plane[cell] = v;
                     }
-                    if (A.halves == 1) sync();
+                    if (halves == 1) sync();
                 }
             } else if (c.simTime >= c.outputLast + s_inst.output_interval) {
                 snapshot(c.mindt);

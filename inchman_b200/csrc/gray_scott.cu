@@ -678,8 +678,8 @@ MCConfig mc_config() {
 }
 constexpr int kMCVariant = 40;
 constexpr int kMCConfigs = 7;
-// the automatic choice for n = 256: 4 clusters, 8 ghost rows (0.587 us per step;
-// (4, 16) 0.594, (4, 32) 0.611, the single-cluster kernel 0.74)
+// the automatic choice for n = 256: 4 clusters, 8 ghost rows (0.513 us per step; 0.587 when
+// the shapes were compared: (4, 16) 0.594, (4, 32) 0.611, the single-cluster kernel 0.74)
 constexpr int kMCDefault = 1;
 const MCConfig& mc_table(int i) {
     static const MCConfig t[kMCConfigs] = {mc_config<256, 2, 8, 9>(),   mc_config<256, 4, 8, 5>(),
@@ -779,7 +779,12 @@ cudaError_t mc_forward(int i, const GSArgs<float>& a0, bool drift, const float* 
 bool gs_own_side(int n) { return n == 64 || n == 128 || n == 256 || n == 512; }
 
 // the sides that take the tiled kernel under the automatic choice: those without a
-// register-resident kernel
+// register-resident kernel.  One solve at a time is 1.6 to 5 times as fast as on one cluster.  A
+// tiled solve fills the chip, though, where eight clusters hold eight solves on as many streams:
+// us per step and lattice with eight streams, one cluster each -> tiles, float32 160^2 0.32 ->
+// 0.19, 240^2 0.54 -> 0.38, 304^2 0.76 -> 0.53, 320^2 0.82 -> 0.93, 368^2 1.18 -> 1.01; float64
+// 160^2 0.35 -> 0.44, 192^2 0.43 -> 0.45, 240^2 0.77 -> 0.89, 256^2 0.50 -> 0.76.  The library
+// does not know the other streams; a program that has them sets the cluster size instead.
 constexpr int kTileVariant = 50;
 bool tile_side(int n, int elem_bytes) {
     return elem_bytes == 8 ? n != 64 && n != 128 : !gs_own_side(n);

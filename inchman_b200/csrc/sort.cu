@@ -341,7 +341,7 @@ struct SortShape {
     static constexpr int kItems = RB == 8 ? 18 : 15;
     static constexpr int kTile = kThreads * kItems;
     static constexpr int kWarps = kThreads / 32;
-    // keys and values of a tile in sorted order (dynamic shared memory: 30 / 60 KB)
+    // keys and values of a tile in sorted order (dynamic shared memory)
     static constexpr int kStagingBytes = 2 * kTile * (int)sizeof(uint32_t);
     static_assert(kTile < 65536, "positions in a tile fit 16 bits");
 };
@@ -936,8 +936,8 @@ SortLayout sort_layout(int64_t n, int key_bits) {
     size_t off = 0;
     L.off_hist = off;    off += align256(sizeof(uint32_t) * kHistWords);
     L.off_counters = off; off += align256(sizeof(uint32_t) * 8);     // tile counters [4], error word [4]
-    // look-back words for the widest layout (4 passes x 256 digits x 3840-key tiles, or
-    // 3 x 1024 x 7680-key tiles), so that the scratch size does not depend on key_bits
+    // look-back words for the widest layout (4 passes x 256 digits of SortShape<8>'s tiles, or
+    // 3 x 1024 of SortShape<10>'s), so that the scratch size does not depend on key_bits
     const int64_t t8 = (n + SortShape<8>::kTile - 1) / SortShape<8>::kTile;
     const int64_t t10 = (n + SortShape<10>::kTile - 1) / SortShape<10>::kTile;
     const int64_t look_words = std::max<int64_t>(std::max<int64_t>(4 * 256 * t8, 3 * 1024 * t10), 3 * 1024);

@@ -275,7 +275,12 @@ typedef struct gpgmp_gs_params {
     int32_t steps;
     double  F, k, Du, Dv, vx, vy, dt;
     int32_t checkpoint_every;   /* <= 0: 100 in float32; in float64 25 at n = 256, up to 100 on smaller lattices */
-    int32_t cluster;            /* CTAs per thread-block cluster, 0 = automatic */
+    int32_t cluster;            /* CTAs per thread-block cluster, 0 = automatic.  A program that
+                                   solves float64 lattices, or float32 ones around n = 320, on
+                                   many streams at once sets it (16 where n is a multiple of
+                                   16): each solve then keeps to its cluster's SMs, where the
+                                   tiled kernel 50 waits until the device has room for all its
+                                   tiles and serves the solves more or less in turn */
     int32_t variant;            /* kernel family (float32): 0 automatic = for n = 256 the
                                    multi-cluster kernel 41 where the device holds its four clusters at
                                    once, else register-resident where the lattice allows (n 64, 128,
@@ -287,14 +292,16 @@ typedef struct gpgmp_gs_params {
                                    CTA; 40 + i multi-cluster (n = 256; clusters, ghost rows):
                                    i = 0 (2, 8), 1 (4, 8), 2 (4, 16), 3 (8, 8), 4 (8, 16),
                                    5 (4, 32), 6 (2, 32), a CUDA error where the device cannot hold
-                                   all its clusters at once; 50 tiled, any n, a CUDA error where
+                                   all its clusters at once; 50 tiled, any n whose lattice a
+                                   cluster can hold (every family asks that), a CUDA error where
                                    the device cannot hold all its tiles at once.  (Under 0,
                                    40 + i and 50 a solve whose outputs overlap its inputs in
                                    part, or in place with no more steps than ghost cells,
                                    runs on one cluster.)  Every float32
                                    family gives the same bits (on sides other than 64, 128, 256,
                                    512 those of 1).  float64: 0 register-resident at n 64 and 128
-                                   on a 16-CTA cluster, else 50 as above; 1; 2; 50.  The
+                                   on a 16-CTA cluster, else 50 as above; 1; 2; 50 (0, 2 and 50
+                                   give the same forward bits on sides 64, 128 and 256).  The
                                    adjoint runs the multi-cluster adjoint under 40 + i (the same
                                    lambda bits); under 0, where the forward is multi-cluster, it
                                    recomputes the segments on two clusters (40) and runs the

@@ -69,3 +69,17 @@ def test_solve_and_gradient_on_views(gpgmp, dtype, n, steps, drift):
     if not drift:
         a, b = gs.forward(_behind(ins[0]), _behind(ins[1]), p)
         assert torch.equal(a, out[1][0]) or other
+
+
+@pytest.mark.parametrize("n", [64, 128, 256])
+@pytest.mark.parametrize("steps,drift", [(40, False), (101, True)])
+def test_float64_forward_bits(gpgmp, n, steps, drift):
+    """The float64 kernels of these sides and the tiles give the bits of the column walk."""
+    import torch
+    from inchman_b200 import gray_scott as gs
+    cfg = gs.GrayScottConfig(n=n, steps=steps, vx=0.05 if drift else 0.0, vy=-0.03 if drift else 0.0)
+    a, b = (torch.from_numpy(x).cuda() for x in cfg.initial_state(np.float64))
+    want = gs.forward(a, b, cfg.params(variant=2))
+    for variant in (0, 50):
+        got = gs.forward(a, b, cfg.params(variant=variant))
+        assert gs.status() == 0 and torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
